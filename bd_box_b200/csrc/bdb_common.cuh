@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -42,6 +43,7 @@ enum : unsigned {
     ST_LAUNCH = 16u,      // a kernel found its launch shape wrong and did nothing
 };
 
+struct EwaldFast;   // converged split of the Ewald sums (ewald_fast.cuh)
 // A bead segment: one independent system inside a batch.
 struct FrameRing;   // asynchronous trajectory frames (frames.cu)
 
@@ -51,10 +53,12 @@ struct Segment {
     int pbegin;    // first padded matrix row (stored-D systems)
 };
 
-// A TEA / D.F work item: bead tiles (I, J), I >= J, of one segment.
+// A TEA / D.F work item (tea.cu): steps [s0, s1) of row tile I (and I + 1)
+// of a segment against the column tiles J0 .. J0 + nJ - 1, and where its
+// records go.
 struct TileJob {
-    int seg;
-    int I, J;
+    int seg, I, J0, nJ, s0, s1, type;
+    int col0, rec0, rec1;
 };
 
 template <typename T>
@@ -104,6 +108,7 @@ struct bdb_system {
     // cell list
     bdb::DevBuf<unsigned long long> sorted_keys;   // (cell << 24 | local) per bead, per segment sorted
     bdb::DevBuf<int> sorted_idx;
+    bdb::DevBuf<double> pos_sorted;            // positions in that order, [3][n] (large systems)
     bdb::DevBuf<double4> grid;                 // per segment: origin xyz, cell size
     bdb::DevBuf<int4> grid_dims;               // per segment: nx, ny, nz, brute flag
     bdb::DevBuf<double4> pos_build;            // positions when the cell list was last sorted
@@ -111,13 +116,15 @@ struct bdb_system {
     bdb::DevBuf<long long> cell_off;           // per segment: offset of its table, capacity
     bdb::DevBuf<int> cells_built;              // per segment: 1 once sorted
     bdb::DevBuf<int> cells_resort;             // per segment above the shared-memory sort: re-sort now
+    bdb::DevBuf<int> cells_moved;              // per segment: a bead has left the skin (k_moved, forces.cu)
     bdb::DevBuf<unsigned long long> big_keys;  // two key buffers of the multi-CTA sort (forces.cu)
     size_t big_npow = 0;                       // their length each: the largest such segment, to a power of 2
     double cell_size = 0;
-    double skin = 0;
+    double skin = 0, reach = 0;                // cells are the widest interaction (reach) plus the skin
 
     // force outputs
     bdb::DevBuf<double> e_part;                // energy partials
+    bdb::DevBuf<unsigned> c_part;              // pair-count partials
     bdb::DevBuf<unsigned> status;              // status word
     bdb::DevBuf<unsigned long long> counts;    // pair counts
 
@@ -127,17 +134,20 @@ struct bdb_system {
     bdb::DevBuf<double> eps_part;
     bdb::DevBuf<double> scal;                  // device scalars (eps, beta, ...)
     bdb::DevBuf<bdb::TileJob> jobs;
-    bdb::DevBuf<int> tea_next;                 // job counter of the persistent TEA pair kernel
+    bdb::DevBuf<int> tea_cols;                 // TEA column records, one per job and column tile
     bdb::DevBuf<float> pscale;                 // mixed Cholesky: FP16 panel scale and 1/scale^2
-    bdb::DevBuf<unsigned char> tea_meta;       // TEA segment table + job offsets
-    int n_jobs = 0;
-    int tea_tile = 32;                         // TEA tile edge (16 or 32 beads)
+    bdb::DevBuf<unsigned char> tea_meta;       // TEA bead-tile and segment tables
+    int n_jobs = 0, tea_tiles = 0;
+    int tea_tile = 32;                         // TEA job length (16: half as long; tunable)
     int mv_warps = 16;                         // stored matvec: target warps per SM
     int chain_sms = 32;                        // Cholesky: SMs the bulk updates leave to the panel chain
                                                // (set per precision at creation)
     bool autotune = false, tea_tuned = false, mv_tuned = false, factor_tuned = false;
-    bdb::DevBuf<double> ewald_tab;             // Ewald lattice tables (rpy_tile.cuh EwaldConst)
-    int ewald_nk = 0, ewald_nimg = 0;
+    bdb::DevBuf<double> ewald_tab;             // Ewald reciprocal weights (rpy_tile.cuh EwaldConst)
+    double ewald_self[2] = {0, 0};             // a bead's sum over its own images: [0] + [1] sigma^2/L^2
+    bool ewald_recip = false;                  // some reciprocal weight is not zero
+    std::shared_ptr<bdb::EwaldFast> ewald_fast;   // the mixed path's converged split (ewald_fast.cuh), if it holds
+    double radius0 = 0;                        // radius of bead 0 at creation
     bdb::DevBuf<double> M64;                   // stored D (upper) + L (lower), FP64
     bdb::DevBuf<float> M32;                    // same, FP32 (mixed path)
     // IGT predictor-corrector: the tensor at the predicted positions, the

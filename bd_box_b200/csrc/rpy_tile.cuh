@@ -6,345 +6,419 @@
 //  * rpy_free: diff_tensor_calc_pos (diff_alg/diff_tensor.c:45-92), the
 //    free-space Rotne-Prager-Yamakawa tensor with the overlap form for
 //    r < a_i + a_j.
-//  * rpy_ewald_tab: diff_tensor_calc_ewald_beenakker (diff_tensor.c:265-401)
-//    with its self term (:404-422): real-space images r + L m and
-//    reciprocal vectors over the same sphere |m|^2 <= R^2, overlap
-//    correction on the raw (not minimum-image) separation, alpha = sqrt(pi)/L
-//    (init_tensor, :546-559). Constants that the reference forms from the
-//    float literal M_PIF are formed the same way on the host.
-//  * rpy_smith_tab: diff_tensor_calc_ewald_smith (diff_tensor.c:102-243) with
-//    its self term (:245-263): Oseen (O) and sigma^2 (Q) sums over the
-//    images r/L + m and the reciprocal vectors of the same sphere, in units
-//    of L, alpha = ewald_alpha, preO = 0.75/L, preQ = sigma^2/(2 L^3).
+//  * rpy_ewald: the lattice sums of diff_tensor_calc_ewald_beenakker
+//    (diff_tensor.c:265-401) and diff_tensor_calc_ewald_smith (:102-243) with
+//    their self terms (:404-422, :245-263): real-space images r + L m and
+//    reciprocal vectors over the same sphere |m|^2 <= R^2, overlap correction
+//    on the raw (not minimum-image) separation. Beenakker's alpha is
+//    sqrt(pi)/L (init_tensor, :546-559), Smith's ewald_alpha/L. Constants that
+//    the reference forms from the float literal M_PIF are formed the same way
+//    on the host.
+//
+// The sums are evaluated in units of L: v = r/L, s2 = sigma^2/L^2 and the
+// dimensionless alpha; the tile is preDii/L times the sum.
 #pragma once
+
+#include <type_traits>
 
 #include "bdb_common.cuh"
 
 namespace bdb {
 
-struct EwaldConst {
-    double L, inv_L, alpha, alpha2, alpha3, inv_alpha2, preQ;
-    double two_pif;      // 2*M_PIF evaluated in float
-    double four_pif2;    // 4*M_PIF*M_PIF evaluated in float
-    double six_pif;      // 6*M_PIF evaluated in float
-    int R, rr_sq;
-    // lattice tables (device memory, built by ewald_tables on the host):
-    // rk[12 k ..]: h, f, g, A_k, B_k, then 2(1 - e_a^2) for a = x, y, z and
-    // -2 e_a e_b for xy, xz, yz, over one half of the reciprocal sphere
-    // (k and -k contribute alike); img[m]: the real-space image offsets L m
-    const double* rk = nullptr;
-    const double4* img = nullptr;
-    int nk = 0, nimg = 0;
-    float rcut_sq = 0.f;   // mixed precision: real-space images beyond this are dropped
-    // Smith (rpy_smith_tab): rk rows are h, f, g, then the identity, e e^T
-    // and sigma^2 e e^T coefficients (k and -k together), then the six
-    // products e_a e_b (xx, yy, zz, xy, xz, yz)
-    int smith = 0;
-    double s_alpha = 0, s_alpha2 = 0, s_alpha3 = 0;
-    float s_rcut_sq = 0.f;   // mixed precision: (4.45/alpha)^2 in units of L^2, erfc(4.45) ~ 3e-10
-};
-
 // 1/sqrt(pi) as the reference's double build spells it (data.h:228)
 #define BDB_M1_SQRTPI 0.5641895835
 
-inline EwaldConst make_ewald(double L, double inv_L, int R)
+static constexpr int EWALD_MAX_R = 5;
+
+struct EwaldConst {
+    int smith = 0, R = 0;
+    double L = 0, inv_L = 0;
+    double alpha = 0, a2 = 0;       // alpha L and its square
+    double isp = 0;                 // 1/sqrt(pi), spelled as each method spells it
+    double two_pif = 0;             // 2*M_PIF evaluated in float
+    double kappa = 0;               // exp(-2 a2): second ratio of the Gaussian along an axis
+    // isqrt(R^2 - q), the extent of a row of the sphere, for q = 0 .. R^2
+    signed char extent[EWALD_MAX_R * EWALD_MAX_R + 1] = {};
+    // reciprocal weights (device memory), see ewald_tables: for h, f, g >= 0
+    // in the sphere, 12 values: the coefficients of xx, yy, zz (with
+    // cos cos cos), xy (sin sin cos), xz (sin cos sin), yz (cos sin sin), then
+    // the same of the terms in s2. recip is 0 when every weight is zero.
+    const double* rk = nullptr;
+    int recip = 0;
+    // the lattice sum of a bead with its own images: self0 + self1 s2
+    double self0 = 0, self1 = 0;
+    float rcut_sq = 0;              // mixed precision: images beyond this are dropped (erfc ~ 3e-10)
+};
+
+// 1/sqrt(x) for normal x: the hardware's estimate and Newton-Raphson steps in
+// residual form, y <- y + y/2 (1 - x y^2). FP64: the estimate has ~20 bits, two
+// steps leave its rounding (1 ulp). FP32: one step, about 0.8 ulp against 2 of
+// the estimate.
+__device__ __forceinline__ double inv_sqrt(double x)
 {
-    EwaldConst e;
-    e.L = L;
-    e.inv_L = inv_L;
-    e.alpha = BDB_SQRTPI * inv_L;
-    e.alpha2 = e.alpha * e.alpha;
-    e.alpha3 = e.alpha * e.alpha2;
-    e.inv_alpha2 = 1.0f / e.alpha2;
-    e.preQ = inv_L * inv_L * inv_L;
-    volatile float pif = BDB_M_PIF;
-    volatile float two = 2 * pif;
-    volatile float four = 4 * pif;
-    volatile float four2 = four * pif;
-    volatile float six = 6 * pif;
-    e.two_pif = two;
-    e.four_pif2 = four2;
-    e.six_pif = six;
-    e.R = R;
-    e.rr_sq = R * R;
-    return e;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+    return fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+}
+__device__ __forceinline__ float inv_sqrt(float x)
+{
+    const float y = rsqrtf(x);
+    return fmaf(0.5f * y, fmaf(-(x * y), y, 1.0f), y);
 }
 
-inline EwaldConst make_ewald_smith(double L, double inv_L, int R, double alpha)
-{
-    EwaldConst e = make_ewald(L, inv_L, R);
-    e.smith = 1;
-    e.s_alpha = alpha;
-    e.s_alpha2 = alpha * alpha;
-    e.s_alpha3 = alpha * e.s_alpha2;
-    e.s_rcut_sq = (float)((4.45 / alpha) * (4.45 / alpha));
-    return e;
-}
-
-// diff_tensor_calc_pos(i, j): sigma_i is bead j's radius, sigma_j bead i's,
-// e = (r_i - r_j)/|r_i - r_j|.
+// diff_tensor_calc_pos(i, j) from the separation d = r_i - r_j and the two
+// radii (which enter symmetrically): A I + B d d^T, with one reciprocal
+// square root instead of a square root and four divisions.
 template <typename T>
-__device__ __forceinline__ void rpy_free(const double4& pi, const double4& pj, T preDii, T preDij, T* t)
+__device__ __forceinline__ void rpy_free_sep(const T* d, T si, T sj, T preDii, T preDij, T* t)
 {
-    const T si = (T)pj.w, sj = (T)pi.w;
-    T e0 = (T)(pi.x - pj.x), e1 = (T)(pi.y - pj.y), e2 = (T)(pi.z - pj.z);
-    const T r_sq = e0 * e0 + e1 * e1 + e2 * e2;
-    const T r = sqrt(r_sq);
-    const T inv = (T)1 / r;
-    e0 *= inv;
-    e1 *= inv;
-    e2 *= inv;
+    const T r_sq = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    const T inv = inv_sqrt(r_sq);
+    const T inv_sq = inv * inv, r = r_sq * inv;
+    T A, B;
     if (r < si + sj) {
         const T sigma = (si + sj) / 2;
         const T pre = preDii / sigma;
         const T q = r / (32 * sigma);
-        const T part1 = 1 - 9 * q;
-        const T q3 = 3 * q;
-        t[0] = (part1 + q3 * e0 * e0) * pre;
-        t[1] = (part1 + q3 * e1 * e1) * pre;
-        t[2] = (part1 + q3 * e2 * e2) * pre;
-        t[3] = pre * q3 * e0 * e1;
-        t[4] = pre * q3 * e0 * e2;
-        t[5] = pre * q3 * e1 * e2;
+        A = (1 - 9 * q) * pre;
+        B = 3 * q * pre * inv_sq;
     } else {
-        const T pre = preDij / r;
-        const T sigm_r = (si * si + sj * sj) / r_sq;
-        const T a = 1 + sigm_r / 3;
-        const T b = 1 - sigm_r;
-        t[0] = (a + e0 * e0 * b) * pre;
-        t[1] = (a + e1 * e1 * b) * pre;
-        t[2] = (a + e2 * e2 * b) * pre;
-        t[3] = pre * e0 * e1 * b;
-        t[4] = pre * e0 * e2 * b;
-        t[5] = pre * e1 * e2 * b;
+        const T pre = preDij * inv;
+        const T sigm_r = (si * si + sj * sj) * inv_sq;
+        A = (1 + sigm_r * ((T)1 / 3)) * pre;
+        B = (1 - sigm_r) * pre * inv_sq;
     }
+    const T bx = B * d[0], by = B * d[1], bz = B * d[2];
+    t[0] = A + bx * d[0];
+    t[1] = A + by * d[1];
+    t[2] = A + bz * d[2];
+    t[3] = bx * d[1];
+    t[4] = bx * d[2];
+    t[5] = by * d[2];
 }
 
-// diff_tensor_calc_ewald_beenakker(i, j) (+ _diag for i == j) from the
-// lattice tables: each reciprocal vector once for the pair k, -k, with its
-// k-only factors precomputed. The FP64 path keeps every real-space image
-// and the reference's cos(2 pi_f k.r). With MIXED the real-space images are
-// summed in FP32 (images beyond rcut dropped) and the reciprocal phases
-// taken as FP32 cosines of the same argument, both accumulated in FP64.
-template <bool MIXED>
-__device__ __forceinline__ void rpy_ewald_tab(const double4& pi, const double4& pj, bool self, double preDii,
-                                              double preDij, const EwaldConst& ec, double* t)
+template <typename T>
+__device__ __forceinline__ void rpy_free(const double4& pi, const double4& pj, T preDii, T preDij, T* t)
 {
-    const double sigma_i = pj.w, sigma_j = pi.w;
-    const double r0 = pj.x - pi.x, r1 = pj.y - pi.y, r2 = pj.z - pi.z;
-    const double sigma_sq = 0.5 * (sigma_i * sigma_i + sigma_j * sigma_j);
-    double O[6] = {0, 0, 0, 0, 0, 0}, Qr[6] = {0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < 6; ++k) t[k] = 0;
-    const double rr = r0 * r0 + r1 * r1 + r2 * r2;
-    if (!self && rr < (sigma_i + sigma_j) * (sigma_i + sigma_j)) {
-        const double r = sqrt(rr), inv = 1 / r;
-        const double e[3] = {r0 * inv, r1 * inv, r2 * inv};
-        const double sigma = (sigma_i + sigma_j) / 2;
-        const double pre = preDii / sigma;
-        const double part1 = 1 - (9 * r / (32 * sigma));
-        const double pre2 = preDij / r;
-        const double sigm_r = (sigma_i * sigma_i + sigma_j * sigma_j) / rr;
-        const double p1 = 1 + sigm_r / 3;
-        const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-        for (int k = 0; k < 3; ++k)
-            t[k] += pre * (part1 + 3 * e[k] * e[k] * r / (32 * sigma)) - pre2 * (p1 + e[k] * e[k] * (1 - sigm_r));
-        for (int k = 3; k < 6; ++k)
-            t[k] += pre * 3 * e[ia[k]] * e[ib[k]] * r / (32 * sigma) - pre2 * e[ia[k]] * e[ib[k]] * (1 - sigm_r);
+    const T d[3] = {(T)(pi.x - pj.x), (T)(pi.y - pj.y), (T)(pi.z - pj.z)};
+    rpy_free_sep<T>(d, (T)pi.w, (T)pj.w, preDii, preDij, t);
+}
+
+// ---- the scaled complementary error function, erfcx(x) = exp(x^2) erfc(x),
+// for x >= 0: (1 + 2x) erfcx(x) as a polynomial in t = (x - K)/(x + K), the
+// transformation of Shepherd and Laframboise (Math. Comp. 36, 249 (1981)).
+// The coefficients are Chebyshev interpolants at K = 3.5 (FP64, 1.2e-16 on
+// x >= 0) and K = 2.5 (FP32, 1.2e-7 on 0 <= x <= 9), computed in 50 digits.
+// One reciprocal serves both quotients: d = 1/((x + K)(1 + 2x)).
+// constant memory: a constant operand of the multiply-add, where a 64-bit
+// immediate would take two more instructions
+static __constant__ double kErfcx64[24] = {
+    1.2423492448711544, -0.1400091801376197, -0.010555596332221669, 0.09751909515328706,
+    -0.11508959816003075, 0.08798315382403678, -0.04882332583088402, 0.019099330953271165,
+    -0.004215019879774186, -0.0003022679534333239, 0.0005643842668705102, -0.00012151212091980101,
+    -4.2781739959539994e-05, 2.4260300984917994e-05, 2.3273309537791425e-06, -3.814012584490695e-06,
+    -4.309237398316666e-08, 6.014823849950426e-07, -8.611571571113718e-09, -9.64004253144383e-08,
+    6.651894382376532e-10, 1.3624442778701048e-08, 6.040390099342991e-11, -1.1656687889203665e-09};
+__device__ __forceinline__ double erfcx_pos(double x)
+{
+    const double p = x + 3.5, q = fma(2.0, x, 1.0), pq = p * q;
+    double d;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(d) : "d"(pq));
+    d = fma(d, fma(-pq, d, 1.0), d);
+    d = fma(d, fma(-pq, d, 1.0), d);
+    const double t = (x - 3.5) * (q * d);
+    // even and odd powers side by side: two chains of 11 instead of one of 23
+    const double u = t * t;
+    double e = kErfcx64[22], o = kErfcx64[23];
+#pragma unroll
+    for (int k = 20; k >= 0; k -= 2) {
+        e = fma(e, u, kErfcx64[k]);
+        o = fma(o, u, kErfcx64[k + 1]);
     }
-    // real space
-    if (MIXED) {
-        const float a = (float)ec.alpha, a2 = (float)ec.alpha2, a3 = (float)ec.alpha3;
-        const float s2 = (float)sigma_sq;
-        const float a5s = 20.f * a2 * a3 * s2, a5s16 = 16.f * a2 * a3 * s2, a7s = 4.f * a3 * a2 * a2 * s2;
-        const float c0 = 14.f * a3 * s2 - 4.5f * a, c0b = -2.f * a3 * s2 + 1.5f * a;
-        const float isp = (float)(1.0 / BDB_SQRTPI);
-        const float fx = (float)r0, fy = (float)r1, fz = (float)r2;
-        float o[6] = {0, 0, 0, 0, 0, 0};
-        for (int m = 0; m < ec.nimg; ++m) {
-            const double4 off = ec.img[m];
-            const float x = fx + (float)off.x, y = fy + (float)off.y, z = fz + (float)off.z;
-            const float r_sq = x * x + y * y + z * z;
-            if (r_sq == 0.f || r_sq > ec.rcut_sq) continue;
-            const float inv_r = rsqrtf(r_sq), inv_r2 = inv_r * inv_r, inv_r3 = inv_r * inv_r2, r = r_sq * inv_r;
-            const float ex = __expf(-a2 * r_sq) * isp;
-            const float ec_ = erfcf(r * a);
-            const float sc = (a * s2 * inv_r2 + c0 - a5s * r_sq + 3.f * a3 * r_sq + a7s * r_sq * r_sq) * ex +
-                             ec_ * (0.75f * inv_r + 0.5f * s2 * inv_r3);
-            const float sc2 = (-3.f * a * s2 * inv_r2 + c0b + a5s16 * r_sq - 3.f * a3 * r_sq - a7s * r_sq * r_sq) * ex +
-                              ec_ * (0.75f * inv_r - 1.5f * s2 * inv_r3);
-            const float e0 = x * inv_r, e1 = y * inv_r, e2 = z * inv_r;
-            o[0] += sc + sc2 * e0 * e0;
-            o[1] += sc + sc2 * e1 * e1;
-            o[2] += sc + sc2 * e2 * e2;
-            o[3] += sc2 * e0 * e1;
-            o[4] += sc2 * e0 * e2;
-            o[5] += sc2 * e1 * e2;
-        }
-        for (int k = 0; k < 6; ++k) O[k] = o[k];
-    } else {
-        const double a = ec.alpha, a2 = ec.alpha2, a3 = ec.alpha3;
-        for (int m = 0; m < ec.nimg; ++m) {
-            const double4 off = ec.img[m];
-            const double x = r0 + off.x, y = r1 + off.y, z = r2 + off.z;
-            const double r_sq = x * x + y * y + z * z;
-            if (r_sq == 0.0) continue;
-            const double r = sqrt(r_sq);
-            const double inv_r = 1 / r, inv_r2 = 1 / r_sq, inv_r3 = inv_r * inv_r2;
-            const double e[3] = {x * inv_r, y * inv_r, z * inv_r};
-            const double ex = exp(-a2 * r_sq);
-            const double ec_ = erfc(r * a);
-            double sc = a * sigma_sq * inv_r2 + 14 * a3 * sigma_sq - 4.5 * a - 20 * a2 * a3 * sigma_sq * r_sq +
-                        3 * a3 * r_sq + 4 * a3 * a2 * a2 * sigma_sq * r_sq * r_sq;
-            sc = sc * ex / BDB_SQRTPI + ec_ * (0.75 * inv_r + 0.5 * sigma_sq * inv_r3);
-            double sc2 = -3 * a * sigma_sq * inv_r2 - 2 * a3 * sigma_sq + 1.5 * a + 16 * a2 * a3 * sigma_sq * r_sq -
-                         3 * a3 * r_sq - 4 * a3 * a2 * a2 * sigma_sq * r_sq * r_sq;
-            sc2 = sc2 * ex / BDB_SQRTPI + ec_ * (0.75 * inv_r - 1.5 * sigma_sq * inv_r3);
-            O[0] += sc + sc2 * e[0] * e[0];
-            O[1] += sc + sc2 * e[1] * e[1];
-            O[2] += sc + sc2 * e[2] * e[2];
-            O[3] += sc2 * e[0] * e[1];
-            O[4] += sc2 * e[0] * e[2];
-            O[5] += sc2 * e[1] * e[2];
-        }
+    const double r = fma(o, t, e);
+    return r * (p * d);
+}
+__device__ __forceinline__ float erfcx_pos(float x)
+{
+    const float p = x + 2.5f, q = fmaf(2.0f, x, 1.0f);
+    float d;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(p * q));
+    const float t = (x - 2.5f) * (q * d);
+    float r = 0.0004457839258919816f;
+    r = fmaf(r, t, 0.00030503612796383756f);
+    r = fmaf(r, t, -0.004302876907248387f);
+    r = fmaf(r, t, 0.0010337509324308317f);
+    r = fmaf(r, t, 0.03274950128568062f);
+    r = fmaf(r, t, -0.1029877887892802f);
+    r = fmaf(r, t, 0.15763045854613184f);
+    r = fmaf(r, t, -0.09902309465772124f);
+    r = fmaf(r, t, -0.12235677564486401f);
+    r = fmaf(r, t, 1.2648381682779481f);
+    return r * (p * d);
+}
+
+// exp(-a2 r2) in FP32 for a2 = -(hi + lo) ln 2: the exponent's rounding error
+// is put back, so that the hardware's exp2 (2 ulp) is what is left of it --
+// __expf loses |a2 r2| half-ulps, 1e-6 at the cutoff
+struct Gauss32 {
+    float hi, lo;
+    __host__ __device__ explicit Gauss32(double a2)
+    {
+        const double c = -a2 * 1.4426950408889634074;   // log2(e)
+        hi = (float)c;
+        lo = (float)(c - (double)hi);
     }
-    // reciprocal space
-    const double v0 = r0 * ec.inv_L, v1 = r1 * ec.inv_L, v2 = r2 * ec.inv_L;
-    for (int k = 0; k < ec.nk; ++k) {
-        const double* q = ec.rk + 12 * k;
-        const double ph = v0 * q[0] + v1 * q[1] + v2 * q[2];
-        double cs;
-        if (MIXED) {
-            // cos(2 pi_f ph), pi_f the float pi of the reference's constants
-            cs = (double)cospif((float)(ph * (ec.two_pif / BDB_PI_D)));
+    __device__ __forceinline__ float operator()(float r2) const
+    {
+        const float t = hi * r2, d = fmaf(lo, r2, fmaf(hi, r2, -t));
+        float e;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+        return fmaf(e, d * 0.693147181f, e);
+    }
+};
+
+// Real-space scalars of one image at squared distance r2 (in L^2), its term
+// being A I + B x x^T; ex = exp(-a2 r2). Beenakker's polynomials in r2 have
+// constants of alpha and s2, times 1/sqrt(pi). In FP32 every constant's own
+// rounding would bias all images of all pairs alike (and with them eps, the
+// tensor's mean), so it is carried along as a second FP32 number.
+template <typename T>
+struct Const2 {
+    T hi, lo;
+    __device__ Const2() {}
+    __device__ explicit Const2(double c) : hi((T)c), lo((T)(c - (double)(T)c)) {}
+};
+
+template <typename T>
+struct RealSpace {
+    Const2<T> alpha, e2, as, c0, c1, c2, d0, d1;   // e2: 2 alpha / sqrt(pi); the others times 1/sqrt(pi)
+    T s2, hs, a2;                                  // hs: s2/2
+    bool smith;
+    static constexpr bool kLo = sizeof(T) == 4;
+    __device__ RealSpace(const EwaldConst& ec, double s2d)
+    {
+        const double a = ec.alpha, a3 = a * ec.a2, a5 = a3 * ec.a2, isp = ec.isp;
+        alpha = Const2<T>(a);
+        e2 = Const2<T>(2 * a * isp);
+        as = Const2<T>(a * s2d * isp);
+        c0 = Const2<T>((14 * a3 * s2d - 4.5 * a) * isp);
+        c1 = Const2<T>((3 * a3 - 20 * a5 * s2d) * isp);
+        c2 = Const2<T>(4 * a5 * ec.a2 * s2d * isp);
+        d0 = Const2<T>((1.5 * a - 2 * a3 * s2d) * isp);
+        d1 = Const2<T>((16 * a5 * s2d - 3 * a3) * isp);
+        a2 = (T)ec.a2;
+        s2 = (T)s2d;
+        hs = (T)(0.5 * s2d);
+        smith = ec.smith;
+    }
+    __device__ __forceinline__ void image(T r2, T ex, T& A, T& B) const
+    {
+        const T i = inv_sqrt(r2), i2 = i * i, r = r2 * i;
+        T x = alpha.hi * r;
+        if (kLo) x += alpha.lo * r;
+        const T er = ex * erfcx_pos(x) * i;      // erfc(alpha r)/r
+        if (smith) {
+            T E = e2.hi * ex;
+            if (kLo) E += e2.lo * ex;
+            const T sq = i2 * (er + E);
+            A = (T)0.75 * er + hs * sq;
+            B = ((T)0.75 * (er + E) - hs * (3 * sq + 2 * a2 * E)) * i2;
         } else {
-            cs = cos(ec.two_pif * ph);
+            const T q = s2 * i2, t = as.hi * i2, r4 = c2.hi * r2;
+            T p = t + c0.hi + (c1.hi + r4) * r2, u = d0.hi - 3 * t + (d1.hi - r4) * r2;
+            if (kLo) {
+                p += c0.lo + c1.lo * r2;
+                u += d0.lo + d1.lo * r2;
+            }
+            A = p * ex + er * ((T)0.75 + (T)0.5 * q);
+            B = (u * ex + er * ((T)0.75 - (T)1.5 * q)) * i2;
         }
-        const double sc = (q[3] - sigma_sq * q[4]) * cs;
-        for (int c = 0; c < 6; ++c) Qr[c] += sc * q[5 + c];
     }
-    for (int k = 0; k < 6; ++k) t[k] += preDii * (O[k] + ec.preQ * Qr[k]);
-    if (self) {
-        const double aw = pi.w;
-        const double a = ec.alpha, a3 = ec.alpha3;
-        const double sc3 = (-6 * a / BDB_SQRTPI + 40 * a3 * aw * aw / (3 * BDB_SQRTPI)) * preDii;
-        for (int k = 0; k < 3; ++k) t[k] = preDii / aw + sc3 + t[k];
-        t[3] = t[4] = t[5] = 0;
+};
+
+__device__ __forceinline__ void add_image(double* o, double A, double B, double x, double y, double z)
+{
+    const double bx = B * x, by = B * y;
+    o[0] += A + bx * x;
+    o[1] += A + by * y;
+    o[2] += A + B * z * z;
+    o[3] += bx * y;
+    o[4] += bx * z;
+    o[5] += by * z;
+}
+__device__ __forceinline__ void add_image(float* o, float A, float B, float x, float y, float z)
+{
+    const float bx = B * x, by = B * y, bz = B * z;
+    o[0] += A + bx * x;
+    o[1] += A + by * y;
+    o[2] += A + bz * z;
+    o[3] += bx * y;
+    o[4] += bx * z;
+    o[5] += by * z;
+}
+
+// The lattice sum S(v) over the reference's sphere of images and reciprocal
+// vectors, v = (r_i - r_j)/L as it is (no minimum image). Bound by FP64
+// multiply-adds and their latency (about 90 a image; N = 777, R = 3, Smith:
+// 941 -> 356 us per pass over all pairs, against exp, erfc, two square roots or
+// divisions per image and a cosine per reciprocal vector).
+//
+// FP64: every image of the sphere. An image costs one Gaussian, one erfcx and
+// the rational terms; the Gaussian along a row of images (g = 0, +-1, ...)
+// follows from its neighbour's by two multiplications (exp(-a2 (z+1)^2) =
+// exp(-a2 z^2) rho, rho' = rho kappa), started at g = 0 where it is largest.
+// With MIXED the images are summed in FP32 and those beyond rcut are dropped.
+// Reciprocal space, FP64 in both: the vectors (+-h, +-f, +-g) share their
+// weight up to signs, so their cosines collapse to products of the axes'
+// cosines and sines: 12 weights and 4 products per class of up to 8 vectors,
+// and no cosine beyond one per axis.
+template <bool MIXED>
+__device__ __forceinline__ void lattice_sum(const EwaldConst& ec, const double* v, double s2, double* S)
+{
+    const int R = ec.R;
+    using T = typename std::conditional<MIXED, float, double>::type;
+    T o[6] = {0, 0, 0, 0, 0, 0};
+    const RealSpace<T> rs(ec, s2);
+    if constexpr (MIXED) {
+        const Gauss32 gauss(ec.a2);
+        for (int h = -R; h <= R; ++h) {
+            const float x = (float)v[0] + h;
+            const int nf = ec.extent[h * h];
+            for (int f = -nf; f <= nf; ++f) {
+                const float y = (float)v[1] + f, xy = x * x + y * y;
+                if (xy > ec.rcut_sq) continue;
+                const int ng = ec.extent[h * h + f * f];
+                for (int g = -ng; g <= ng; ++g) {
+                    const float z = (float)v[2] + g, r2 = xy + z * z;
+                    if (r2 == 0.f || r2 > ec.rcut_sq) continue;
+                    float A, B;
+                    rs.image(r2, gauss(r2), A, B);
+                    add_image(o, A, B, x, y, z);
+                }
+            }
+        }
+    } else {
+        const double z0 = v[2];
+        const double up0 = exp(-ec.a2 * (1 + 2 * z0)), down0 = exp(-ec.a2 * (1 - 2 * z0));
+        // a Gaussian that may underflow at g = 0 is taken image by image
+        const bool run = ec.a2 * (R + 2) * (R + 2) < 600.0;
+        for (int h = -R; h <= R; ++h) {
+            const double x = v[0] + h;
+            const int nf = ec.extent[h * h];
+            for (int f = -nf; f <= nf; ++f) {
+                const double y = v[1] + f, xy = x * x + y * y;
+                const int ng = ec.extent[h * h + f * f];
+                const double mid = exp(-ec.a2 * (xy + z0 * z0));
+                for (int dir = 0; dir < 2; ++dir) {
+                    // g = 0, 1, .. ng, then g = -1, .. -ng
+                    double ex = dir ? mid * down0 : mid;
+                    double rho = dir ? down0 * ec.kappa : up0;
+                    const double step = dir ? -1.0 : 1.0;
+                    double z = dir ? z0 - 1.0 : z0;
+                    for (int g = dir; g <= ng; ++g) {
+                        const double r2 = xy + z * z;
+                        if (r2 != 0.0) {
+                            double A, B;
+                            rs.image(r2, run ? ex : exp(-ec.a2 * r2), A, B);
+                            add_image(o, A, B, x, y, z);
+                        }
+                        z += step;
+                        ex *= rho;
+                        rho *= ec.kappa;
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) S[k] = o[k];
+    if (!ec.recip) return;
+    double cx1, sx1, cy1, sy1, cz1, sz1;
+    sincos(ec.two_pif * v[0], &sx1, &cx1);
+    sincos(ec.two_pif * v[1], &sy1, &cy1);
+    sincos(ec.two_pif * v[2], &sz1, &cz1);
+    const double* w = ec.rk;
+    double cx = 1, sx = 0;
+    for (int h = 0; h <= R; ++h) {
+        double cy = 1, sy = 0;
+        const int nf = ec.extent[h * h];
+        for (int f = 0; f <= nf; ++f) {
+            double q[6] = {0, 0, 0, 0, 0, 0};
+            double cz = 1, sz = 0;
+            const int ng = ec.extent[h * h + f * f];
+            for (int g = 0; g <= ng; ++g, w += 12) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) q[k] += (w[k] + s2 * w[6 + k]) * (k < 4 ? cz : sz);
+                const double c = cz * cz1 - sz * sz1;
+                sz = sz * cz1 + cz * sz1;
+                cz = c;
+            }
+            const double cc = cx * cy;
+            S[0] += cc * q[0];
+            S[1] += cc * q[1];
+            S[2] += cc * q[2];
+            S[3] += sx * sy * q[3];
+            S[4] += sx * cy * q[4];
+            S[5] += cx * sy * q[5];
+            const double c = cy * cy1 - sy * sy1;
+            sy = sy * cy1 + cy * sy1;
+            cy = c;
+        }
+        const double c = cx * cx1 - sx * sx1;
+        sx = sx * cx1 + cx * sx1;
+        cx = c;
     }
 }
 
-// diff_tensor_calc_ewald_smith(i, j) (+ _diag for i == j) from the lattice
-// tables. The FP64 path keeps every real-space image; with MIXED the
-// real-space images are summed in FP32 (images beyond 4.45/alpha dropped,
-// 2.5 L at the default alpha = sqrt(pi): erfc there is below 3e-10) and the
-// reciprocal phases taken as FP32 cosines of the same argument, both
-// accumulated in FP64.
-template <bool MIXED>
-__device__ __forceinline__ void rpy_smith_tab(const double4& pi, const double4& pj, bool self, double preDii,
-                                              double preDij, const EwaldConst& ec, double* t)
+// The self tile of a bead of radius a (diagonal, isotropic): its own term,
+// the method's self correction and its images.
+__device__ __forceinline__ double ewald_self(const EwaldConst& ec, double a, double preDii)
 {
-    const double sigma_i = pj.w, sigma_j = pi.w;
-    // dist_vec(coord_j, coord_i): v = r_i - r_j, no minimum image
-    const double r0 = pi.x - pj.x, r1 = pi.y - pj.y, r2 = pi.z - pj.z;
-    const double sigma_sq = 0.5 * (sigma_i * sigma_i + sigma_j * sigma_j);
-    const double preO = 0.75 * ec.inv_L;
-    const double preQ = 0.5 * sigma_sq * ec.inv_L * ec.inv_L * ec.inv_L;
-    for (int k = 0; k < 6; ++k) t[k] = 0;
-    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-    const double rr = r0 * r0 + r1 * r1 + r2 * r2;
-    if (!self && rr < (sigma_i + sigma_j) * (sigma_i + sigma_j)) {
-        const double r = sqrt(rr), inv = 1 / r;
-        const double e[3] = {r0 * inv, r1 * inv, r2 * inv};
-        const double sigma = (sigma_i + sigma_j) / 2;
-        const double pre = preDii / sigma;
-        const double part1 = 1 - (9 * r / (32 * sigma));
-        const double pre2 = preDij / r;
-        const double sigm_r = (sigma_i * sigma_i + sigma_j * sigma_j) / rr;
-        const double p1 = 1 + sigm_r / 3;
-        for (int k = 0; k < 3; ++k)
-            t[k] += pre * (part1 + 3 * e[k] * e[k] * r / (32 * sigma)) - pre2 * (p1 + e[k] * e[k] * (1 - sigm_r));
-        for (int k = 3; k < 6; ++k)
-            t[k] += pre * 3 * e[ia[k]] * e[ib[k]] * r / (32 * sigma) - pre2 * e[ia[k]] * e[ib[k]] * (1 - sigm_r);
+    const double il = ec.inv_L, a3 = ec.alpha * ec.a2, q = a * il;
+    double sc;
+    if (ec.smith) {
+        sc = ec.alpha * a * il;
+        sc = sc * sc * sc * BDB_M1_SQRTPI / 3;
+        sc = -(0.75 * il * 1.5 * ec.alpha * a * BDB_M1_SQRTPI * il + 0.5 * a * a * il * il * il * sc);
+    } else {
+        sc = (-6 * ec.alpha + 40 * a3 * q * q / 3) / BDB_SQRTPI * il;
     }
-    const double v0 = r0 * ec.inv_L, v1 = r1 * ec.inv_L, v2 = r2 * ec.inv_L;
-    const double a = ec.s_alpha, a2 = ec.s_alpha2, a3 = ec.s_alpha3;
-    double O[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0};
-    // real space: images v + m (m from the image table, stored as L m)
-    if (MIXED) {
-        const float fa = (float)a, fa2 = (float)a2, fa3 = (float)a3, isp = (float)BDB_M1_SQRTPI;
-        const float fx = (float)v0, fy = (float)v1, fz = (float)v2;
-        float o[6] = {0, 0, 0, 0, 0, 0}, qq[6] = {0, 0, 0, 0, 0, 0};
-        for (int m = 0; m < ec.nimg; ++m) {
-            const double4 off = ec.img[m];
-            const float x = fx + (float)rint(off.x * ec.inv_L), y = fy + (float)rint(off.y * ec.inv_L),
-                        z = fz + (float)rint(off.z * ec.inv_L);
-            const float r_sq = x * x + y * y + z * z;
-            if (r_sq == 0.f || r_sq > ec.s_rcut_sq) continue;
-            const float inv_r = rsqrtf(r_sq), r = r_sq * inv_r, inv_r3 = inv_r * inv_r * inv_r;
-            const float e0 = x * inv_r, e1 = y * inv_r, e2 = z * inv_r;
-            const float er = erfcf(r * fa), ex = __expf(-fa2 * r_sq);
-            const float so = er * inv_r, so2 = so + 2.f * fa * isp * ex;
-            const float sq = inv_r3 * (er + 2.f * fa * r * isp * ex);
-            const float sq2 = -3.f * sq - 4.f * fa3 * isp * ex;
-            o[0] += so + so2 * e0 * e0;
-            o[1] += so + so2 * e1 * e1;
-            o[2] += so + so2 * e2 * e2;
-            o[3] += so2 * e0 * e1;
-            o[4] += so2 * e0 * e2;
-            o[5] += so2 * e1 * e2;
-            qq[0] += sq + sq2 * e0 * e0;
-            qq[1] += sq + sq2 * e1 * e1;
-            qq[2] += sq + sq2 * e2 * e2;
-            qq[3] += sq2 * e0 * e1;
-            qq[4] += sq2 * e0 * e2;
-            qq[5] += sq2 * e1 * e2;
-        }
-        for (int k = 0; k < 6; ++k) {
-            O[k] = o[k];
-            Q[k] = qq[k];
-        }
-    }
-    for (int m = 0; !MIXED && m < ec.nimg; ++m) {
-        const double4 off = ec.img[m];
-        const double x = v0 + rint(off.x * ec.inv_L), y = v1 + rint(off.y * ec.inv_L), z = v2 + rint(off.z * ec.inv_L);
-        const double r_sq = x * x + y * y + z * z;
-        if (r_sq == 0.0) continue;
-        const double r = sqrt(r_sq);
-        const double inv_r = 1 / r, inv_r3 = 1 / (r * r_sq);
-        const double e[3] = {x * inv_r, y * inv_r, z * inv_r};
-        const double er = erfc(r * a), ex = exp(-a2 * r_sq);
-        const double so = er * inv_r, so2 = so + 2 * a * BDB_M1_SQRTPI * ex;
-        const double sq = inv_r3 * (er + 2 * a * r * BDB_M1_SQRTPI * ex);
-        const double sq2 = -3 * sq - 4 * a3 * BDB_M1_SQRTPI * ex;
-        for (int k = 0; k < 3; ++k) {
-            O[k] += so + so2 * e[k] * e[k];
-            Q[k] += sq + sq2 * e[k] * e[k];
-        }
-        for (int k = 3; k < 6; ++k) {
-            O[k] += so2 * e[ia[k]] * e[ib[k]];
-            Q[k] += sq2 * e[ia[k]] * e[ib[k]];
-        }
-    }
-    // reciprocal space: one row per pair k, -k
-    double Rc[6] = {0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < ec.nk; ++k) {
-        const double* q = ec.rk + 12 * k;
-        const double ph = v0 * q[0] + v1 * q[1] + v2 * q[2];
-        // cos(2 pi_f ph), pi_f the float pi of the reference's constants
-        const double cs = MIXED ? (double)cospif((float)(ph * (ec.two_pif / BDB_PI_D))) : cos(ec.two_pif * ph);
-        const double ci = q[3] * cs, ce = (q[4] + sigma_sq * q[5]) * cs;
-        for (int c = 0; c < 3; ++c) Rc[c] += ci + ce * q[6 + c];
-        for (int c = 3; c < 6; ++c) Rc[c] += ce * q[6 + c];
-    }
-    for (int k = 0; k < 6; ++k) t[k] += preDii * (preO * O[k] + preQ * Q[k] + Rc[k]);
+    return preDii / a + sc * preDii + preDii * (il * (ec.self0 + ec.self1 * q * q));
+}
+
+// diff_tensor_calc_ewald_* (i, j), and _diag for i == j
+template <bool MIXED>
+__device__ __forceinline__ void rpy_ewald(const double4& pi, const double4& pj, bool self, double preDii,
+                                          double preDij, const EwaldConst& ec, double* t)
+{
     if (self) {
-        const double aw = pi.w, il = ec.inv_L;
-        double sc3 = a * aw * il;
-        sc3 = sc3 * sc3 * sc3 * BDB_M1_SQRTPI / 3;
-        sc3 = 0.75 * il * 1.5 * a * aw * BDB_M1_SQRTPI * il + 0.5 * aw * aw * il * il * il * sc3;
-        sc3 *= preDii;
-        for (int k = 0; k < 3; ++k) t[k] = preDii / aw - sc3 + t[k];
+        t[0] = t[1] = t[2] = ewald_self(ec, pi.w, preDii);
         t[3] = t[4] = t[5] = 0;
+        return;
     }
+    const double r0 = pi.x - pj.x, r1 = pi.y - pj.y, r2 = pi.z - pj.z;
+    const double sum = pi.w + pj.w, ss = pi.w * pi.w + pj.w * pj.w;
+    for (int k = 0; k < 6; ++k) t[k] = 0;
+    const double rr = r0 * r0 + r1 * r1 + r2 * r2;
+    if (rr < sum * sum) {
+        // the overlap form in place of the far field
+        const double r = sqrt(rr), inv = 1 / r, sigma = sum / 2;
+        const double pre = preDii / sigma, q = r / (32 * sigma), pre2 = preDij * inv, sr = ss / rr;
+        const double A = pre * (1 - 9 * q) - pre2 * (1 + sr / 3), B = pre * 3 * q - pre2 * (1 - sr);
+        const double e[3] = {r0 * inv, r1 * inv, r2 * inv};
+        t[0] = A + B * e[0] * e[0];
+        t[1] = A + B * e[1] * e[1];
+        t[2] = A + B * e[2] * e[2];
+        t[3] = B * e[0] * e[1];
+        t[4] = B * e[0] * e[2];
+        t[5] = B * e[1] * e[2];
+    }
+    const double v[3] = {r0 * ec.inv_L, r1 * ec.inv_L, r2 * ec.inv_L};
+    double S[6];
+    lattice_sum<MIXED>(ec, v, 0.5 * ss * ec.inv_L * ec.inv_L, S);
+    const double pre = preDii * ec.inv_L;
+    for (int k = 0; k < 6; ++k) t[k] += pre * S[k];
 }
 
 }  // namespace bdb

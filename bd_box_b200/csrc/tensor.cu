@@ -1,6 +1,6 @@
 // Diffusion tensor on the device.
 //
-// 1. k_build: the stored 3N x 3N tensor of compute_D (diff_tensor.c:472-544)
+// k_build: the stored 3N x 3N tensor of compute_D (diff_tensor.c:472-544)
 //    for the Cholesky path. One CTA per 32x32-bead tile (I >= J) evaluates
 //    the 1024 RPY tiles into shared memory and writes the 96x96 block twice
 //    with coalesced rows: as rows of block (I, J) below the diagonal and,
@@ -8,16 +8,7 @@
 //    The factorisation later overwrites the lower triangle with L; the upper
 //    triangle keeps D (the reference keeps Ds and S separately,
 //    diff_rand.c:76-82). The diagonal of D goes to dD.
-// 2. k_tea: matrix-free D.F (compute_Rf_geyer_in_fly, diff_equation.c:55-117)
-//    and the Geyer-Winter sums C_i, Feff_i, eps (compute_r DIFF_GEYER,
-//    diff_rand.c:86-196) in one pass over tile pairs (I >= J): every bead
-//    pair is evaluated once, staged in shared memory, and summed by rows
-//    (into bead i) and by columns (into bead j). Per (tile, bead) partials
-//    go to a scratch buffer that k_tea_finish reduces in a fixed order, so
-//    the result does not depend on scheduling.
-// 3. k_eps_beta + k_tea_finish: eps -> beta (diff_rand.c:197-217), the TEA
-//    displacement (:219-228) and the position update with the periodic wrap
-//    (compute_hydro_ermak, diff_equation.c:254-264), fused.
+// The matrix-free pair sums (D.F, TEA noise) are in tea.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,86 +16,303 @@
 #include <vector>
 
 #include "bdb_common.cuh"
-#include "rpy_tile.cuh"
+#include "ewald_fast.cuh"
+#include "tensor_args.cuh"
 
 namespace bdb {
 
 static constexpr int TB = 32;   // beads per tile
 
-struct TensorArgs {
-    int n, npad;
-    double preDii, preDij;
-    int ewald;
-    EwaldConst ec;
-};
-
-// Lattice tables of the Ewald sums (see EwaldConst), built once per system
-// in the order diff_tensor_calc_ewald_beenakker walks the sphere |m|^2 <= R^2
-// (diff_tensor.c:319-326); the k-only factors of the reciprocal term are
-// evaluated as the device evaluates them per pair.
+// Constants of a system's Ewald sums (no device data).
 static EwaldConst system_ewald(const bdb_system* s)
 {
-    if (s->p.ewald_method == BDB_EWALD_SMITH)
-        return make_ewald_smith(s->p.box[0], s->inv_L[0], s->p.ewald_real,
-                                s->p.ewald_alpha > 0 ? s->p.ewald_alpha : BDB_SQRTPI);
-    return make_ewald(s->p.box[0], s->inv_L[0], s->p.ewald_real);
+    EwaldConst e;
+    if (!s->p.ewald) return e;
+    e.smith = s->p.ewald_method == BDB_EWALD_SMITH;
+    e.R = s->p.ewald_real;
+    e.L = s->p.box[0];
+    e.inv_L = s->inv_L[0];
+    e.alpha = e.smith && s->p.ewald_alpha > 0 ? s->p.ewald_alpha : BDB_SQRTPI;
+    e.a2 = e.alpha * e.alpha;
+    e.isp = e.smith ? BDB_M1_SQRTPI : 1 / BDB_SQRTPI;
+    volatile float pif = BDB_M_PIF;
+    volatile float two = 2 * pif;
+    e.two_pif = two;
+    e.kappa = std::exp(-2 * e.a2);
+    for (int q = 0; q <= e.R * e.R; ++q) e.extent[q] = (signed char)std::sqrt((double)(e.R * e.R - q));
+    // images beyond 2.5 L (Beenakker), 4.45/alpha (Smith): erfc ~ 3e-10
+    const double rc = e.smith ? 4.45 / e.alpha : 2.5;
+    e.rcut_sq = (float)(rc * rc);
+    return e;
 }
 
-static int ewald_tables(bdb_system* s)
+// the reciprocal weights I and e e^T of a vector of |k|^2 = k_sq: {I, ee} and
+// the same of the terms in s2. The k-only factors are the reference's
+// (diff_tensor.c:360-395, :206-239), with its float constants; Beenakker's
+// k^2/alpha^2 is formed there as (2 pi_f k)^2 over alpha^2 = pi/L^2, which
+// leaves weights of exp(-pi L^2 k^2): zero for boxes above ~15.
+static void recip_weights(const EwaldConst& ec, double k_sq, double* w)
+{
+    volatile float pif = BDB_M_PIF;
+    if (ec.smith) {
+        volatile float npif2 = -pif * pif;
+        volatile float four_pif = 4 * pif;
+        const double m = (double)npif2 / ec.a2 * k_sq;
+        const double ex = std::exp(m);
+        const double A = 2 * ex / ((double)pif * k_sq);
+        w[0] = 0.75 * A;
+        w[1] = 0.75 * A * (-1 + m);
+        w[2] = 0;
+        w[3] = 0.5 * (double)four_pif * ex;
+    } else {
+        volatile float four = 4 * pif;
+        volatile float four2 = four * pif;
+        volatile float six = 6 * pif;
+        const double k2 = k_sq * (double)four2;
+        const double alpha = ec.alpha * ec.inv_L, ia2 = 1.0f / (alpha * alpha);
+        double P = 1 + (ia2 * k2 / 4) * (1 + ia2 * k2 / 2);
+        P *= (double)six * std::exp(-ia2 * k2 / 4) / k2;
+        w[0] = P * ec.inv_L * ec.inv_L;
+        w[1] = -w[0];
+        w[2] = -k2 / 3 * P;
+        w[3] = -w[2];
+    }
+}
+
+// Real-space scalars of an image (RealSpace::image) on the host, the parts
+// without and with s2: A0, B0, A1, B1
+static void real_scalars(const EwaldConst& ec, double r2, double* q)
+{
+    const double a = ec.alpha, a3 = a * ec.a2, a5 = a3 * ec.a2, a7 = a5 * ec.a2;
+    const double r = std::sqrt(r2), i = 1 / r, i2 = 1 / r2;
+    const double ex = std::exp(-ec.a2 * r2), er = std::erfc(a * r) * i;
+    if (ec.smith) {
+        const double E = 2 * a * ec.isp * ex, sq = i2 * (er + E);
+        q[0] = 0.75 * er;
+        q[1] = 0.75 * (er + E) * i2;
+        q[2] = 0.5 * sq;
+        q[3] = 0.5 * (-3 * sq - 2 * ec.a2 * E) * i2;
+    } else {
+        const double g = ec.isp * ex;
+        q[0] = (-4.5 * a + 3 * a3 * r2) * g + 0.75 * er;
+        q[1] = ((1.5 * a - 3 * a3 * r2) * g + 0.75 * er) * i2;
+        q[2] = (a * i2 + 14 * a3 - 20 * a5 * r2 + 4 * a7 * r2 * r2) * g + 0.5 * er * i2;
+        q[3] = ((-3 * a * i2 - 2 * a3 + 16 * a5 * r2 - 4 * a7 * r2 * r2) * g - 1.5 * er * i2) * i2;
+    }
+}
+
+// S(v) of the reference on the host, v in L (raw), s2 = sigma^2/L^2: the
+// sphere of images and the reciprocal sum
+static void reference_sum(const EwaldConst& ec, const double* v, double s2, double* S)
+{
+    const int R = ec.R;
+    for (int k = 0; k < 6; ++k) S[k] = 0;
+    for (int h = -R; h <= R; ++h)
+        for (int f = -R; f <= R; ++f)
+            for (int g = -R; g <= R; ++g) {
+                const int m2 = h * h + f * f + g * g;
+                if (m2 > R * R) continue;
+                const double x[3] = {v[0] + h, v[1] + f, v[2] + g};
+                double q[4], A = 0, B = 0;
+                real_scalars(ec, x[0] * x[0] + x[1] * x[1] + x[2] * x[2], q);
+                A = q[0] + s2 * q[2];
+                B = q[1] + s2 * q[3];
+                S[0] += A + B * x[0] * x[0];
+                S[1] += A + B * x[1] * x[1];
+                S[2] += A + B * x[2] * x[2];
+                S[3] += B * x[0] * x[1];
+                S[4] += B * x[0] * x[2];
+                S[5] += B * x[1] * x[2];
+                if (m2 == 0) continue;
+                recip_weights(ec, m2, q);
+                const double cs = std::cos(ec.two_pif * (v[0] * h + v[1] * f + v[2] * g));
+                const double ci = (q[0] + s2 * q[2]) * cs, ce = (q[1] + s2 * q[3]) * cs / m2;
+                S[0] += ci + ce * h * h;
+                S[1] += ci + ce * f * f;
+                S[2] += ci + ce * g * g;
+                S[3] += ce * h * f;
+                S[4] += ce * h * g;
+                S[5] += ce * f * g;
+            }
+}
+
+// Fourier weights {I, ee} at |k|^2 = k_sq of the converged split (see
+// ewald_fast.cuh), on top of the near part
+static void fast_weights(const EwaldConst& ec, double k_sq, double s2, double* w)
+{
+    const double b = EF_SPLIT * BDB_SQRTPI, y = BDB_PI_D * BDB_PI_D * k_sq / (b * b), ex = std::exp(-y);
+    w[0] = 1.5 * ex / (BDB_PI_D * k_sq);
+    w[1] = -w[0] * (1 + y) + 2 * BDB_PI_D * s2 * ex;
+    if (ec.smith) return;
+    // Beenakker's screening of the same tensor at alpha = sqrt(pi)/L, whose
+    // real-space sum the reference takes, and the reference's reciprocal sum
+    const double k2 = 4 * BDB_PI_D * BDB_PI_D * k_sq, x = k2 / (4 * ec.a2);
+    const double P = (1 + x + 2 * x * x) * 6 * BDB_PI_D * std::exp(-x) / k2 * (1 - s2 * k2 / 3);
+    w[0] -= P;
+    w[1] += P;
+    if (k_sq <= ec.R * ec.R) {
+        double q[4];
+        recip_weights(ec, k_sq, q);
+        w[0] += q[0] + s2 * q[2];
+        w[1] += q[1] + s2 * q[3];
+    }
+}
+
+// The converged split for a mixed system, or nothing (false) where the
+// reference's truncated sums differ from it. The sphere of images truncates
+// first for separations far apart in the box, so the two are compared there:
+// at |v| = 1.5 and within (they must agree to 2e-7 in preDii/L, where the tile
+// is ~1 and its FP32 rounding in the reference's split ~7e-7), then in the
+// box's corners, without which the split covers |v| <= 1.5 only. At the
+// default alpha, Beenakker: 2.4e-8 at R = 4 within 1.5 (1e-5 in the
+// corners), 2.5e-4 at R = 3.
+static bool ewald_fast_setup(const bdb_system* s, EwaldFast* E)
+{
+    const EwaldConst ec = system_ewald(s);
+    const double a = s->radius0, s2 = a * a * ec.inv_L * ec.inv_L, b = EF_SPLIT * BDB_SQRTPI;
+    if (!(s2 < 0.25)) return false;
+    static const double pt[10][3] = {{0.31, 0.17, 0.23},   {0.49, 0.48, 0.47},    {0.97, 0.03, 0.99}, {0.07, 0.04, 0.09},
+                                     {0.97, 0.81, -0.81},  {-0.99, -0.99, 0.53},  {0.866, 0.866, 0.866},
+                                     {0.96, -0.97, 0.98},  {-0.995, -0.99, 0.999}, {0.99, 0.98, -0.7}};
+    static const int corner0 = 7;   // the last three lie beyond 1.5
+    double dev[10][6], C = 0;
+    std::vector<double> w;
+    for (int h = 0; h <= EF_K; ++h)
+        for (int f = 0; f <= EF_K; ++f)
+            for (int g = 0; g <= EF_K; ++g) {
+                const int m2 = h * h + f * f + g * g;
+                if (m2 > EF_K2) continue;
+                double q[6] = {0, 0, 0, 0, 0, 0}, c[2];
+                if (m2) {
+                    const double mult = (h ? 2.0 : 1.0) * (f ? 2.0 : 1.0) * (g ? 2.0 : 1.0);
+                    fast_weights(ec, m2, s2, c);
+                    q[0] = mult * (c[0] + c[1] * h * h / m2);
+                    q[1] = mult * (c[0] + c[1] * f * f / m2);
+                    q[2] = mult * (c[0] + c[1] * g * g / m2);
+                    q[3] = -mult * c[1] * h * f / m2;
+                    q[4] = -mult * c[1] * h * g / m2;
+                    q[5] = -mult * c[1] * f * g / m2;
+                }
+                w.insert(w.end(), q, q + 6);
+            }
+    EwaldConst near;   // Smith's real-space functions at the split's screening
+    near.smith = 1;
+    near.alpha = b;
+    near.a2 = b * b;
+    near.isp = 1 / BDB_SQRTPI;
+    for (int p = 0; p < 10; ++p) {
+        double S[6], o[6] = {0, 0, 0, 0, 0, 0}, u[3], sg[3];
+        reference_sum(ec, pt[p], s2, S);
+        for (int k = 0; k < 3; ++k) {
+            u[k] = pt[p][k] - std::rint(pt[p][k]);
+            sg[k] = u[k] < 0 ? -1 : 1;
+            u[k] = std::fabs(u[k]);
+        }
+        for (int m = 0; m < 8; ++m) {
+            const double x[3] = {u[0] - (m & 1), u[1] - ((m >> 1) & 1), u[2] - (m >> 2)};
+            double q[4];
+            real_scalars(near, x[0] * x[0] + x[1] * x[1] + x[2] * x[2], q);
+            const double A = q[0] + s2 * q[2], B = q[1] + s2 * q[3];
+            for (int k = 0; k < 3; ++k) o[k] += A + B * x[k] * x[k];
+            o[3] += B * x[0] * x[1];
+            o[4] += B * x[0] * x[2];
+            o[5] += B * x[1] * x[2];
+        }
+        size_t n = 0;
+        const double tp = 2 * BDB_PI_D;
+        for (int h = 0; h <= EF_K; ++h)
+            for (int f = 0; f <= EF_K; ++f)
+                for (int g = 0; g <= EF_K; ++g) {
+                    if (h * h + f * f + g * g > EF_K2) continue;
+                    const double cx = std::cos(tp * h * u[0]), sx = std::sin(tp * h * u[0]), cy = std::cos(tp * f * u[1]),
+                                 sy = std::sin(tp * f * u[1]), cz = std::cos(tp * g * u[2]), sz = std::sin(tp * g * u[2]);
+                    const double* q = &w[n];
+                    for (int k = 0; k < 3; ++k) o[k] += q[k] * cx * cy * cz;
+                    o[3] += q[3] * sx * sy * cz;
+                    o[4] += q[4] * sx * cy * sz;
+                    o[5] += q[5] * cx * sy * sz;
+                    n += 6;
+                }
+        o[3] *= sg[0] * sg[1];
+        o[4] *= sg[0] * sg[2];
+        o[5] *= sg[1] * sg[2];
+        for (int k = 0; k < 6; ++k) dev[p][k] = S[k] - o[k];
+        for (int k = 0; k < 3 && p < corner0; ++k) C += dev[p][k] / (3 * corner0);
+    }
+    bool corners = true;
+    for (int p = 0; p < 10; ++p)
+        for (int k = 0; k < 6; ++k)
+            if (!(std::fabs(dev[p][k] - (k < 3 ? C : 0.0)) < 2e-7)) {
+                if (p < corner0) return false;
+                corners = false;
+            }
+    for (size_t q = 0; q < w.size(); ++q) E->w[q / 6][q % 6] = (float)w[q];
+    E->beta = (float)b;
+    E->b2 = (float)(b * b);
+    E->e2 = (float)(2 * b / BDB_SQRTPI);
+    E->hs = (float)(0.5 * s2);
+    E->diag = (float)C;
+    E->radius = (float)a;
+    const Gauss32 gauss(b * b);
+    E->g_hi = gauss.hi;
+    E->g_lo = gauss.lo;
+    E->near_sq = (float)(4 * s2);
+    E->far_sq = corners ? 3.01f : 2.25f;
+    E->pre = (float)(s->preDii * ec.inv_L);
+    return true;
+}
+
+// The reciprocal weight table and a bead's sum over its own images, once per
+// system (see EwaldConst)
+int ewald_tables(bdb_system* s)
 {
     if (!s->p.ewald || s->ewald_tab.p) return BDB_OK;
     const EwaldConst ec = system_ewald(s);
-    // Smith's k-only factors (diff_tensor.c:206-239 with init_tensor's
-    // M_PI_ALPHA_SQ = -pi_f^2/alpha^2, pi_f^2 formed in float)
-    volatile float pif = BDB_M_PIF;
-    volatile float npif2 = -pif * pif;
-    volatile float four_pif = 4 * pif;
-    const double m_pi_alpha_sq = ec.smith ? (double)npif2 / ec.s_alpha2 : 0.0;
-    const double preO = 0.75 * ec.inv_L;
-    const double qL3 = ec.inv_L * ec.inv_L * ec.inv_L;
-    std::vector<double> rk, img;
     const int R = ec.R;
-    for (int h = -R; h <= R; ++h) {
-        const int nf = (int)std::sqrt((double)(ec.rr_sq - h * h));
-        for (int f = -nf; f <= nf; ++f) {
-            const int ng = (int)std::sqrt((double)(ec.rr_sq - h * h - f * f));
-            for (int g = -ng; g <= ng; ++g) {
-                img.insert(img.end(), {ec.L * h, ec.L * f, ec.L * g, 0.0});
-                const bool half = h > 0 || (h == 0 && (f > 0 || (f == 0 && g > 0)));
-                if (!half) continue;
+    std::vector<double> rk;
+    double self0 = 0, self1 = 0;
+    bool any = false;
+    for (int h = 0; h <= R; ++h)
+        for (int f = 0; f <= ec.extent[h * h]; ++f)
+            for (int g = 0; g <= ec.extent[h * h + f * f]; ++g) {
+                double w[12] = {0};
                 const double k_sq = (double)(h * h + f * f + g * g);
-                const double kn = std::sqrt(k_sq), ik = 1 / kn;
-                const double e[3] = {h * ik, f * ik, g * ik};
-                if (ec.smith) {
-                    // Op: A (I + (m k^2 - 1) e e^T), Qp: C e e^T, both times cos;
-                    // k and -k together: 2x
-                    const double ex = std::exp(m_pi_alpha_sq * k_sq);
-                    const double A = 2 * ex / ((double)pif * k_sq);
-                    const double C = (double)four_pif * ex;
-                    rk.insert(rk.end(), {(double)h, (double)f, (double)g, 2 * preO * A,
-                                         2 * preO * A * (-1 + m_pi_alpha_sq * k_sq), 2 * 0.5 * qL3 * C,
-                                         e[0] * e[0], e[1] * e[1], e[2] * e[2], e[0] * e[1], e[0] * e[2], e[1] * e[2]});
-                    continue;
+                if (k_sq > 0) {
+                    const double mult = (h ? 2.0 : 1.0) * (f ? 2.0 : 1.0) * (g ? 2.0 : 1.0);
+                    const double ik = 1 / std::sqrt(k_sq), e[3] = {h * ik, f * ik, g * ik};
+                    double c[4];
+                    recip_weights(ec, k_sq, c);
+                    for (int q = 0; q < 2; ++q) {
+                        for (int k = 0; k < 3; ++k) w[6 * q + k] = mult * (c[2 * q] + c[2 * q + 1] * e[k] * e[k]);
+                        // cos of a sum with both signs of two axes: -sin sin
+                        w[6 * q + 3] = -mult * c[2 * q + 1] * e[0] * e[1];
+                        w[6 * q + 4] = -mult * c[2 * q + 1] * e[0] * e[2];
+                        w[6 * q + 5] = -mult * c[2 * q + 1] * e[1] * e[2];
+                    }
+                    self0 += w[0];
+                    self1 += w[6];
+                    // the sphere's images of a bead itself: mean of the three axes
+                    double q[4];
+                    real_scalars(ec, k_sq, q);
+                    self0 += mult * (q[0] + q[1] * h * h);
+                    self1 += mult * (q[2] + q[3] * h * h);
                 }
-                const double k2 = k_sq * ec.four_pif2;
-                double P = 1 + (ec.inv_alpha2 * k2 / 4) * (1 + ec.inv_alpha2 * k2 / 2);
-                P *= ec.six_pif * std::exp(-ec.inv_alpha2 * k2 / 4) / k2;
-                rk.insert(rk.end(), {(double)h, (double)f, (double)g, P, k2 / 3 * P, 2 * (1 - e[0] * e[0]),
-                                     2 * (1 - e[1] * e[1]), 2 * (1 - e[2] * e[2]), -2 * e[0] * e[1], -2 * e[0] * e[2],
-                                     -2 * e[1] * e[2], 0.0});
+                for (double x : w) any = any || x != 0.0;
+                rk.insert(rk.end(), w, w + 12);
             }
-        }
+    if (s->ewald_tab.alloc(rk.size())) return BDB_ERR_NOMEM;
+    BDB_CUDA(h2d(s, s->ewald_tab.p, rk.data(), sizeof(double) * rk.size()));
+    s->ewald_self[0] = self0;
+    s->ewald_self[1] = self1;
+    s->ewald_recip = any;
+    if (s->p.precision != BDB_PREC_FP64) {
+        s->ewald_fast = std::make_shared<EwaldFast>();
+        if (!ewald_fast_setup(s, s->ewald_fast.get())) s->ewald_fast.reset();
     }
-    s->ewald_nk = (int)(rk.size() / 12);
-    s->ewald_nimg = (int)(img.size() / 4);
-    if (s->ewald_tab.alloc(rk.size() + img.size())) return BDB_ERR_NOMEM;
-    if (!rk.empty())
-        BDB_CUDA(h2d(s, s->ewald_tab.p, rk.data(), sizeof(double) * rk.size()));
-    BDB_CUDA(h2d(s, s->ewald_tab.p + rk.size(), img.data(), sizeof(double) * img.size()));
     return BDB_OK;
 }
 
-static TensorArgs targs(const bdb_system* s)
+TensorArgs targs(const bdb_system* s)
 {
     TensorArgs a;
     a.n = s->n;
@@ -113,46 +321,11 @@ static TensorArgs targs(const bdb_system* s)
     a.preDij = s->preDij;
     a.ewald = s->p.ewald;
     a.ec = system_ewald(s);
-    if (s->p.ewald) {
-        a.ec.rk = s->ewald_tab.p;
-        a.ec.nk = s->ewald_nk;
-        a.ec.img = reinterpret_cast<const double4*>(s->ewald_tab.p + 12 * (size_t)s->ewald_nk);
-        a.ec.nimg = s->ewald_nimg;
-        const double rc = 2.5 * s->p.box[0];   // erfc(2.5 sqrt(pi)) ~ 3e-10
-        a.ec.rcut_sq = (float)(rc * rc);
-    }
+    a.ec.rk = s->ewald_tab.p;
+    a.ec.recip = s->ewald_recip;
+    a.ec.self0 = s->ewald_self[0];
+    a.ec.self1 = s->ewald_self[1];
     return a;
-}
-
-template <typename T, bool kEwald>
-__device__ __forceinline__ void tile_of_k(const TensorArgs& A, const double4* pos, int i, int j, T* t)
-{
-    const double4 pi = pos[i], pj = pos[j];
-    if constexpr (kEwald) {
-        double d[6];
-        if (A.ec.smith)
-            rpy_smith_tab<sizeof(T) == 4>(pi, pj, i == j, A.preDii, A.preDij, A.ec, d);
-        else
-            rpy_ewald_tab<sizeof(T) == 4>(pi, pj, i == j, A.preDii, A.preDij, A.ec, d);
-        for (int k = 0; k < 6; ++k) t[k] = (T)d[k];
-    } else if (i == j) {
-        const T d = (T)(A.preDii / pi.w);
-        t[0] = t[1] = t[2] = d;
-        t[3] = t[4] = t[5] = 0;
-    } else if (i > j) {
-        rpy_free<T>(pi, pj, (T)A.preDii, (T)A.preDij, t);
-    } else {
-        rpy_free<T>(pj, pi, (T)A.preDii, (T)A.preDij, t);
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void tile_of(const TensorArgs& A, const double4* pos, int i, int j, T* t)
-{
-    if (A.ewald)
-        tile_of_k<T, true>(A, pos, i, j, t);
-    else
-        tile_of_k<T, false>(A, pos, i, j, t);
 }
 
 // One CTA per pair of 32-bead blocks (I >= J): the 96x96 tile of D in
@@ -266,362 +439,6 @@ int tensor_tile_host(bdb_system* s, int i, int j, double* tD)
     BDB_CUDA(cudaGetLastError());
     BDB_CUDA(cudaMemcpyAsync(tD, d, 9 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     BDB_CUDA(cudaStreamSynchronize(s->stream));
-    return BDB_OK;
-}
-
-// ------------------------------------------------------------------ TEA
-
-// part layout: record (9 doubles: Rf[3], C[3], Feff[3]) for (tile_other T,
-// bead b) of segment g at index  g.part_begin + T * g.count + (b - g.begin).
-struct TeaSeg {
-    int begin, count, ntile, part_begin;
-};
-
-// One job = the tile pair (I, J) of a segment (TT x TT beads). Warp w holds
-// rows li of the pair (32 / TT rows at a time, one lane per column lj); each
-// lane evaluates its tile D_ij in registers and uses it twice: in the row
-// sums of bead i (a shuffle tree over the row's lanes) and in the column
-// sums of bead j (accumulated by the lane over the rows it visits, then the
-// warps' partials added in warp order through shared memory). The tiles never
-// go through shared memory. Within a job the sums run in T (FP32 on the mixed
-// path); the records they produce and every sum across jobs are FP64. The
-// free-space variant (kEwald false) carries none of the lattice-sum code.
-// The grid is persistent, as many CTAs as the SMs hold: each CTA takes the
-// next job of the whole batch (every replica's tile pairs in one list) from
-// a counter until none is left -- fetching its next job while it works on
-// the current one -- so replicas of uneven size share the GPU in one launch
-// and a CTA that drew short jobs draws more. A job writes only its own
-// records, so which CTA runs it does not change a bit.
-template <typename T, int TT, bool kEwald>
-__global__ void __launch_bounds__(256)
-k_tea(TensorArgs A, const TileJob* __restrict__ jobs, int n_jobs, int* __restrict__ next,
-      const TeaSeg* __restrict__ segs, const double4* __restrict__ pos, const double* __restrict__ F,
-      const double* __restrict__ X, double* __restrict__ part, double* __restrict__ eps_part, int want_rs)
-{
-    constexpr int NW = 8;              // warps
-    constexpr int RPW = 32 / TT;       // rows a warp holds at once
-    constexpr int RSTEP = NW * RPW;    // rows of one pass of the block
-    static_assert(TT == 16 || TT == 32, "tile edge");
-    __shared__ T sF[2][TT][3], sX[2][TT][3], sInv[2][TT];
-    __shared__ T sCol[NW][TT][9];      // the warps' column partials
-    __shared__ T sRowDiag[TT][9];      // diagonal job: row sums, added to the column records
-    __shared__ double sEps[NW];
-    __shared__ int sJob[2];
-    if (threadIdx.x == 0) sJob[0] = atomicAdd(next, 1);
-    __syncthreads();
-    int slot = 0;
-    for (int job = sJob[0]; job < n_jobs; job = sJob[slot]) {
-    // the next job, read after this one's last barrier
-    if (threadIdx.x == 0) sJob[slot ^ 1] = atomicAdd(next, 1);
-    const TileJob jb = jobs[job];
-    const TeaSeg g = segs[jb.seg];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int bi0 = g.begin + jb.I * TT, bj0 = g.begin + jb.J * TT;
-    const int ni = min(TT, g.count - jb.I * TT), nj = min(TT, g.count - jb.J * TT);
-    const bool diag = jb.I == jb.J;
-    if (tid < TT) {
-        for (int side = 0; side < 2; ++side) {
-            const int b = (side ? bj0 : bi0) + tid;
-            const bool ok = tid < (side ? nj : ni);
-            for (int k = 0; k < 3; ++k) {
-                sF[side][tid][k] = ok ? (T)F[3 * b + k] : (T)0;
-                sX[side][tid][k] = ok && want_rs ? (T)X[3 * b + k] : (T)0;
-            }
-            sInv[side][tid] = ok ? (T)(pos[b].w / A.preDii) : (T)0;   // 1/diag_D (diff_decl.c:94-99)
-        }
-    }
-    __syncthreads();
-    const int lj = lane % TT, sub = lane / TT;
-    const T* fc = sF[1][lj];
-    const T* xc = sX[1][lj];
-    const T invc = sInv[1][lj];
-    T col[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    T eps = 0;
-#pragma unroll 1
-    for (int r0 = 0; r0 < TT; r0 += RSTEP) {
-        const int li = r0 + warp * RPW + sub;
-        T t[6] = {0, 0, 0, 0, 0, 0};
-        if (li < ni && lj < nj && (!diag || lj < li)) tile_of_k<T, kEwald>(A, pos, bi0 + li, bj0 + lj, t);
-        const T xx = t[0], yy = t[1], zz = t[2], xy = t[3], xz = t[4], yz = t[5];
-        // bead li: products with bead lj's F, X and 1/D_jj
-        T row[9];
-        row[0] = xx * fc[0] + xy * fc[1] + xz * fc[2];
-        row[1] = xy * fc[0] + yy * fc[1] + yz * fc[2];
-        row[2] = xz * fc[0] + yz * fc[1] + zz * fc[2];
-        row[3] = (xx * xx + xy * xy + xz * xz) * invc;
-        row[4] = (xy * xy + yy * yy + yz * yz) * invc;
-        row[5] = (xz * xz + yz * yz + zz * zz) * invc;
-        row[6] = xx * xc[0] + xy * xc[1] + xz * xc[2];
-        row[7] = xy * xc[0] + yy * xc[1] + yz * xc[2];
-        row[8] = xz * xc[0] + yz * xc[1] + zz * xc[2];
-        eps += xx + yy + zz + 2 * (xy + xz + yz);
-        // bead lj: products with bead li's
-        const T* fr = sF[0][li];
-        const T* xr = sX[0][li];
-        const T invr = sInv[0][li];
-        col[0] += xx * fr[0] + xy * fr[1] + xz * fr[2];
-        col[1] += xy * fr[0] + yy * fr[1] + yz * fr[2];
-        col[2] += xz * fr[0] + yz * fr[1] + zz * fr[2];
-        col[3] += (xx * xx + xy * xy + xz * xz) * invr;
-        col[4] += (xy * xy + yy * yy + yz * yz) * invr;
-        col[5] += (xz * xz + yz * yz + zz * zz) * invr;
-        col[6] += xx * xr[0] + xy * xr[1] + xz * xr[2];
-        col[7] += xy * xr[0] + yy * xr[1] + yz * xr[2];
-        col[8] += xz * xr[0] + yz * xr[1] + zz * xr[2];
-#pragma unroll
-        for (int o = 1; o < TT; o <<= 1)
-#pragma unroll
-            for (int k = 0; k < 9; ++k) row[k] += __shfl_xor_sync(0xffffffffu, row[k], o);
-        if (lj == 0 && li < ni) {
-            if (diag) {
-                for (int k = 0; k < 9; ++k) sRowDiag[li][k] = row[k];
-            } else {
-                // record (T = J, bead in I)
-                double* dst = part + 9 * ((size_t)g.part_begin + (size_t)jb.J * g.count + jb.I * TT + li);
-                for (int k = 0; k < 9; ++k) dst[k] = (double)row[k];
-            }
-        }
-    }
-    if constexpr (RPW == 2) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) col[k] += __shfl_xor_sync(0xffffffffu, col[k], 16);
-    }
-    if (sub == 0)
-        for (int k = 0; k < 9; ++k) sCol[warp][lj][k] = col[k];
-    {
-        double e = (double)eps;
-        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) sEps[warp] = e;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double e = 0;
-        for (int w = 0; w < NW; ++w) e += sEps[w];
-        eps_part[job] = e;
-    }
-    // column records (T = I, bead in J), the warps' partials in order; on a
-    // diagonal job the row sums of the same bead join them
-    for (int q = tid; q < TT * 9; q += blockDim.x) {
-        const int c = q / 9, k = q % 9;
-        if (c < nj) {
-            T a = 0;
-            for (int w = 0; w < NW; ++w) a += sCol[w][c][k];
-            double v = (double)a;
-            if (diag) v += (double)sRowDiag[c][k];
-            part[9 * ((size_t)g.part_begin + (size_t)jb.I * g.count + jb.J * TT + c) + k] = v;
-        }
-    }
-    __syncthreads();   // the job's shared arrays are read; the next job may write them
-    slot ^= 1;
-    }
-}
-
-// eps -> beta per segment (diff_rand.c:197-217); scal[4g+0] = eps, [4g+1] = beta
-__global__ void k_eps_beta(const TeaSeg* __restrict__ segs, const int* __restrict__ job_begin,
-                           const double* __restrict__ eps_part, double* __restrict__ scal, unsigned* status)
-{
-    __shared__ double sh[256];
-    const TeaSeg g = segs[blockIdx.x];
-    const int b = job_begin[blockIdx.x], e = job_begin[blockIdx.x + 1];
-    double a = 0;
-    for (int k = b + threadIdx.x; k < e; k += blockDim.x) a += eps_part[k];
-    sh[threadIdx.x] = a;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const int n3 = 3 * g.count;
-        double eps = sh[0];
-        eps /= n3;
-        eps /= (n3 - 1);
-        eps *= 2;
-        if (eps > 1.0) eps = 1.0;
-        const double aa = (3 * g.count - 1) * eps * eps - (3 * g.count - 2) * eps;
-        double beta;
-        if (fabs(aa) < (double)0.0000001f) beta = 0.5;
-        else beta = (1 - sqrt(1 - aa)) / aa;
-        scal[4 * blockIdx.x] = eps;
-        scal[4 * blockIdx.x + 1] = beta;
-    }
-}
-
-__global__ void k_tea_finish(TensorArgs A, int n, const TeaSeg* __restrict__ segs, const int* __restrict__ bead_seg,
-                             const double* __restrict__ part, const double* __restrict__ scal,
-                             const double4* __restrict__ pos_in, const double* __restrict__ F,
-                             const double* __restrict__ X, double pre_f, int want_rs, int hydro,
-                             double* __restrict__ Rf, double* __restrict__ Rs)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int gi = bead_seg[i];
-    const TeaSeg g = segs[gi];
-    const int local = i - g.begin;
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (hydro) {
-        for (int T = 0; T < g.ntile; ++T) {
-            const double* src = part + 9 * ((size_t)g.part_begin + (size_t)T * g.count + local);
-            for (int k = 0; k < 9; ++k) acc[k] += src[k];
-        }
-    }
-    // self tile: D.F uses only its diagonal (diff_equation.c:96-102)
-    double self[6];
-    tile_of<double>(A, pos_in, i, i, self);
-    const double d = A.preDii / pos_in[i].w;   // diag_D (diff_decl.c:94-99)
-    const double inv_d = 1 / d;
-    for (int k = 0; k < 3; ++k) {
-        double rf = hydro ? acc[k] + F[3 * i + k] * self[k] : d * F[3 * i + k];
-        Rf[3 * i + k] = hydro ? rf * pre_f : pre_f * d * F[3 * i + k];
-    }
-    if (want_rs && !hydro) {
-        // DIFF_NONE (diff_rand.c:55-63): X already carries sqrt(2 dt D_ii)
-        for (int k = 0; k < 3; ++k) Rs[3 * i + k] = X[3 * i + k];
-    } else if (want_rs) {
-        const double beta = scal[4 * gi + 1];
-        for (int k = 0; k < 3; ++k) {
-            double c = acc[3 + k] * (beta * beta * inv_d);
-            c = 1 / (1 + c);
-            c = sqrt(c);
-            Rs[3 * i + k] = c * (beta * acc[6 + k] + d * X[3 * i + k]);
-        }
-    }
-}
-
-int tea_setup(bdb_system* s);
-
-template <int TT>
-static void tea_launch(bdb_system* s, const TensorArgs& A, const TeaSeg* tsegs, bool want_rs)
-{
-    // persistent grid: the SMs' capacity for this variant, at most one CTA per job
-    auto go = [&](auto kern) {
-        int occ = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, 0);
-        const int grid = std::max(1, std::min(s->n_jobs, std::max(1, occ) * s->sm_count));
-        cudaMemsetAsync(s->tea_next.p, 0, sizeof(int), s->stream);
-        kern<<<grid, 256, 0, s->stream>>>(A, s->jobs.p, s->n_jobs, s->tea_next.p, tsegs, s->pos.p, s->F.p, s->X.p,
-                                          s->part.p, s->eps_part.p, want_rs);
-    };
-    if (s->p.precision == BDB_PREC_FP64) {
-        if (A.ewald) go(k_tea<double, TT, true>);
-        else go(k_tea<double, TT, false>);
-    } else {
-        if (A.ewald) go(k_tea<float, TT, true>);
-        else go(k_tea<float, TT, false>);
-    }
-}
-
-static void tea_dispatch(bdb_system* s, const TensorArgs& A, const TeaSeg* tsegs, bool want_rs)
-{
-    if (s->tea_tile == 16) tea_launch<16>(s, A, tsegs, want_rs);
-    else tea_launch<32>(s, A, tsegs, want_rs);
-}
-
-// Autotuning of the TEA tile (16 or 32 beads): each candidate's work list
-// is built and its pair kernel timed twice on the system's stream; the
-// faster one is kept. Runs at the first TEA call of a system with
-// autotuning on (which comes before any graph capture).
-static int tea_tune(bdb_system* s, bool want_rs)
-{
-    const int cands[2] = {16, 32};
-    float best_ms = 1e30f;
-    int best = s->tea_tile;
-    cudaEvent_t e0, e1;
-    BDB_CUDA(cudaEventCreate(&e0));
-    BDB_CUDA(cudaEventCreate(&e1));
-    for (int c : cands) {
-        s->tea_tile = c;
-        int rc = tea_setup(s);
-        if (rc) return rc;
-        if (int rc_e = ewald_tables(s)) return rc_e;
-        const TensorArgs A = targs(s);
-        const TeaSeg* tsegs = reinterpret_cast<const TeaSeg*>(s->tea_meta.p);
-        tea_dispatch(s, A, tsegs, want_rs);   // warm-up
-        BDB_CUDA(cudaEventRecord(e0, s->stream));
-        tea_dispatch(s, A, tsegs, want_rs);
-        tea_dispatch(s, A, tsegs, want_rs);
-        BDB_CUDA(cudaEventRecord(e1, s->stream));
-        BDB_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        BDB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        s->launches += 3;
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = c;
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    s->tea_tile = best;
-    s->tea_tuned = true;
-    return tea_setup(s);
-}
-
-int tea_run(bdb_system* s, bool want_rs)
-{
-    int rc0 = tensor_attrs();
-    if (rc0) return rc0;
-    if (s->autotune && !s->tea_tuned && s->p.hydro && s->n_jobs >= 0) {
-        int rc = tea_tune(s, want_rs);
-        if (rc) return rc;
-    } else if (!s->tea_meta.p) {
-        int rc = tea_setup(s);
-        if (rc) return rc;
-    }
-    if (int rc_e = ewald_tables(s)) return rc_e;
-    const TensorArgs A = targs(s);
-    TeaSeg* tsegs = reinterpret_cast<TeaSeg*>(s->tea_meta.p);
-    if (s->p.hydro && s->n_jobs) {
-        tea_dispatch(s, A, tsegs, want_rs);
-        BDB_CUDA(cudaGetLastError());
-        if (want_rs) {
-            const int* job_begin = reinterpret_cast<const int*>(tsegs + s->segs.size());
-            k_eps_beta<<<(int)s->segs.size(), 256, 0, s->stream>>>(tsegs, job_begin, s->eps_part.p, s->scal.p + 64,
-                                                                   s->status.p);
-            BDB_CUDA(cudaGetLastError());
-        }
-    }
-    s->launches += 1 + ((s->p.hydro && s->n_jobs) ? (want_rs ? 2 : 1) : 0);
-    const double pre_f = s->p.dt / (BDB_KB * s->p.T);
-    k_tea_finish<<<(s->n + 127) / 128, 128, 0, s->stream>>>(A, s->n, tsegs, s->d_bead_seg.p, s->part.p, s->scal.p + 64,
-                                                            s->pos.p, s->F.p, s->X.p, pre_f, want_rs,
-                                                            s->p.hydro, s->Rf.p, s->Rs.p);
-    BDB_CUDA(cudaGetLastError());
-    return BDB_OK;
-}
-
-// Work list and scratch layout for k_tea: the TeaSeg table followed by the
-// per-segment job offsets, in tea_meta.
-int tea_setup(bdb_system* s)
-{
-    std::vector<TileJob> jobs;
-    std::vector<TeaSeg> ts;
-    std::vector<int> job_begin;
-    size_t part_records = 0;
-    for (size_t g = 0; g < s->segs.size(); ++g) {
-        const Segment& sg = s->segs[g];
-        TeaSeg t;
-        t.begin = sg.begin;
-        t.count = sg.count;
-        t.ntile = (sg.count + s->tea_tile - 1) / s->tea_tile;
-        t.part_begin = (int)part_records;
-        part_records += (size_t)t.ntile * sg.count;
-        ts.push_back(t);
-        job_begin.push_back((int)jobs.size());
-        for (int I = 0; I < t.ntile; ++I)
-            for (int J = 0; J <= I; ++J) jobs.push_back(TileJob{(int)g, I, J});
-    }
-    job_begin.push_back((int)jobs.size());
-    s->n_jobs = (int)jobs.size();
-    if (s->jobs.alloc(std::max<size_t>(1, jobs.size()))) return BDB_ERR_NOMEM;
-    if (!s->tea_next.p && s->tea_next.alloc(1)) return BDB_ERR_NOMEM;
-    if (s->eps_part.alloc(std::max<size_t>(1, jobs.size()))) return BDB_ERR_NOMEM;
-    if (s->part.alloc(std::max<size_t>(9, 9 * part_records))) return BDB_ERR_NOMEM;
-    const size_t head = sizeof(TeaSeg) * ts.size() + sizeof(int) * job_begin.size();
-    if (s->tea_meta.alloc(head)) return BDB_ERR_NOMEM;
-    BDB_CUDA(h2d(s, s->jobs.p, jobs.data(), sizeof(TileJob) * jobs.size()));
-    BDB_CUDA(h2d(s, s->tea_meta.p, ts.data(), sizeof(TeaSeg) * ts.size()));
-    BDB_CUDA(h2d(s, s->tea_meta.p + sizeof(TeaSeg) * ts.size(), job_begin.data(), sizeof(int) * job_begin.size()));
     return BDB_OK;
 }
 

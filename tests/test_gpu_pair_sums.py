@@ -1,0 +1,93 @@
+"""The matrix-free pair sums (tea.cu) against BD_BOX's restatement (the
+oracle), at sizes where the work split changes: tile edges, one bead over,
+odd numbers of tiles, jobs of several column and row tiles; and the converged
+split of the lattice sums (ewald_fast.cuh) against the reference's own sums in
+FP64, over what decides between the two."""
+import numpy as np
+import pytest
+
+from conftest import gpu_available
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="needs a CUDA device")]
+
+from bd_box_b200 import decks, engine  # noqa: E402
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [2, 3, 31, 32, 33, 64, 65, 95, 97, 161])
+def test_drift_and_noise_at_tile_edges(n, deck_dir):
+    import pyoracle
+    d = decks.read_deck(decks.write_chain_deck(deck_dir, f"pairs{n}", n, seed=50 + n, hydro="geyer"))
+    o = pyoracle.Oracle(d)
+    g = np.random.default_rng(n).standard_normal(3 * n)
+    F = o.forces()[0]
+    dt = d.prm["dt"]
+    df, tea = o.df(F, dt), o.tea(g, dt)
+    tea = tea[0] if isinstance(tea, tuple) else tea
+    s = engine.System(d, precision=engine.PREC_FP64, noise=engine.NOISE_HOST)
+    # 3N additions of ~1 ulp each side
+    assert rel(s.compute_Rf(), df) <= 1e-13
+    assert rel(s.compute_r(g), tea) <= 1e-13
+    m = engine.System(d, precision=engine.PREC_MIXED, noise=engine.NOISE_HOST)
+    assert rel(m.compute_Rf(), df) <= 2e-6
+    assert rel(m.compute_r(g), tea) <= 2e-6
+
+
+@pytest.mark.parametrize("sizes", [(2, 33, 700, 64, 31), tuple(range(600, 900, 6)), (1500,) * 6 + (1441, 1409)])
+def test_mixed_batch_follows_fp64(sizes, deck_dir):
+    """Batches whose jobs hold 1, 2 and more column tiles, with and without
+    row-tile pairs (odd and even tile counts)."""
+    ds = [decks.read_deck(decks.write_chain_deck(deck_dir, f"b{n}", n, seed=n, hydro="geyer")) for n in sorted(set(sizes))]
+    by_n = {d.n: d for d in ds}
+    batch = [by_n[n] for n in sizes]
+    n3 = 3 * sum(sizes)
+    g = np.random.default_rng(1).standard_normal(n3)
+    out = {}
+    for p in (engine.PREC_FP64, engine.PREC_MIXED):
+        s = engine.System(batch, precision=p, noise=engine.NOISE_HOST)
+        out[p] = s.compute_Rf(), s.compute_r(g)
+        s.close()
+    for a, b in zip(out[engine.PREC_MIXED], out[engine.PREC_FP64]):
+        assert np.isfinite(a).all()
+        assert rel(a, b) <= 1e-6
+
+
+@pytest.mark.parametrize("method", ["beenakker", "smith"])
+@pytest.mark.parametrize("r", [2, 3, 4, 5])
+@pytest.mark.parametrize("kind", ["plain", "radii", "outside", "overlap"])
+def test_lattice_sums_mixed_against_fp64(method, r, kind, deck_dir):
+    """R = 4 and 5 take the converged split where it holds; other radii than
+    bead 0's, beads outside the box and overlapping pairs go back to the
+    reference's sums, pair by pair."""
+    n = 97
+    d = decks.read_deck(decks.write_suspension_deck(deck_dir, f"lat_{method}{r}", n, seed=3, ewald_r=r,
+                                                    extra={"ewald_method": method}))
+    d.coord = d.coord.copy()
+    if kind == "radii":
+        d.coord[::3, 3] *= 0.7
+    elif kind == "outside":
+        d.coord[5, 0] += d.box[0]
+        d.coord[40, 2] -= 2 * d.box[0]
+    elif kind == "overlap":
+        d.coord[11, :3] = d.coord[60, :3] + [0.9, 0.4, -0.3]
+    g = np.random.default_rng(4).standard_normal(3 * n)
+    s64 = engine.System(d, precision=engine.PREC_FP64, noise=engine.NOISE_HOST)
+    mix = engine.System(d, precision=engine.PREC_MIXED, noise=engine.NOISE_HOST)
+    assert rel(mix.compute_Rf(), s64.compute_Rf()) <= 2e-6
+    if kind in ("plain", "radii"):   # the others make eps, hence TEA, meaningless
+        assert rel(mix.compute_r(g), s64.compute_r(g)) <= 4e-6
+
+
+@pytest.mark.parametrize("method", ["beenakker", "smith"])
+def test_lattice_sums_fp64_against_oracle(method, deck_dir):
+    import pyoracle
+    d = decks.read_deck(decks.write_suspension_deck(deck_dir, f"lo_{method}", 40, seed=9, ewald_r=5,
+                                                    extra={"ewald_method": method}))
+    o = pyoracle.Oracle(d)
+    s = engine.System(d, precision=engine.PREC_FP64, noise=engine.NOISE_HOST)
+    for i, j in ((0, 1), (7, 30), (39, 2), (5, 5)):
+        a, b = s.compute_Dij(i, j), np.asarray(o.tile(max(i, j), min(i, j))).reshape(3, 3)
+        assert np.abs(a - b).max() <= 1e-13 * np.abs(o.tile(0, 0)).max()
