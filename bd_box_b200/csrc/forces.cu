@@ -46,6 +46,8 @@ struct ForceParams {
     double bond_lj_scale, bond_c_scale;
     int check_overlap;
     int conn_live;
+    double g_elec;      // gamma_c / epsilon_c
+    double reach_sq;    // squared reach of the widest interaction, padded
 };
 
 static ForceParams make_fp(const bdb_system* s)
@@ -68,6 +70,8 @@ static ForceParams make_fp(const bdb_system* s)
     f.bond_c_scale = s->p.bond_c_scale;
     f.check_overlap = s->p.check_overlap;
     f.conn_live = s->conn_live;
+    f.g_elec = s->p.gamma_c / s->p.epsilon_c;
+    f.reach_sq = s->reach * s->reach * (1 + 1e-9);
     return f;
 }
 
@@ -87,12 +91,40 @@ __device__ __forceinline__ int cell_axis(double x, double o, double w, int n, bo
     return ci < 0 ? 0 : (ci >= n ? n - 1 : ci);
 }
 
+// more than skin/2 away from where it was when the cells were sorted
+__device__ __forceinline__ bool has_moved(const double4& a, const double4& b, double skin, int periodic,
+                                          const double3& box)
+{
+    double d[3] = {a.x - b.x, a.y - b.y, a.z - b.z};
+    if (periodic) {
+        d[0] -= box.x * floor(d[0] / box.x + 0.5);
+        d[1] -= box.y * floor(d[1] / box.y + 0.5);
+        d[2] -= box.z * floor(d[2] / box.z + 0.5);
+    }
+    return d[0] * d[0] + d[1] * d[1] + d[2] * d[2] > 0.25 * skin * skin;
+}
+
+// The skin test over the whole GPU, for systems of MOVED_MIN beads or more:
+// one CTA per segment is bound by the latency of its own loads (31 us at
+// N = 20,000, 10 at 4,096; 5 and 4 with this launch in front). The flags are
+// cleared by k_cells. Segments not sorted yet are sorted anyway.
+static constexpr int MOVED_MIN = 2048;
+__global__ void k_moved(int n, const double4* __restrict__ pos, const double4* __restrict__ pos_build,
+                        const int* __restrict__ bead_seg, double skin, int periodic, double3 box,
+                        const int* __restrict__ built, int* __restrict__ moved_flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int g = bead_seg[i];
+    if (built[g] && has_moved(pos[i], pos_build[i], skin, periodic, box)) moved_flag[g] = 1;
+}
+
 __global__ void k_cells(const double4* __restrict__ pos, const Segment* __restrict__ segs,
                         double cell, double skin, int periodic, double3 box,
                         unsigned long long* __restrict__ keys_out, int* __restrict__ idx_out,
                         double4* __restrict__ grid, int4* __restrict__ dims, double4* __restrict__ pos_build,
                         int* __restrict__ built, int2* __restrict__ cell_range, const long long* __restrict__ cell_off,
-                        int* __restrict__ resort)
+                        int* __restrict__ resort, int* __restrict__ moved_flag)
 {
     extern __shared__ unsigned long long sk[];
     __shared__ double red[6][32];
@@ -104,25 +136,20 @@ __global__ void k_cells(const double4* __restrict__ pos, const Segment* __restri
     const bool big = sg.count > SORT_MAX;   // sorted by the multi-CTA kernels below
     if (big && tid == 0) resort[blockIdx.x] = 0;
     if (built[blockIdx.x]) {
-        // re-sort only when a bead has moved more than skin/2 since the last sort
-        if (tid == 0) moved = 0;
+        // re-sort only when a bead has moved more than skin/2 since the last
+        // sort: k_moved has looked (large systems), or this CTA does
+        if (tid == 0) moved = moved_flag ? moved_flag[blockIdx.x] : 0;
         __syncthreads();
-        const double lim = 0.25 * skin * skin;
-        bool far = false;
-        for (int i = tid; i < sg.count; i += nt) {
-            const double4 a = pos[sg.begin + i], b = pos_build[sg.begin + i];
-            double d[3] = {a.x - b.x, a.y - b.y, a.z - b.z};
-            if (periodic) {
-                d[0] -= box.x * floor(d[0] / box.x + 0.5);
-                d[1] -= box.y * floor(d[1] / box.y + 0.5);
-                d[2] -= box.z * floor(d[2] / box.z + 0.5);
-            }
-            if (d[0] * d[0] + d[1] * d[1] + d[2] * d[2] > lim) far = true;
+        if (!moved_flag) {
+            bool far = false;
+            for (int i = tid; i < sg.count; i += nt)
+                far = far || has_moved(pos[sg.begin + i], pos_build[sg.begin + i], skin, periodic, box);
+            if (far) moved = 1;
+            __syncthreads();
         }
-        if (far) moved = 1;
-        __syncthreads();
         if (!moved) return;
     }
+    if (moved_flag && tid == 0) moved_flag[blockIdx.x] = 0;
     if (!periodic) {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int i = tid; i < sg.count; i += nt) {
@@ -385,26 +412,35 @@ __global__ void k_big_fill(int g, const int* __restrict__ resort, const Segment*
     if (blockIdx.x == 0 && threadIdx.x == 0) built[g] = 1;
 }
 
-// ------------------------------------------------------------- non-bonded
-
-__device__ __forceinline__ bool is_conn(const int* conn_ptr, const int* conn_list, int i, int j)
+// The positions in the order of the sorted beads, one array per coordinate:
+// the candidates of a cell are then contiguous loads. Gathering them one by
+// one (32 bytes each, 32 lines a load) held the non-bonded kernel of a dense
+// system to the L1's rate. For large periodic boxes with 8 beads a cell and
+// more; a chain's cells hold a few beads, where neither helps (N = 4096: 11.0
+// us without, 12.8 with, and the launch).
+__global__ void k_sorted_pos(int n, const double4* __restrict__ pos, const int* __restrict__ bead_seg,
+                             const int4* __restrict__ dims, const int* __restrict__ sidx, double* __restrict__ sp)
 {
-    for (int k = conn_ptr[i]; k < conn_ptr[i + 1]; ++k)
-        if (conn_list[k] == j) return true;
-    return false;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n || dims[bead_seg[k]].w) return;
+    const double4 p = pos[sidx[k]];
+    sp[k] = p.x;
+    sp[n + k] = p.y;
+    sp[2 * (size_t)n + k] = p.z;
 }
 
-// force_single for the pair (a, b), a < b, accumulating the force on `self`
-// (a or b). Energies and pair counts are credited only when self == a.
-__device__ __forceinline__ void pair_term(const ForceParams& fp, const double4* pos, const double* Q,
-                                          const double2* LJ, const int* conn_ptr, const int* conn_list,
-                                          int a, int b, int self, double* f, double& e_lj, double& e_c,
-                                          unsigned& cnt_c, unsigned& cnt_lj, unsigned& rep)
+// ------------------------------------------------------------- non-bonded
+
+// force_single for the pair (a, b), a < b, at separation v = r_b - r_a,
+// accumulating the force on a (self_a) or b. Energies and pair counts are
+// credited only to a. conn: 1-2 bonded, with the scale factors in force. The cutoff tests and the overlap decision
+// use the exact r_norm; the magnitudes share one reciprocal of it.
+template <bool kEnergy>
+__device__ __forceinline__ void pair_term(const ForceParams& fp, const double* v, double qa, double qb,
+                                          const double2& la, const double2& lb, bool conn, bool self_a, double* f,
+                                          double& e_lj, double& e_c, unsigned& cnt_c, unsigned& cnt_lj, unsigned& rep)
 {
-    double v[3];
-    dist_vec(pos[a], pos[b], fp.periodic, fp.box, fp.inv_L, v);
     const double r_sq = sq3(v);
-    const double2 la = LJ[a], lb = LJ[b];
     const double sig = la.x + lb.x;
     const double lj_lim = fp.cutoff_lj > 0.0 ? fp.cutoff_lj : (double)1.122462f * sig;
     const double r_norm = __dsqrt_rn(r_sq);
@@ -417,27 +453,21 @@ __device__ __forceinline__ void pair_term(const ForceParams& fp, const double4* 
     }
     const double inv = 1.0 / r_norm;
     const double e[3] = {v[0] * inv, v[1] * inv, v[2] * inv};
-    const double sgn = self == a ? -1.0 : 1.0;   // F1 -= e F on a, F2 += e F on b
-    const bool conn = fp.conn_live && is_conn(conn_ptr, conn_list, a, b);
+    const double sgn = self_a ? -1.0 : 1.0;   // F1 -= e F on a, F2 += e F on b
     int r = 0;
     if (elec_in) {
-        if (self == a) cnt_c++;
+        if (kEnergy && self_a) cnt_c++;
         double scale = 1.0;
         bool on = true;
         if (conn) {
             if (fp.bond_c_scale != 0.0) scale = fp.bond_c_scale; else on = false;
         }
         if (on) {
-            const double g = fp.gamma_c / fp.epsilon_c;
-            double Fm = g * Q[a] * Q[b] * (1 + fp.kappa_c * r_norm);
+            const double gq = fp.g_elec * qa * qb;
             const double ex = exp(-fp.kappa_c * r_norm);
-            Fm *= ex / r_sq;
+            double Fm = gq * (1 + fp.kappa_c * r_norm) * (ex * inv * inv);
             if (scale != 1.0) Fm *= scale;
-            if (self == a) {
-                double en = g * Q[a] * Q[b] * ex / r_norm;
-                if (scale != 1.0) en = scale * g * Q[a] * Q[b] * ex / r_norm;
-                e_c += en;
-            }
+            if (kEnergy && self_a) e_c += scale * gq * ex * inv;
             f[0] += sgn * e[0] * Fm;
             f[1] += sgn * e[1] * Fm;
             f[2] += sgn * e[2] * Fm;
@@ -445,16 +475,16 @@ __device__ __forceinline__ void pair_term(const ForceParams& fp, const double4* 
         }
     }
     if (lj_in) {
-        if (self == a) cnt_lj++;
+        if (kEnergy && self_a) cnt_lj++;
         if (!conn || fp.bond_lj_scale != 0.0) {
             const double scale = conn ? fp.bond_lj_scale : 1.0;
             const double eps_ij = sqrt(la.y * lb.y);
-            double s6 = sig / r_norm;
+            double s6 = sig * inv;
             s6 *= s6;
             s6 *= s6 * s6;
-            double Fm = fp.alpha_lj * eps_ij * 6 * (s6 * (2 * s6 - fp.lj6)) / r_norm;
+            double Fm = fp.alpha_lj * eps_ij * 6 * (s6 * (2 * s6 - fp.lj6)) * inv;
             if (scale != 1.0) Fm *= scale;
-            if (self == a) e_lj += scale * (fp.alpha_lj * eps_ij * (s6 * (s6 - fp.lj6)));
+            if (kEnergy && self_a) e_lj += scale * (fp.alpha_lj * eps_ij * (s6 * (s6 - fp.lj6)));
             f[0] += sgn * e[0] * Fm;
             f[1] += sgn * e[1] * Fm;
             f[2] += sgn * e[2] * Fm;
@@ -469,39 +499,92 @@ __device__ __forceinline__ void pair_term(const ForceParams& fp, const double4* 
     if (fp.check_overlap && r) rep = 1;
 }
 
-// One warp per bead i: the lanes split the candidate beads of the 27
-// neighbour cells (or of the whole segment for brute-force segments); each
-// lane accumulates in a fixed order and the warp combines the lanes with a
-// fixed xor tree, so the result is deterministic.
-__global__ void __launch_bounds__(NB_THREADS)
-k_nonbonded(ForceParams fp, int n, const double4* __restrict__ pos, const double* __restrict__ Q,
+// separation r_b - r_a as dist_vec gives it, with the image shift only where
+// it is not zero
+__device__ __forceinline__ void pair_sep(const double4& a, const double4& b, const ForceParams& fp, double* v)
+{
+    v[0] = sub(b.x, a.x);
+    v[1] = sub(b.y, a.y);
+    v[2] = sub(b.z, a.z);
+    if (fp.periodic) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double t = add(mul(v[k], fp.inv_L[k]), 0.5);
+            if (!(t >= 0.0 && t < 1.0)) v[k] = sub(v[k], mul(fp.box[k], floor(t)));
+        }
+    }
+}
+
+// One warp per bead i over the candidate beads of its 27 neighbour cells
+// (or of the whole segment for brute-force segments). A cell is as wide as
+// the widest interaction plus the skin, so only about a seventh of the
+// candidates of a dense system interact: the lanes first keep those within
+// `reach` (the widest interaction, padded: the exact cutoff tests follow) in
+// a list per warp, and the pair terms -- some 150 FP64 operations -- run in
+// full rounds of 32 from it, not once per round of candidates with a few
+// lanes live. What does not depend on the candidates (the bead's bonded slots
+// and neighbours) is loaded before them: a warp is bound by the latency of its
+// chain of loads. N = 20,000 at 173 neighbours of 1,480 candidates: 398 -> 240
+// us (300 from unsorted positions); 256 chains of 64..1024 beads:
+// 287 -> 260.
+// Each lane accumulates in a fixed order and the warp combines the lanes with
+// a fixed xor tree, so the result is deterministic. kEnergy: energies and pair
+// counts per bead (steps need neither), for k_energy_reduce.
+// kDense (cells of many beads in a large periodic box): coalesced candidates
+// from the sorted positions.
+template <bool kEnergy, bool kDense>
+__global__ void __launch_bounds__(NB_THREADS, kDense ? 8 : 7)
+k_nonbonded(const __grid_constant__ ForceParams fp, int n, const double4* __restrict__ pos, const double* __restrict__ Q,
             const double2* __restrict__ LJ, const int* __restrict__ bead_seg,
             const Segment* __restrict__ segs, const int2* __restrict__ cell_range,
-            const long long* __restrict__ cell_off, const int* __restrict__ sidx,
+            const long long* __restrict__ cell_off, const int* __restrict__ sidx, const double* __restrict__ sp,
             const double4* __restrict__ grid, const int4* __restrict__ dims, const int* __restrict__ conn_ptr,
-            const int* __restrict__ conn_list, const double* __restrict__ F_bonded,
-            double* __restrict__ F, double* __restrict__ e_part,
-            unsigned long long* __restrict__ counts, unsigned* __restrict__ status)
+            const int* __restrict__ conn_list, const double* __restrict__ F_bonded, const int* __restrict__ slot_ptr,
+            const int* __restrict__ slot_list, const double* __restrict__ contrib, double* __restrict__ F,
+            double* __restrict__ e_part, unsigned* __restrict__ c_part, unsigned* __restrict__ status)
 {
-    const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= n) return;
+    __shared__ int s_j[NB_THREADS / 32][64];          // partners kept, not yet processed
+    __shared__ double s_v[NB_THREADS / 32][3][64];    // their separations
+    __shared__ int2 s_cell[NB_THREADS / 32][kDense ? 32 : 1];   // cells: end of its entries in the list, first bead
+    __shared__ int s_conn[NB_THREADS / 32][8];        // the bead's 1-2 neighbours
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= n) return;
     double f[3] = {0, 0, 0};
     double e_lj = 0, e_c = 0;
     unsigned cnt_c = 0, cnt_lj = 0, rep = 0;
-    const int sgi = bead_seg[i];
+    const int sgi = bead_seg[w];
     const Segment sg = segs[sgi];
     const int4 gd = dims[sgi];
+    const bool cells = !gd.w;
+    // dense systems: beads in cell order, so that the warps of a CTA share most
+    // of their candidates
+    const int i = kDense && cells ? sidx[w] : w;
+    const double4 p = pos[i];
+    // the bead's bonded force: gathered already (F_bonded), or its slots,
+    // lane l component l mod 3 of slot l / 3 (the first ten)
+    int slot0 = 0, nslot = 0;
+    double bond = 0;
+    if (F_bonded) {
+        if (lane < 3) bond = F_bonded[3 * i + lane];
+    } else if (slot_ptr) {
+        slot0 = slot_ptr[i];
+        nslot = slot_ptr[i + 1] - slot0;
+        if (lane < 30 && lane / 3 < nslot) bond = contrib[3 * slot_list[slot0 + lane / 3] + lane % 3];
+    }
+    int nconn = 0, conn0 = 0;
+    if (fp.conn_live) {
+        conn0 = conn_ptr[i];
+        nconn = conn_ptr[i + 1] - conn0;
+        if (lane < min(nconn, 8)) s_conn[warp][lane] = conn_list[conn0 + lane];
+    }
+    int total = 0;
+    int2 rg = make_int2(0, 0);
+    int incl = 0;
     if (fp.elec || fp.alpha_lj != 0.0) {
-        if (gd.w) {
-            for (int j = sg.begin + lane; j < sg.begin + sg.count; j += 32) {
-                if (j == i) continue;
-                const int a = i < j ? i : j, b = i < j ? j : i;
-                pair_term(fp, pos, Q, LJ, conn_ptr, conn_list, a, b, i, f, e_lj, e_c, cnt_c, cnt_lj, rep);
-            }
-        } else {
+        total = sg.count;
+        if (cells) {
             const double4 gr = grid[sgi];
-            const double4 p = pos[i];
             const double x[3] = {p.x, p.y, p.z};
             int c[3];
             const int nn[3] = {gd.x, gd.y, gd.z};
@@ -510,7 +593,6 @@ k_nonbonded(ForceParams fp, int n, const double4* __restrict__ pos, const double
                                  nn[k], fp.periodic);
             const int2* tab = cell_range + cell_off[2 * sgi];
             // lanes 0..26 fetch the [first, end) range of one neighbour cell each
-            int2 rg = make_int2(0, 0);
             if (lane < 27) {
                 int cc[3] = {c[0] + lane % 3 - 1, c[1] + (lane / 3) % 3 - 1, c[2] + lane / 9 - 1};
                 bool skip = false;
@@ -523,37 +605,16 @@ k_nonbonded(ForceParams fp, int n, const double4* __restrict__ pos, const double
                 if (!skip) rg = tab[((long long)cc[2] * nn[1] + cc[1]) * nn[0] + cc[0]];
             }
             // the 27 cells' beads as one list: lane k's candidates are
-            // entries k, k + 32, ... of it (a scan of the cell counts and a
-            // search over it), so a warp does a few full rounds instead of
-            // one sparse round per cell; the rounds are warp-uniform
-            const int cnt = rg.y - rg.x;
-            int incl = cnt;
+            // entries k, k + 32, ... of it (a scan of the cell counts), so a
+            // warp does a few full rounds instead of one sparse round per cell
+            incl = rg.y - rg.x;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int v = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += v;
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            for (int base = 0; base < total; base += 32) {
-                const int q = base + lane;
-                // the cell holding entry q: the first lane whose inclusive
-                // count exceeds q (cells 27..31 add nothing)
-                int c = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int probe = __shfl_sync(0xffffffffu, incl, c + step - 1);
-                    if (probe <= q) c += step;
-                }
-                const int first = __shfl_sync(0xffffffffu, rg.x, c);
-                const int excl = __shfl_sync(0xffffffffu, incl, c) - __shfl_sync(0xffffffffu, cnt, c);
-                if (q < total) {
-                    const int j = sidx[first + (q - excl)];
-                    if (j != i) {
-                        const int a = i < j ? i : j, b = i < j ? j : i;
-                        pair_term(fp, pos, Q, LJ, conn_ptr, conn_list, a, b, i, f, e_lj, e_c, cnt_c, cnt_lj, rep);
-                    }
-                }
-            }
+            if (kDense) s_cell[warp][lane] = make_int2(incl, rg.y - incl);   // bead of entry q: q + .y
+            total = __shfl_sync(0xffffffffu, incl, 31);
         }
     } else if (fp.check_overlap) {
         for (int j = sg.begin + lane; j < sg.begin + sg.count; j += 32) {
@@ -565,25 +626,106 @@ k_nonbonded(ForceParams fp, int n, const double4* __restrict__ pos, const double
             if (sig * sig > sq3(v)) rep = 1;
         }
     }
+    __syncwarp();
+    int kept = 0, base = 0;
+    int2 cell = kDense && cells && total ? s_cell[warp][0] : make_int2(0, 0);
+    int at_cell = 0;
+    for (;;) {
+        // candidates until a round of partners is full
+        while (kept < 32 && base < total) {
+            const int q = base + lane;
+            int k = q, j = -1;
+            if (!kDense && cells) {
+                // the cell holding entry q: the first lane whose inclusive
+                // count exceeds q (cells 27..31 add nothing)
+                int c = 0;
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) {
+                    const int probe = __shfl_sync(0xffffffffu, incl, c + step - 1);
+                    if (probe <= q) c += step;
+                }
+                k += __shfl_sync(0xffffffffu, rg.y - incl, c);
+            }
+            bool keep = false;
+            double v[3];
+            if (q < total) {
+                double4 pj;
+                if (cells) {
+                    if (kDense) {
+                        // cells of many beads: an entry's cell only moves on
+                        while (q >= cell.x) cell = s_cell[warp][++at_cell];
+                        k += cell.y;
+                    }
+                    j = sidx[k];
+                    pj = kDense ? make_double4(sp[k], sp[n + k], sp[2 * (size_t)n + k], 0.0) : pos[j];
+                } else {
+                    j = sg.begin + q;
+                    pj = pos[j];
+                }
+                if (j != i) {
+                    if (i < j) pair_sep(p, pj, fp, v);
+                    else pair_sep(pj, p, fp, v);
+                    keep = sq3(v) <= fp.reach_sq;
+                }
+            }
+            base += 32;
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int at = kept + __popc(m & ((1u << lane) - 1));
+                s_j[warp][at] = j;
+                s_v[warp][0][at] = v[0];
+                s_v[warp][1][at] = v[1];
+                s_v[warp][2][at] = v[2];
+            }
+            kept += __popc(m);
+        }
+        if (!kept) break;
+        __syncwarp();
+        // the last min(32, kept) of the list
+        const int m = min(kept, 32), at = kept - m + lane;
+        if (lane < m) {
+            const int j = s_j[warp][at];
+            const double v[3] = {s_v[warp][0][at], s_v[warp][1][at], s_v[warp][2][at]};
+            const int a = min(i, j), b = max(i, j);
+            bool conn = false;
+            for (int k = 0; k < min(nconn, 8); ++k) conn = conn || s_conn[warp][k] == j;
+            for (int k = 8; k < nconn; ++k) conn = conn || conn_list[conn0 + k] == j;
+            pair_term<kEnergy>(fp, v, Q[a], Q[b], LJ[a], LJ[b], conn, i == a, f, e_lj, e_c, cnt_c, cnt_lj, rep);
+        }
+        kept -= m;
+        __syncwarp();
+    }
     for (int o = 16; o > 0; o >>= 1) {
         f[0] += __shfl_xor_sync(0xffffffffu, f[0], o);
         f[1] += __shfl_xor_sync(0xffffffffu, f[1], o);
         f[2] += __shfl_xor_sync(0xffffffffu, f[2], o);
-        e_lj += __shfl_xor_sync(0xffffffffu, e_lj, o);
-        e_c += __shfl_xor_sync(0xffffffffu, e_c, o);
-        cnt_c += __shfl_xor_sync(0xffffffffu, cnt_c, o);
-        cnt_lj += __shfl_xor_sync(0xffffffffu, cnt_lj, o);
-        rep |= __shfl_xor_sync(0xffffffffu, rep, o);
+        if (kEnergy) {
+            e_lj += __shfl_xor_sync(0xffffffffu, e_lj, o);
+            e_c += __shfl_xor_sync(0xffffffffu, e_c, o);
+            cnt_c += __shfl_xor_sync(0xffffffffu, cnt_c, o);
+            cnt_lj += __shfl_xor_sync(0xffffffffu, cnt_lj, o);
+        }
     }
+    const bool any_rep = __any_sync(0xffffffffu, rep != 0);
+    // the bonded force first, slots in order
+    double g = 0;
+    if (F_bonded) {
+        g = bond;
+    } else {
+        for (int k = 0; k < nslot; ++k) {
+            const double c = __shfl_sync(0xffffffffu, bond, min(3 * k + lane, 31));
+            if (lane < 3) g += k < 10 ? c : contrib[3 * slot_list[slot0 + k] + lane];
+        }
+    }
+    if (lane < 3) F[3 * i + lane] = g + (lane == 0 ? f[0] : lane == 1 ? f[1] : f[2]);
     if (lane == 0) {
-        F[3 * i] = F_bonded[3 * i] + f[0];
-        F[3 * i + 1] = F_bonded[3 * i + 1] + f[1];
-        F[3 * i + 2] = F_bonded[3 * i + 2] + f[2];
-        e_part[2 * i] = e_lj;
-        e_part[2 * i + 1] = e_c;
-        if (cnt_c) atomicAdd(&counts[0], (unsigned long long)cnt_c);
-        if (cnt_lj) atomicAdd(&counts[1], (unsigned long long)cnt_lj);
-        if (rep) atomicOr(status, ST_OVERLAP);
+        if (kEnergy) {
+            e_part[2 * i] = e_lj;
+            e_part[2 * i + 1] = e_c;
+            c_part[2 * i] = cnt_c;
+            c_part[2 * i + 1] = cnt_lj;
+        }
+        if (any_rep) atomicOr(status, ST_OVERLAP);
     }
 }
 
@@ -935,30 +1077,45 @@ struct TermRanges {
     int lim[6];   // [lim[t], lim[t+1]) are the terms of type t
 };
 
-__global__ void k_energy_reduce(int nb_blocks, const double* __restrict__ e_part,
-                                const double* __restrict__ term_energy, TermRanges tr, double* __restrict__ E)
+// One CTA per energy type and pair count (7, 8), fixed order (one CTA for all
+// energies: 40 us at N = 20,000, now 7; a pair-count atomic per bead on one
+// address cost 0.1 ms more)
+__global__ void __launch_bounds__(1024) k_energy_reduce(int nb, const double* __restrict__ e_part,
+                                                        const unsigned* __restrict__ c_part,
+                                                        const double* __restrict__ term_energy, TermRanges tr,
+                                                        double* __restrict__ E, unsigned long long* __restrict__ counts)
 {
-    __shared__ double sh[256];
-    const int tid = threadIdx.x;
-    for (int type = 0; type < 7; ++type) {
-        double a = 0;
-        if (type < 5) {
-            for (int k = tr.lim[type] + tid; k < tr.lim[type + 1]; k += blockDim.x) a += term_energy[k];
-        } else {
-            for (int k = tid; k < nb_blocks; k += blockDim.x) a += e_part[2 * k + (type - 5)];
-        }
-        sh[tid] = a;
+    __shared__ double sh[32];
+    __shared__ unsigned long long shc;
+    const int tid = threadIdx.x, type = blockIdx.x;
+    if (type >= 7) {
+        unsigned long long c = 0;
+        if (tid == 0) shc = 0;
         __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (tid < o) sh[tid] += sh[tid + o];
-            __syncthreads();
-        }
-        if (tid == 0) E[1 + type] = sh[0];
+        for (int k = tid; k < nb; k += blockDim.x) c += c_part[2 * k + (type - 7)];
+        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if ((tid & 31) == 0) atomicAdd(&shc, c);
         __syncthreads();
+        if (tid == 0) counts[type - 7] = shc;
+        return;
     }
-    if (tid == 0) {
-        E[0] = 0;
-        E[8] = 0;
+    double a = 0;
+    if (type < 5) {
+        for (int k = tr.lim[type] + tid; k < tr.lim[type + 1]; k += blockDim.x) a += term_energy[k];
+    } else {
+        for (int k = tid; k < nb; k += blockDim.x) a += e_part[2 * k + (type - 5)];
+    }
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((tid & 31) == 0) sh[tid >> 5] = a;
+    __syncthreads();
+    if (tid < 32) {
+        a = sh[tid];
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (tid == 0) {
+            E[1 + type] = a;
+            if (type == 0) E[0] = 0;
+            if (type == 1) E[8] = 0;
+        }
     }
 }
 
@@ -1062,6 +1219,8 @@ int forces_setup(bdb_system* s)
     if (s->cell_range.alloc(tot) || s->cell_off.alloc(2 * nseg)) return BDB_ERR_NOMEM;
     if (s->cells_resort.alloc(nseg)) return BDB_ERR_NOMEM;
     BDB_CUDA(dzero(s, s->cells_resort.p, sizeof(int) * nseg));
+    if (s->cells_moved.alloc(nseg)) return BDB_ERR_NOMEM;
+    BDB_CUDA(dzero(s, s->cells_moved.p, sizeof(int) * nseg));
     int big = 0;
     for (auto& g : s->segs) big = std::max(big, g.count > SORT_MAX ? g.count : 0);
     if (big) {
@@ -1075,7 +1234,7 @@ int forces_setup(bdb_system* s)
                                       SORT_MAX * (int)sizeof(unsigned long long)));
     }
     BDB_CUDA(h2d(s, s->cell_off.p, off.data(), sizeof(long long) * 2 * nseg));
-    if (s->e_part.alloc(2 * s->n + 16)) return BDB_ERR_NOMEM;
+    if (s->e_part.alloc(2 * s->n + 16) || s->c_part.alloc(2 * s->n)) return BDB_ERR_NOMEM;
     if (s->status.alloc(4)) return BDB_ERR_NOMEM;
     if (s->counts.alloc(2)) return BDB_ERR_NOMEM;
     if (s->F.alloc(3 * s->n) || s->F_save.alloc(3 * s->n) || s->work.alloc(3 * s->n + 16)) return BDB_ERR_NOMEM;
@@ -1091,8 +1250,15 @@ int forces_setup(bdb_system* s)
     if (s->p.elec) c = std::max(c, s->p.cutoff_c);
     if (s->p.alpha_lj != 0) c = std::max(c, s->p.cutoff_lj > 0 ? s->p.cutoff_lj : (double)1.122462f * 2 * maxsig);
     c = std::max(c, s->p.max_force_cutoff);
+    s->reach = c;
     s->skin = std::max(0.5, 0.1 * c);
     s->cell_size = (c + s->skin) * (1 + 1e-12) + 1e-9;
+    // a dense periodic box: 8 beads a cell and more
+    if (s->p.bc == 1 && s->n >= MOVED_MIN) {
+        double cells = nseg;
+        for (int k = 0; k < 3; ++k) cells *= std::max(1.0, std::floor(s->p.box[k] / s->cell_size));
+        if (s->n >= 8 * cells && s->pos_sorted.alloc(s->n3)) return BDB_ERR_NOMEM;
+    }
     return BDB_OK;
 }
 
@@ -1128,18 +1294,24 @@ int forces_run(bdb_system* s, bool want_energy, bool want_counts)
 {
     cudaStream_t st = s->stream;
     const int nseg = (int)s->segs.size();
-    (void)want_counts;
-    BDB_CUDA(cudaMemsetAsync(s->counts.p, 0, 2 * sizeof(unsigned long long), st));
     double3 box = make_double3(s->p.box[0], s->p.box[1], s->p.box[2]);
     int smax = 0;
     for (auto& g : s->segs) smax = std::max(smax, g.count);
     int np = 1;
     while (np < smax) np <<= 1;
     size_t shm = sizeof(unsigned long long) * (size_t)std::min(np, SORT_MAX);
+    int* moved = nullptr;
+    if (s->n >= MOVED_MIN) {
+        moved = s->cells_moved.p;
+        k_moved<<<(s->n + 127) / 128, 128, 0, st>>>(s->n, s->pos.p, s->pos_build.p, s->d_bead_seg.p, s->skin,
+                                                    s->p.bc == 1, box, s->cells_built.p, moved);
+        BDB_CUDA(cudaGetLastError());
+        s->launches += 1;
+    }
     k_cells<<<nseg, 1024, shm, st>>>(s->pos.p, s->d_segs.p, s->cell_size, s->skin, s->p.bc == 1, box,
                                       s->sorted_keys.p, s->sorted_idx.p, s->grid.p, s->grid_dims.p,
                                       s->pos_build.p, s->cells_built.p, s->cell_range.p, s->cell_off.p,
-                                      s->cells_resort.p);
+                                      s->cells_resort.p, moved);
     BDB_CUDA(cudaGetLastError());
     for (int g = 0; g < nseg; ++g) {
         const int cnt = s->segs[g].count;
@@ -1164,15 +1336,20 @@ int forces_run(bdb_system* s, bool want_energy, bool want_counts)
         s->launches += 2;
         BDB_CUDA(cudaGetLastError());
     }
-    double* Fb = s->work.p;
+    // bonded terms into their slots; the non-bonded kernel adds a bead's
+    // slots up, except with external forces, which come between the two
+    double* Fb = has_external(s) ? s->work.p : nullptr;
     if (s->n_terms) {
         BondedArgs A = bonded_args(s);
         k_bonded<<<(s->n_terms + 127) / 128, 128, 0, st>>>(A, s->pos.p, s->contrib.p, s->term_energy.p,
                                                            s->status.p);
         BDB_CUDA(cudaGetLastError());
+    }
+    if (Fb && s->n_terms) {
         k_bonded_gather<<<(s->n + 127) / 128, 128, 0, st>>>(s->n, s->slot_ptr.p, s->slot_list.p,
                                                              s->contrib.p, Fb);
-    } else {
+        s->launches += 1;
+    } else if (Fb) {
         BDB_CUDA(cudaMemsetAsync(Fb, 0, sizeof(double) * 3 * s->n, st));
     }
     BDB_CUDA(cudaGetLastError());
@@ -1195,12 +1372,23 @@ int forces_run(bdb_system* s, bool want_energy, bool want_counts)
         s->launches += 1;
     }
     const int nblk = (s->n * 32 + NB_THREADS - 1) / NB_THREADS;
-    k_nonbonded<<<nblk, NB_THREADS, 0, st>>>(make_fp(s), s->n, s->pos.p, s->Q.p, s->LJ.p, s->d_bead_seg.p,
-                                             s->d_segs.p, s->cell_range.p, s->cell_off.p, s->sorted_idx.p, s->grid.p,
-                                             s->grid_dims.p, s->conn_ptr.p, s->conn_list.p, Fb, s->F.p,
-                                             s->e_part.p, s->counts.p, s->status.p);
+    const double* sp = s->pos_sorted.p;
+    if (sp) {
+        k_sorted_pos<<<(s->n + 127) / 128, 128, 0, st>>>(s->n, s->pos.p, s->d_bead_seg.p, s->grid_dims.p,
+                                                         s->sorted_idx.p, s->pos_sorted.p);
+        BDB_CUDA(cudaGetLastError());
+        s->launches += 1;
+    }
+    auto nonbonded = [&](auto kern) {
+        kern<<<nblk, NB_THREADS, 0, st>>>(make_fp(s), s->n, s->pos.p, s->Q.p, s->LJ.p, s->d_bead_seg.p, s->d_segs.p,
+                                          s->cell_range.p, s->cell_off.p, s->sorted_idx.p, sp, s->grid.p, s->grid_dims.p,
+                                          s->conn_ptr.p, s->conn_list.p, Fb, s->n_terms ? s->slot_ptr.p : nullptr, s->slot_list.p,
+                                          s->contrib.p, s->F.p, s->e_part.p, s->c_part.p, s->status.p);
+    };
+    if (want_energy || want_counts) sp ? nonbonded(k_nonbonded<true, true>) : nonbonded(k_nonbonded<true, false>);
+    else sp ? nonbonded(k_nonbonded<false, true>) : nonbonded(k_nonbonded<false, false>);
     BDB_CUDA(cudaGetLastError());
-    if (want_energy) {
+    if (want_energy || want_counts) {
         TermRanges tr;
         tr.lim[0] = 0;
         tr.lim[1] = s->n_bond;
@@ -1208,10 +1396,11 @@ int forces_run(bdb_system* s, bool want_energy, bool want_counts)
         tr.lim[3] = tr.lim[2] + s->n_angle_cos;
         tr.lim[4] = tr.lim[3] + s->n_dihe;
         tr.lim[5] = tr.lim[4] + s->n_dihe_angle;
-        k_energy_reduce<<<1, 256, 0, st>>>(s->n, s->e_part.p, s->term_energy.p, tr, s->scal.p + 16);
+        k_energy_reduce<<<9, 1024, 0, st>>>(s->n, s->e_part.p, s->c_part.p, s->term_energy.p, tr, s->scal.p + 16,
+                                            s->counts.p);
         BDB_CUDA(cudaGetLastError());
     }
-    s->launches += 2 + (s->n_terms ? 2 : 0) + (want_energy ? 1 : 0);
+    s->launches += 2 + (s->n_terms ? 1 : 0) + (want_energy || want_counts ? 1 : 0);
     s->have_forces = true;
     return BDB_OK;
 }
