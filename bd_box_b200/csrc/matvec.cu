@@ -5,15 +5,19 @@
 //   Rs = L X   (my_dtrmv, myblas.c:94-118)
 // HBM-bound: every element of M is read once per step.
 //
-// Work item = one warp on (strip of 32 rows) x (column segment). A lane
-// owns 4 consecutive columns of every 128-column tile (one 16-byte load of
-// FP32 or two of FP64 per row). For each tile the 32 per-row lane partials
-// go through a per-warp shared-memory transpose, after which lane q adds
-// row q's sum. The transposed part of D F (left of the diagonal)
-// accumulates per column over the strip's 32 rows and is written as one
-// partial per (strip, column); k_mv_finish adds all partials in a fixed
-// order and applies the position update, so results are deterministic.
-// Products are accumulated in FP64.
+// FP64 matrix, and the FP32 matrix of the allocation-free entry point
+// (k_strip_mv): a warp takes a strip of 32 rows and a run of 128-column
+// tiles. A lane owns 4 consecutive columns of a tile (one 16-byte load of FP32
+// or two of FP64 per row). Of every 8 rows' lane partials the lanes keep one
+// row's each, after 7 exchanges (transposing sum), and add it over the run;
+// the last 4 lanes of a row meet once, at the end of the run. The
+// transposed part of D F (right of the diagonal) accumulates per column over
+// the strip's 32 rows and is written as one partial per (strip, column);
+// k_mv_finish adds all partials in a fixed order, so results are
+// deterministic. Products are accumulated in FP64.
+// (Handing every tile's row sums through shared memory, 64 accesses per 32
+// loads, held the earlier kernel to 0.8 TB/s at 3N = 3072 FP32 and 4.2 at
+// 3N = 6003 FP64.)
 #include <cuda_runtime.h>
 
 #include <cudaTypedefs.h>
@@ -29,9 +33,8 @@
 namespace bdb {
 
 static constexpr int STRIP = 32;
-static constexpr int WARPS = 4;
 
-__device__ __forceinline__ void load4(const float* p, double* o)
+__device__ __forceinline__ void load4(const float* p, float* o)
 {
     const float4 v = __ldcs(reinterpret_cast<const float4*>(p));
     o[0] = v.x;
@@ -50,129 +53,186 @@ __device__ __forceinline__ void load4(const double* p, double* o)
     o[3] = b.y;
 }
 
-// rowp: [nseg][n3][2] row partials (Rs, Rf right part); colp: [nstrip][n3]
+static constexpr int MV_TILE = 128;   // columns of a tile: 4 a lane
+
+// warps of a CTA and rows of loads in flight. 3N = 3072 in FP32 has 2,304
+// tiles, one a warp: single-warp CTAs with 4 rows in flight (more CTAs fit)
+// take 19.9 us with the finisher, 24.6 with 4 warps, 26.3 with 4 warps and 8
+// rows. 3N = 6003 in FP64 is bandwidth-bound, 4 warps and 8 rows: 52 us.
 template <typename T>
-__global__ void __launch_bounds__(32 * WARPS)
-k_strip_mv(const T* __restrict__ M, int n3, int npad, int nseg, int seg_cols,
-           const double* __restrict__ F, const double* __restrict__ X, double* __restrict__ rowp,
-           double* __restrict__ colp)
+struct MvShape {
+    static constexpr int warps = sizeof(T) == 4 ? 1 : 4, rows = sizeof(T) == 4 ? 4 : 8;
+};
+
+// Column partials, one per (tile J, strip) on or above the diagonal: strips
+// 0 .. 4 J + 3 of tile J, 128 columns each
+__host__ __device__ inline size_t colp_at(int J, int strip)
 {
-    __shared__ double sF[WARPS][STRIP];
-    __shared__ double red[WARPS][32][STRIP + 1];   // [lane][row] partials of one tile
+    return (size_t)MV_TILE * (2 * (size_t)J * (J + 1) + strip);
+}
+
+// One tile of a strip: PART 0 adds M x to the row sums, PART 1 M f to the row
+// sums and M^T f (f of the strip's rows, sF) to the column sums. MASK: the
+// tile crosses the diagonal (PART 0 takes columns <= row, PART 1 the others)
+// or the matrix's edge.
+template <typename T, int PART, bool MASK>
+__device__ __forceinline__ void mv_tile(const T* __restrict__ M, size_t ld, int n3, int r0, int c,
+                                        const double* __restrict__ w, const double* sF, double* sRow, int lane,
+                                        double (&pc)[4])
+{
+    constexpr int G = MvShape<T>::rows;   // rows of loads in flight, and of an exchange
+    double x[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) x[v] = !MASK || c + v < n3 ? w[c + v] : 0.0;
+#pragma unroll 1
+    for (int g = 0; g < STRIP; g += G) {
+        T m[G][4];
+        double p[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const int r = r0 + g + u;
+            if (!MASK || (r < n3 && c < n3)) {
+                load4(M + (size_t)r * ld + c, m[u]);
+            } else {
+                m[u][0] = m[u][1] = m[u][2] = m[u][3] = (T)0;
+            }
+            if (MASK)
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (c + v >= n3 || (PART == 0 ? c + v > r : c + v <= r)) m[u][v] = (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            const double m0 = m[u][0], m1 = m[u][1], m2 = m[u][2], m3 = m[u][3];
+            p[u] = (m0 * x[0] + m1 * x[1]) + (m2 * x[2] + m3 * x[3]);
+            if (PART == 1) {
+                const double fq = sF[g + u];
+                pc[0] += m0 * fq;
+                pc[1] += m1 * fq;
+                pc[2] += m2 * fq;
+                pc[3] += m3 * fq;
+            }
+        }
+        // the upper lane bits choose a row each: bit 4 the upper half of the
+        // group, and so on down
+#pragma unroll
+        for (int h = G / 2; h > 0; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < G / 2; ++k)
+                if (k < h) {
+                    const bool up = lane & (32 / G * h);
+                    const double give = up ? p[k] : p[k + h], keep = up ? p[k + h] : p[k];
+                    p[k] = keep + __shfl_xor_sync(0xffffffffu, give, 32 / G * h);
+                }
+#pragma unroll
+        for (int o = 16 / G; o > 0; o >>= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], o);
+        if (lane % (32 / G) == 0) sRow[g + lane / (32 / G)] += p[0];
+    }
+}
+
+// the run's row sums go out and start again from zero
+__device__ __forceinline__ void mv_rows(double* sRow, double* __restrict__ dst, int r0, int n3, int lane)
+{
+    __syncwarp();
+    if (r0 + lane < n3) dst[r0 + lane] = sRow[lane];
+    sRow[lane] = 0;
+    __syncwarp();
+}
+
+// rowp: [nseg][n3], row sums of a run: Rs for runs left of the diagonal's
+// tile, the right part of Rf for runs right of it; a run that holds it writes
+// Rs there and Rf to rowp[nseg][n3]. colp: colp_at.
+template <typename T>
+__global__ void __launch_bounds__(32 * MvShape<T>::warps)
+k_strip_mv(const T* __restrict__ M, int n3, size_t ld, int nseg, int seg_tiles, const double* __restrict__ F,
+           const double* __restrict__ X, double* __restrict__ rowp, double* __restrict__ colp)
+{
+    constexpr int WARPS = MvShape<T>::warps;
+    __shared__ double s_f[WARPS][STRIP], s_row[WARPS][STRIP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * WARPS + warp;
-    const int nstrip = (n3 + STRIP - 1) / STRIP;
-    if (item >= nstrip * nseg) return;
-    const int strip = item / nseg, seg = item % nseg;
-    const int r0 = strip * STRIP;
-    const int nrow = min(STRIP, n3 - r0);
-    const int c_beg = seg * seg_cols, c_end = min(n3, c_beg + seg_cols);
-    sF[warp][lane] = lane < nrow ? F[r0 + lane] : 0.0;
-    __syncwarp();
-    double (*rd)[STRIP + 1] = red[warp];
-    double rs_acc = 0, rf_acc = 0;
-    for (int c0 = c_beg; c0 < c_end; c0 += 128) {
-        const int c = c0 + 4 * lane;
-        double x[4], f[4], pc[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const bool ok = c + v < c_end;
-            x[v] = ok ? X[c + v] : 0.0;
-            f[v] = ok ? F[c + v] : 0.0;
+    const int nstrip = (n3 + STRIP - 1) / STRIP, ntile = (n3 + MV_TILE - 1) / MV_TILE;
+    if (item < nstrip * nseg) {
+        const int strip = item / nseg, seg = item % nseg;
+        const int r0 = strip * STRIP, Jd = r0 / MV_TILE;   // the diagonal's tile
+        const int J0 = seg * seg_tiles, J1 = min(ntile, J0 + seg_tiles);
+        const double* sF = s_f[warp];
+        double* sRow = s_row[warp];
+        sRow[lane] = 0;
+        s_f[warp][lane] = r0 + lane < n3 ? F[r0 + lane] : 0.0;
+        __syncwarp();
+        const bool rows_in = r0 + STRIP <= n3;
+        double pc[4] = {0, 0, 0, 0};
+        auto put_cols = [&](int J) {
+            double2* o = reinterpret_cast<double2*>(colp + colp_at(J, strip)) + 2 * lane;
+            o[0] = make_double2(pc[0], pc[1]);
+            o[1] = make_double2(pc[2], pc[3]);
+        };
+        int J = J0;
+        for (; J < min(J1, Jd); ++J) {
+            // columns left of the diagonal's tile: never at the matrix's edge
+            if (rows_in) mv_tile<T, 0, false>(M, ld, n3, r0, MV_TILE * J + 4 * lane, X, sF, sRow, lane, pc);
+            else mv_tile<T, 0, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, X, sF, sRow, lane, pc);
         }
-        const bool lower = c0 + 127 < r0;
-        const bool upper = c0 > r0 + STRIP - 1;
-        // warp-uniform choice: every lane of an interior tile has 4 columns
-        if ((lower || upper) && nrow == STRIP && c0 + 127 < c_end) {
-            // interior tile: 8 rows of loads in flight at a time
-            const double* w = lower ? x : f;
-            double (*dst)[STRIP + 1] = rd;
-#pragma unroll 8
-            for (int q = 0; q < STRIP; ++q) {
-                double m[4];
-                load4(M + (size_t)(r0 + q) * npad + c, m);
-                dst[lane][q] = m[0] * w[0] + m[1] * w[1] + m[2] * w[2] + m[3] * w[3];
-                if (upper) {
-                    const double fq = sF[warp][q];
-                    pc[0] += m[0] * fq;
-                    pc[1] += m[1] * fq;
-                    pc[2] += m[2] * fq;
-                    pc[3] += m[3] * fq;
-                }
-            }
-            __syncwarp();
-            double sum = 0;
-#pragma unroll 8
-            for (int l = 0; l < 32; ++l) sum += dst[l][lane];
-            if (lower) rs_acc += sum; else rf_acc += sum;
-            __syncwarp();
-        } else {
-            // edge tile or tile crossing the diagonal: per element, the L
-            // part (columns <= row) first, then the D part
-            for (int part = 0; part < 2; ++part) {
-                for (int q = 0; q < STRIP; ++q) {
-                    const int r = r0 + q;
-                    double m[4] = {0, 0, 0, 0};
-                    if (q < nrow)
-                        for (int v = 0; v < 4; ++v)
-                            if (c + v < c_end) m[v] = (double)M[(size_t)r * npad + c + v];
-                    double a = 0;
-                    const double fq = sF[warp][q];
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        if (part == 0 && c + v <= r) a += m[v] * x[v];
-                        if (part == 1 && c + v > r) {
-                            a += m[v] * f[v];
-                            pc[v] += m[v] * fq;
-                        }
-                    }
-                    rd[lane][q] = a;
-                }
-                __syncwarp();
-                double sa = 0;
-                for (int l = 0; l < 32; ++l) sa += rd[l][lane];
-                if (part == 0) rs_acc += sa; else rf_acc += sa;
-                __syncwarp();
-            }
+        if (J < J1 && J == Jd) {
+            mv_tile<T, 0, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, X, sF, sRow, lane, pc);
+            mv_rows(sRow, rowp + (size_t)seg * n3, r0, n3, lane);
+            pc[0] = pc[1] = pc[2] = pc[3] = 0;
+            mv_tile<T, 1, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, F, sF, sRow, lane, pc);
+            put_cols(J);
+            ++J;
         }
-        if (!lower) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                if (c + v < c_end && c + v > r0) colp[(size_t)strip * n3 + c + v] = pc[v];
+        for (; J < J1; ++J) {
+            pc[0] = pc[1] = pc[2] = pc[3] = 0;
+            if (rows_in && MV_TILE * (J + 1) <= n3)
+                mv_tile<T, 1, false>(M, ld, n3, r0, MV_TILE * J + 4 * lane, F, sF, sRow, lane, pc);
+            else
+                mv_tile<T, 1, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, F, sF, sRow, lane, pc);
+            put_cols(J);
         }
+        mv_rows(sRow, rowp + (size_t)(J0 <= Jd && Jd < J1 ? nseg : seg) * n3, r0, n3, lane);
     }
-    if (lane < nrow) {
-        rowp[((size_t)seg * n3 + r0 + lane) * 2] = rs_acc;
-        rowp[((size_t)seg * n3 + r0 + lane) * 2 + 1] = rf_acc;
-    }
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // Rs = sum of row partials; Rf = pre * (row partials + dD F + column partials
 // of the strips above). A block covers 32 rows; its 8 thread rows take every
 // 8th strip (4 independent sums each) and are combined in a fixed order.
+// Launched as a programmatic dependent of the product.
 static constexpr int FIN_ROWS = 32, FIN_GROUPS = 8;
 
 __global__ void __launch_bounds__(FIN_ROWS * FIN_GROUPS)
-k_mv_finish(int n3, int nseg, const double* __restrict__ rowp, const double* __restrict__ colp,
+k_mv_finish(int n3, int nseg, int seg_tiles, const double* __restrict__ rowp, const double* __restrict__ colp,
             const double* __restrict__ dD, const double* __restrict__ F, double pre, double* __restrict__ Rf,
             double* __restrict__ Rs, int want_rs)
 {
-    __shared__ double part[FIN_GROUPS][FIN_ROWS + 1];
+    __shared__ double part[FIN_GROUPS][FIN_ROWS + 1], rows[FIN_GROUPS][2][FIN_ROWS + 1];
     const int tx = threadIdx.x % FIN_ROWS, ty = threadIdx.x / FIN_ROWS;
     const int r = blockIdx.x * FIN_ROWS + tx;
-    double c[4] = {0, 0, 0, 0};
+    const int J = r / MV_TILE, gd = J / seg_tiles;   // the row's diagonal tile and the run that holds it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    double c[4] = {0, 0, 0, 0}, s = 0, f = 0;
     if (r < n3) {
         const int nst = (r + STRIP - 1) / STRIP;   // strips st with st * STRIP < r
+        const double* src = colp + colp_at(J, 0) + r % MV_TILE;
         int st = ty, q = 0;
-        for (; st < nst; st += FIN_GROUPS, q = (q + 1) & 3) c[q] += colp[(size_t)st * n3 + r];
+        for (; st < nst; st += FIN_GROUPS, q = (q + 1) & 3) c[q] += src[(size_t)st * MV_TILE];
+        for (int g = ty; g < nseg; g += FIN_GROUPS) {
+            const double v = rowp[(size_t)g * n3 + r];
+            if (g <= gd) s += v;
+            else f += v;
+        }
     }
     part[ty][tx] = (c[0] + c[1]) + (c[2] + c[3]);
+    rows[ty][0][tx] = s;
+    rows[ty][1][tx] = f;
     __syncthreads();
     if (ty == 0 && r < n3) {
-        double s = 0, f = 0;
-        for (int g = 0; g < nseg; ++g) {
-            s += rowp[((size_t)g * n3 + r) * 2];
-            f += rowp[((size_t)g * n3 + r) * 2 + 1];
+        s = 0;
+        f = rowp[(size_t)nseg * n3 + r];
+        for (int g = 0; g < FIN_GROUPS; ++g) {
+            s += rows[g][0][tx];
+            f += rows[g][1][tx];
         }
         f += dD[r] * F[r];
         for (int g = 0; g < FIN_GROUPS; ++g) f += part[g][tx];
@@ -181,11 +241,40 @@ k_mv_finish(int n3, int nseg, const double* __restrict__ rowp, const double* __r
     }
 }
 
-static void mv_finish(cudaStream_t st, int n3, int nseg, const double* rowp, const double* colp, const double* dD,
-                      const double* F, double pre, double* Rf, double* Rs, int want_rs)
+// the product and its finisher on stream st; part: mv_part_doubles
+template <typename T>
+static cudaError_t mv_product(cudaStream_t st, const T* M, int n3, size_t ld, int nseg, int seg_tiles, double* part,
+                              const double* dD, const double* F, const double* X, double pre, double* Rf, double* Rs,
+                              int want_rs, bool finish = true)
 {
-    k_mv_finish<<<(n3 + FIN_ROWS - 1) / FIN_ROWS, FIN_ROWS * FIN_GROUPS, 0, st>>>(n3, nseg, rowp, colp, dD, F, pre, Rf,
-                                                                                Rs, want_rs);
+    constexpr int WARPS = MvShape<T>::warps;
+    const int nstrip = (n3 + STRIP - 1) / STRIP;
+    double* rowp = part;
+    double* colp = part + (size_t)(nseg + 1) * n3;
+    colp += (16 - reinterpret_cast<uintptr_t>(colp) % 16) % 16 / 8;   // pairs are stored
+    k_strip_mv<T><<<(nstrip * nseg + WARPS - 1) / WARPS, 32 * WARPS, 0, st>>>(M, n3, ld, nseg, seg_tiles, F, X, rowp,
+                                                                             colp);
+    if (!finish) return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((n3 + FIN_ROWS - 1) / FIN_ROWS);
+    cfg.blockDim = dim3(FIN_ROWS * FIN_GROUPS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_mv_finish, n3, nseg, seg_tiles, (const double*)rowp, (const double*)colp, dD, F,
+                              pre, Rf, Rs, want_rs);
+}
+
+// doubles of the row and column partials
+static size_t mv_part_doubles(int n3, int nseg)
+{
+    const int ntile = (n3 + MV_TILE - 1) / MV_TILE;
+    return (size_t)(nseg + 1) * n3 + colp_at(ntile, 0) + 2;
 }
 
 // ---------------------------------------------------------------------------
@@ -589,35 +678,27 @@ k_mv_finish_tma(int n3, int ntc, long long T, int G, int slots, const double* __
     }
 }
 
-// column segmentation of the strip products: enough warps for the machine
-// (warps_per_sm per SM), columns in multiples of 128
-static void mv_split(int n3, int warps_per_sm, int sms, int* nseg_out, int* seg_cols_out)
+// runs of column tiles: enough warps for the machine (warps_per_sm per SM)
+static void mv_split(int n3, int warps_per_sm, int sms, int* nseg_out, int* seg_tiles_out)
 {
-    const int nstrip = (n3 + STRIP - 1) / STRIP;
-    int nseg = std::max(1, (sms * warps_per_sm + nstrip - 1) / nstrip);
-    const int seg_cols = ((n3 + nseg - 1) / nseg + 127) / 128 * 128;
-    nseg = (n3 + seg_cols - 1) / seg_cols;
-    *nseg_out = nseg;
-    *seg_cols_out = seg_cols;
+    const int nstrip = (n3 + STRIP - 1) / STRIP, ntile = (n3 + MV_TILE - 1) / MV_TILE;
+    const int seg = std::max(1, (int)((long long)nstrip * ntile / ((long long)sms * warps_per_sm)));
+    *seg_tiles_out = seg;
+    *nseg_out = (ntile + seg - 1) / seg;
 }
 
-static void mv_launch(bdb_system* s, int nseg, int seg_cols, const double* X, double* rowp, double* colp)
+static cudaError_t mv_launch(bdb_system* s, int warps, const double* X, int want_rs, bool finish)
 {
-    const int n3 = s->n3;
-    const int nstrip = (n3 + STRIP - 1) / STRIP;
-    const int blocks = (nstrip * nseg + WARPS - 1) / WARPS;
-    if (s->p.precision == BDB_PREC_FP64)
-        k_strip_mv<double><<<blocks, 32 * WARPS, 0, s->stream>>>(s->M64.p, n3, s->npad, nseg, seg_cols, s->F.p, X,
-                                                                 rowp, colp);
-    else
-        k_strip_mv<float><<<blocks, 32 * WARPS, 0, s->stream>>>(s->M32.p, n3, s->npad, nseg, seg_cols, s->F.p, X,
-                                                                rowp, colp);
+    int nseg, seg_tiles;
+    mv_split(s->n3, warps, s->sm_count, &nseg, &seg_tiles);
+    return mv_product<double>(s->stream, s->M64.p, s->n3, s->npad, nseg, seg_tiles, s->part.p, s->dD.p, s->F.p, X,
+                              s->p.dt / (BDB_KB * s->p.T), s->Rf.p, s->Rs.p, want_rs, finish);
 }
 
-// Autotuning of the segmentation: 8, 16 or 32 warps per SM, each timed
+// Autotuning of the runs: 8, 16 or 32 warps per SM, each timed
 // twice after a warm-up; runs at the first product of a system with
 // autotuning on (before any graph capture).
-static int mv_tune(bdb_system* s, const double* X, double* part)
+static int mv_tune(bdb_system* s, const double* X)
 {
     const int cands[3] = {8, 16, 32};
     float best_ms = 1e30f;
@@ -626,14 +707,10 @@ static int mv_tune(bdb_system* s, const double* X, double* part)
     BDB_CUDA(cudaEventCreate(&e0));
     BDB_CUDA(cudaEventCreate(&e1));
     for (int w : cands) {
-        int nseg, seg_cols;
-        mv_split(s->n3, w, s->sm_count, &nseg, &seg_cols);
-        double* rowp = part;
-        double* colp = part + (size_t)nseg * s->n3 * 2;
-        mv_launch(s, nseg, seg_cols, X, rowp, colp);
+        BDB_CUDA(mv_launch(s, w, X, 0, false));
         BDB_CUDA(cudaEventRecord(e0, s->stream));
-        mv_launch(s, nseg, seg_cols, X, rowp, colp);
-        mv_launch(s, nseg, seg_cols, X, rowp, colp);
+        BDB_CUDA(mv_launch(s, w, X, 0, false));
+        BDB_CUDA(mv_launch(s, w, X, 0, false));
         BDB_CUDA(cudaEventRecord(e1, s->stream));
         BDB_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
@@ -740,30 +817,20 @@ int stored_matvec_step(bdb_system* s) { return stored_matvec_tma(s, true, true);
 int stored_matvec(bdb_system* s, bool want_rs)
 {
     if (s->p.precision != BDB_PREC_FP64) return stored_matvec_tma(s, want_rs);
-    const int n3 = s->n3;
-    const int nstrip = (n3 + STRIP - 1) / STRIP;
-    // room for the largest segmentation any tuning candidate can pick
-    int nseg_max, cols_max;
-    mv_split(n3, 32, s->sm_count, &nseg_max, &cols_max);
-    const size_t need = (size_t)std::max(nseg_max, 1) * n3 * 2 + (size_t)nstrip * n3;
+    // room for the shortest runs any tuning candidate can pick
+    int nseg_max, tiles;
+    mv_split(s->n3, 64, s->sm_count, &nseg_max, &tiles);
+    const size_t need = mv_part_doubles(s->n3, nseg_max);
     if (s->part.n < need) {
         if (s->part.alloc(need)) return BDB_ERR_NOMEM;
     }
     const double* X = want_rs ? s->X.p : s->F.p;   // any valid vector when Rs is not wanted
     if (s->autotune && !s->mv_tuned) {
-        int rc = mv_tune(s, X, s->part.p);
+        int rc = mv_tune(s, X);
         if (rc) return rc;
     }
-    int nseg, seg_cols;
-    mv_split(n3, s->mv_warps, s->sm_count, &nseg, &seg_cols);
-    double* rowp = s->part.p;
-    double* colp = s->part.p + (size_t)nseg * n3 * 2;
-    mv_launch(s, nseg, seg_cols, X, rowp, colp);
-    BDB_CUDA(cudaGetLastError());
+    BDB_CUDA(mv_launch(s, s->mv_warps, X, want_rs, true));
     s->launches += 2;
-    const double pre = s->p.dt / (BDB_KB * s->p.T);
-    mv_finish(s->stream, n3, nseg, rowp, colp, s->dD.p, s->F.p, pre, s->Rf.p, s->Rs.p, want_rs);
-    BDB_CUDA(cudaGetLastError());
     return BDB_OK;
 }
 
@@ -773,9 +840,7 @@ int stored_matvec(bdb_system* s, bool want_rs)
 // device memory instead of a buffer obtained from cudaMalloc.
 
 static constexpr int NOALLOC_MAX_N3 = 3072;              // 1024 beads
-static constexpr int NOALLOC_MAX_SEG = 4;
-static constexpr size_t NOALLOC_SCRATCH =
-    (size_t)NOALLOC_MAX_SEG * NOALLOC_MAX_N3 * 2 + (size_t)(NOALLOC_MAX_N3 / STRIP) * NOALLOC_MAX_N3;
+static constexpr size_t NOALLOC_SCRATCH = 319488;        // doubles (mv_part_doubles at 3N = 3072: 230,402)
 
 // Scratch for row and column partial sums (2.5 MB of doubles), one copy on
 // every device that loads the library, kept until the process exits.
@@ -864,24 +929,13 @@ extern "C" int bdb_stored_matvec_noalloc(const float* M, int n3, int ld, const d
     int rc = noalloc_setup(dev, &scratch, &sms);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int nstrip = (n3 + STRIP - 1) / STRIP;
-    // the segmentation of the system path (16 warps per SM), with no more
-    // column segments than the row partials' share of the array holds
-    int nseg, seg_cols;
-    mv_split(n3, 16, sms, &nseg, &seg_cols);
-    const int max_seg = (int)((NOALLOC_SCRATCH - (size_t)nstrip * n3) / (2 * (size_t)n3));
-    if (nseg > max_seg) {
-        seg_cols = ((n3 + max_seg - 1) / max_seg + 127) / 128 * 128;
-        nseg = (n3 + seg_cols - 1) / seg_cols;
-    }
+    // one tile a warp up to 3N = 3072 (2,304 warps), the array holds that many
+    // row partials at any size it takes
+    int nseg, seg_tiles;
+    mv_split(n3, 16, sms, &nseg, &seg_tiles);
+    if (mv_part_doubles(n3, nseg) > NOALLOC_SCRATCH) return fail(BDB_ERR_ARG, "scratch array too small");
     // every partial that k_mv_finish reads is written first by k_strip_mv,
     // so nothing in the scratch has to start at zero
-    double* rowp = scratch;
-    double* colp = rowp + (size_t)nseg * n3 * 2;
-    const int blocks = (nstrip * nseg + WARPS - 1) / WARPS;
-    k_strip_mv<float><<<blocks, 32 * WARPS, 0, st>>>(M, n3, ld, nseg, seg_cols, F, X, rowp, colp);
-    BDB_CUDA(cudaGetLastError());
-    mv_finish(st, n3, nseg, rowp, colp, dD, F, pre, Rf, Rs, 1);
-    BDB_CUDA(cudaGetLastError());
+    BDB_CUDA(mv_product<float>(st, M, n3, (size_t)ld, nseg, seg_tiles, scratch, dD, F, X, pre, Rf, Rs, 1));
     return BDB_OK;
 }
