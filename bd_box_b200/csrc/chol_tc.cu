@@ -1627,8 +1627,10 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
     BDB_CUDA(launch_potrf(s, st, M, 0, lkk));
     phase_mark_on(s, P_POTRF, st);
     s->launches += 1;
-    BDB_CUDA(cudaEventRecord(ev_potrf, st));
-    BDB_CUDA(cudaStreamWaitEvent(st2, ev_potrf, 0));   // the bulk stream starts after what came before
+    if (nt > 1) {
+        BDB_CUDA(cudaEventRecord(ev_potrf, st));
+        BDB_CUDA(cudaStreamWaitEvent(st2, ev_potrf, 0));   // the bulk stream starts after what came before
+    }
     for (int P = 0; P + 1 < nt; ++P) {
         const int set = P % PANEL_SETS;
         panel_ptrs(s, set, &hi, &lo, &lkk);
@@ -1699,7 +1701,9 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
         BDB_CUDA(cudaEventRecord(ev_potrf, st));
         s->launches += 3;
     }
-    // join the side and bulk streams
+    // join the side and bulk streams (a single panel has not used them: in a
+    // capture the side stream would not belong to it)
+    if (nt == 1) return BDB_OK;
     BDB_CUDA(cudaEventRecord(ev_side, st3));
     BDB_CUDA(cudaStreamWaitEvent(st, ev_side, 0));
     BDB_CUDA(cudaEventRecord(ev_end, st2));
