@@ -18,14 +18,16 @@
 // * The Cholesky factor's derivative dB = B Phi(B^-1 dD B^-T), Phi = lower
 //   triangle with half the diagonal, gives
 //     lambda'^T dB X = <Dbar, dD>,  Dbar = B^-T Phi(v X^T) B^-1,  v = B^T lambda',
-//   formed with two blocked triangular solves (k_gemm_tn, k_trinv64).
-// The forward pass is recomputed from checkpoints every `checkpoint` steps.
+//   formed from the inverse of B by products of full tiles (adjoint_linalg).
+// The forward pass is recomputed from checkpoints every `checkpoint` steps. A
+// segment's steps leave what their reverse needs -- positions, forces, and,
+// where the device has room for them, D and B -- so that each step is factored
+// once more, not twice; the last segment's are kept by the forward pass itself.
 // Precision follows the system's: FP64 throughout for an FP64 system; for a
 // mixed-precision system (FP32 tensor, FP16-split Cholesky) the forward steps
-// are the mixed path's, and the backward's O(n^3) part -- Phi(v X^T), the
-// two blocked triangular solves and their transposes -- runs in FP32 on its
-// FP32 factor, while the O(N^2) tile gradients and force products keep FP64
-// arithmetic and FP64 sums.
+// are the mixed path's, and the backward's O(n^3) part -- the inverse and the
+// products with Phi(v X^T) B^-1 -- runs in FP32 on its FP32 factor, while the
+// O(N^2) tile gradients and force products keep FP64 arithmetic and FP64 sums.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -138,7 +140,7 @@ __device__ __forceinline__ void pair_jvp(double Fm, double dFm, const double* d,
     for (int a = 0; a < 3; ++a) jvp[a] += phi * du[a] + k2 * dd * d[a];
 }
 
-// grad_i += c (dF/dx u)_i and ppart[4 i + k] = c u_i . dF_i/ds_k for the
+// grad_i += c (dF/dx u)_i and ppart[4 i + k] += c u_i . dF_i/ds_k for the
 // scale factors s = (LJ epsilon, LJ sigma, bond H, Debye length), following
 // force_single (calc_func.c:370-409), LJ_force (LJ.c:37-64), electro_force
 // (electro.c:36-56) and bond_calc (bond.c:43-85). One warp per bead: lanes
@@ -217,7 +219,7 @@ __global__ void k_force_jvp(int n, AdjForce fp, const double4* __restrict__ pos,
     }
     if (lane == 0) {
         for (int a = 0; a < 3; ++a) grad[3 * i + a] += c * jvp[a];
-        for (int k = 0; k < 4; ++k) ppart[4 * i + k] = c * pp[k];
+        for (int k = 0; k < 4; ++k) ppart[4 * i + k] += c * pp[k];
     }
 }
 
@@ -289,130 +291,315 @@ __global__ void k_mv2_finish(int n, int nrb, int ncb, const double* __restrict__
     v[a] = sl;
 }
 
-// R = Phi(v X^T): lower triangle, half the diagonal
-template <typename T>
-__global__ void k_phi(int n, const double* __restrict__ v, const double* __restrict__ X, T* __restrict__ R)
-{
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)n * n) return;
-    const int a = (int)(idx / n), b = (int)(idx % n);
-    R[idx] = (T)(a > b ? v[a] * X[b] : (a == b ? 0.5 * v[a] * X[a] : 0.0));
-}
+// The Cholesky factor's adjoint as products of full matrices. With A = B^-1
+// (lower triangular) Dbar = A^T Phi(v X^T) A, and Phi(v X^T) A needs no
+// product: row a of it is v_a times the running sum over c < a of X_c A_c (half
+// of c = a), O(n^2). So with G = Phi A
+//     S = Z + Z^T = A^T G + G^T A,  S_ij = sum over k >= max(i, j),
+// n^3/3 multiply-adds for one half of it and n^3/6 for the inverse, all in
+// 128 x 128 tiles, in about 18 launches; two blocked triangular solves with n
+// right-hand sides take n^3 in 190 launches of narrow updates (n = 3072, FP32:
+// 4.2 ms a step before, 1.35 now).
 
-// out = in^T (n x n, row-major), or out = in + in^T when sym
-template <typename T>
-__global__ void k_transpose(int n, const T* __restrict__ in, T* __restrict__ out, int sym)
-{
-    __shared__ T t[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int r = by + k, c = bx + threadIdx.x;
-        if (r < n && c < n) t[k][threadIdx.x] = in[(size_t)r * n + c];
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int r = bx + k, c = by + threadIdx.x;
-        if (r < n && c < n) {
-            const T tv = t[threadIdx.x][k];
-            out[(size_t)r * n + c] = sym ? in[(size_t)r * n + c] + tv : tv;
-        }
-    }
-}
-
-// inverses of the 64x64 diagonal blocks of the lower-triangular B (ld):
-// Winv[k] row-major 64x64, column c by forward substitution (thread c),
+// inverses of the 64x64 diagonal blocks of the lower-triangular B (ld) into A
+// (n x n, zero above the diagonal), column c by forward substitution: four
+// lanes share a column's dot products (one lane each: 83 us at n = 3072),
 // accumulated in FP64 over the column's entries as stored (T)
 template <typename TM, typename T>
-__global__ void k_trinv64(const TM* __restrict__ B, int ld, T* __restrict__ Winv)
+__global__ void __launch_bounds__(256) k_trinv64(const TM* __restrict__ B, int ld, int n, T* __restrict__ A)
 {
-    __shared__ double Bs[64][65];
-    const int k = blockIdx.x, c = threadIdx.x;
-    const size_t o = (size_t)k * 64;
-    for (int r = 0; r < 64; ++r) Bs[r][c] = c <= r ? (double)B[(o + r) * ld + o + c] : 0.0;
+    extern __shared__ __align__(16) unsigned char trinv_smem[];
+    T(*Bs)[65] = reinterpret_cast<T(*)[65]>(trinv_smem);
+    T(*W)[65] = reinterpret_cast<T(*)[65]>(trinv_smem + sizeof(T) * 64 * 65);
+    __shared__ double dinv[64];
+    const int tid = threadIdx.x, c = tid >> 2, q = tid & 3;
+    const size_t o = (size_t)blockIdx.x * 64;
+    for (int e = tid; e < 64 * 64; e += 256) {
+        const int r = e >> 6, k = e & 63;
+        Bs[r][k] = k <= r ? (T)B[(o + r) * ld + o + k] : (T)0;
+        if (k > r) W[r][k] = (T)0;
+    }
+    if (tid < 64) dinv[tid] = 1.0 / (double)B[(o + tid) * ld + o + tid];
     __syncthreads();
-    T* W = Winv + (size_t)k * 64 * 64;
-    for (int i = 0; i < 64; ++i) {
-        double w;
-        if (i < c) {
-            w = 0.0;
-        } else {
-            double s = i == c ? 1.0 : 0.0;
-            for (int m = c; m < i; ++m) s -= Bs[i][m] * (double)W[m * 64 + c];
-            w = s / Bs[i][i];
-        }
-        W[i * 64 + c] = (T)w;
+    for (int i = 8 * (tid >> 5); i < 64; ++i) {   // rows above the warp's columns are zero
+        double a = 0.0;
+        for (int m = c + q; m < i; m += 4) a += (double)Bs[i][m] * (double)W[m][c];
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        if (q == 0 && i >= c) W[i][c] = (T)(((i == c ? 1.0 : 0.0) - a) * dinv[i]);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int e = tid; e < 64 * 64; e += 256) A[(o + (e >> 6)) * n + o + (e & 63)] = W[e >> 6][e & 63];
+}
+
+// ---- tile products: TILE x TILE (128 or 64) on TILE^2 / 64 threads with 8 x 8
+// outputs each (rows and columns 4 t and TILE/2 + 4 t of the tile), K in steps
+// of 16 through two shared-memory stages; the next step's operands are loaded
+// into registers while the present one is multiplied. FP32 or FP64
+// multiply-adds as the matrices are stored; bound by those.
+static constexpr int GT = 128, GK = 16;
+constexpr int gemm_threads(int tile) { return tile * tile / 64; }
+
+// In FP32 a thread's sums over 64 k are added to their running sums in shared
+// memory (a 64th of the multiply-adds), so that a sum of thousands rounds like
+// one of a hundred.
+static constexpr int GFLUSH = 64;
+
+template <typename T, int TILE>
+struct GemmSmem {
+    T a[2][GK][TILE + 4], b[2][GK][TILE + 4];
+    T sum[sizeof(T) == 4 ? 64 : 1][sizeof(T) == 4 ? gemm_threads(TILE) : 1];
+};
+
+// 8 consecutive elements (16-byte aligned)
+__device__ __forceinline__ void load8(const float* p, float* v)
+{
+    const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+}
+__device__ __forceinline__ void load8(const double* p, double* v)
+{
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(p + k);
+        v[k] = x.x, v[k + 1] = x.y;
     }
 }
 
-// C[M x N] = alpha A^T B + beta C in T (FP64 or FP32) arithmetic; A is
-// K x M (lda, elements TA), B K x N (ldb), C M x N (ldc), all row-major; M,
-// N multiples of 64, K of 16. 64x64 tiles, 256 threads with 4x4 outputs
-// each (rows ty + 16 i, columns tx + 16 j).
-template <typename T, typename TA>
-__global__ void __launch_bounds__(256) k_gemm_tn(int M, int N, int K, T alpha, const TA* __restrict__ A, int lda,
-                                                 const T* __restrict__ B, int ldb, T beta, T* __restrict__ C, int ldc)
+// acc += op(A) B over k0 <= k < k1 (multiples of 16). op(A)(m, k) is
+// A[m lda + k] or, with TA, A[k lda + m]; B(k, c) is B[k ldb + c]. Rows m >= ml
+// and columns c >= nl (multiples of 8) are zero.
+template <typename T, bool TA, int TILE>
+__device__ __forceinline__ void gemm_tile(GemmSmem<T, TILE>& sm, const T* __restrict__ A, size_t lda,
+                                          const T* __restrict__ B, size_t ldb, int k0, int k1, int ml, int nl,
+                                          T (&acc)[8][8])
 {
-    __shared__ T As[16][64 + 2], Bs[16][64 + 2];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    T acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            const int kk = e >> 6, mm = e & 63;
-            As[kk][mm] = (T)A[(size_t)(k0 + kk) * lda + m0 + mm];
-            Bs[kk][mm] = B[(size_t)(k0 + kk) * ldb + n0 + mm];
+    constexpr int NT = gemm_threads(TILE), NP = 2 * TILE / NT;   // pieces of 8 per thread and operand
+    constexpr int HX = TILE / 8;                                 // threads along a tile's side
+    const int tid = threadIdx.x, tx = tid % HX, ty = tid / HX;
+    T ra[NP][8], rb[NP][8];
+    auto load = [&](int k) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const int e = tid + NT * p, kr = e / HX, c8 = 8 * (e % HX);   // a row of TILE in pieces of 8
+            const int mr = e >> 1, k8 = 8 * (e & 1);                      // 16 k of one row
+#pragma unroll
+            for (int u = 0; u < 8; ++u) ra[p][u] = rb[p][u] = (T)0;
+            if (TA) {
+                if (c8 < ml) load8(A + (size_t)(k + kr) * lda + c8, ra[p]);
+            } else {
+                if (mr < ml) load8(A + (size_t)mr * lda + k + k8, ra[p]);
+            }
+            if (c8 < nl) load8(B + (size_t)(k + kr) * ldb + c8, rb[p]);
         }
-        __syncthreads();
+    };
+    auto store = [&](int st) {
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            T a[4], b[4];
+        for (int p = 0; p < NP; ++p) {
+            const int e = tid + NT * p, kr = e / HX, c8 = 8 * (e % HX), mr = e >> 1, k8 = 8 * (e & 1);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = As[kk][ty + 16 * i];
-                b[i] = Bs[kk][tx + 16 * i];
+            for (int u = 0; u < 8; ++u) {
+                if (TA) sm.a[st][kr][c8 + u] = ra[p][u];
+                else sm.a[st][k8 + u][mr] = ra[p][u];
+                sm.b[st][kr][c8 + u] = rb[p][u];
+            }
+        }
+    };
+    if (k0 >= k1) return;
+    load(k0);
+    __syncthreads();   // an earlier product's stages are read
+    int since = 0;
+    store(0);
+    __syncthreads();
+    int st = 0;
+    for (int k = k0; k < k1; k += GK, st ^= 1) {
+        const bool more = k + GK < k1;
+        if (more) load(k + GK);
+#pragma unroll
+        for (int kk = 0; kk < GK; ++kk) {
+            T a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                a[u] = sm.a[st][kk][4 * ty + u];
+                a[4 + u] = sm.a[st][kk][TILE / 2 + 4 * ty + u];
+                b[u] = sm.b[st][kk][4 * tx + u];
+                b[4 + u] = sm.b[st][kk][TILE / 2 + 4 * tx + u];
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
+                for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
+        }
+        if (more) store(st ^ 1);
+        if (sizeof(T) == 4 && ((since += GK) == GFLUSH)) {
+            since = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    sm.sum[8 * i + j][tid] += acc[i][j];
+                    acc[i][j] = (T)0;
+                }
         }
         __syncthreads();
     }
+}
+
+// a thread's sums before and after its products
+template <typename T, int TILE>
+__device__ __forceinline__ void gemm_begin(GemmSmem<T, TILE>& sm, T (&acc)[8][8])
+{
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            T* cp = C + (size_t)(m0 + ty + 16 * i) * ldc + n0 + tx + 16 * j;
-            *cp = beta == (T)0 ? alpha * acc[i][j] : alpha * acc[i][j] + beta * *cp;
+        for (int j = 0; j < 8; ++j) {
+            acc[i][j] = (T)0;
+            if (sizeof(T) == 4) sm.sum[8 * i + j][threadIdx.x] = (T)0;
+        }
+}
+template <typename T, int TILE>
+__device__ __forceinline__ void gemm_end(const GemmSmem<T, TILE>& sm, T (&acc)[8][8])
+{
+    if (sizeof(T) == 4)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] += sm.sum[8 * i + j][threadIdx.x];
+}
+
+// row or column u of a thread's 8
+template <int TILE>
+__device__ __forceinline__ int gemm_at(int t, int u)
+{
+    return (u < 4 ? 0 : TILE / 2 - 4) + 4 * t + u;
+}
+
+// One level of the inverse: blocks of s rows are inverted; pair z joins block
+// 2 z (rows c0) and 2 z + 1 (rows r0, cut at n): A21 = -A22 (B21 A11). STAGE 0:
+// W21 = B21 A11, STAGE 1: A21 = -A22 W21 (W: n x n scratch). 64 x 64 tiles: the
+// levels have few outputs and long sums (n = 3072: 128 tiles of 128 with k up
+// to 2048 at the last one, 0.92 ms in all levels; 0.69 with 64).
+template <typename T, int STAGE>
+__global__ void __launch_bounds__(gemm_threads(64), sizeof(T) == 4 ? 6 : 4)
+k_tri_level(int n, int s, const T* __restrict__ B, int ldb, T* __restrict__ A, T* __restrict__ W)
+{
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    constexpr int TL = 64;
+    GemmSmem<T, TL>& sm = *reinterpret_cast<GemmSmem<T, TL>*>(gemm_smem);
+    const int c0 = 2 * blockIdx.z * s, r0 = c0 + s;
+    const int m0 = blockIdx.y * TL, n0 = blockIdx.x * TL;
+    const int ml = min(s, n - r0) - m0, nl = s - n0;   // rows and columns left
+    if (ml <= 0 || nl <= 0) return;
+    T acc[8][8];
+    gemm_begin(sm, acc);
+    if (STAGE == 0)   // A11 is zero above its diagonal: k >= n0
+        gemm_tile<T, false, TL>(sm, B + (size_t)(r0 + m0) * ldb + c0, ldb, A + (size_t)c0 * n + c0 + n0, n, n0, s, ml, nl,
+                            acc);
+    else              // A22 likewise: k < m0 + 64
+        gemm_tile<T, false, TL>(sm, A + (size_t)(r0 + m0) * n + r0, n, W + (size_t)r0 * n + c0 + n0, n, 0,
+                            min(m0 + TL, min(s, n - r0)), ml, nl, acc);
+    gemm_end(sm, acc);
+    T* O = (STAGE == 0 ? W : A) + (size_t)(r0 + m0) * n + c0 + n0;
+    const int tx = threadIdx.x % (TL / 8), ty = threadIdx.x / (TL / 8);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int r = gemm_at<TL>(ty, i), c = gemm_at<TL>(tx, j);
+            if (r < ml && c < nl) O[(size_t)r * n + c] = STAGE == 0 ? acc[i][j] : -acc[i][j];
         }
 }
 
-template <typename T, typename TA>
-static void gemm_tn(cudaStream_t st, int M, int N, int K, T alpha, const TA* A, int lda, const T* B, int ldb, T beta,
-                    T* C, int ldc)
+// G = Phi(v X^T) A in two passes over blocks of 64 rows: the blocks' sums of
+// X_c A_c, then each block's running sum from those before it (FP64)
+template <typename T>
+__global__ void k_phi_sums(int n, const double* __restrict__ X, const T* __restrict__ A, double* __restrict__ sums)
 {
-    dim3 grid(N / 64, M / 64);
-    k_gemm_tn<T, TA><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    const int b = blockIdx.x * blockDim.x + threadIdx.x, r0 = 64 * blockIdx.y;
+    if (b >= n) return;
+    double a = 0;
+    if (b < r0 + 64)
+        for (int c = r0; c < r0 + 64; ++c) a += X[c] * (double)A[(size_t)c * n + b];
+    sums[(size_t)blockIdx.y * n + b] = a;
+}
+template <typename T>
+__global__ void k_phi_rows(int n, const double* __restrict__ v, const double* __restrict__ X, const T* __restrict__ A,
+                           const double* __restrict__ sums, T* __restrict__ G)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x, r0 = 64 * blockIdx.y;
+    if (b >= n) return;
+    double run = 0;
+    for (int q = b / 64; q < (int)blockIdx.y; ++q) run += sums[(size_t)q * n + b];
+    for (int c = r0; c < r0 + 64; ++c) {
+        const double t = b <= c ? X[c] * (double)A[(size_t)c * n + b] : 0.0;
+        G[(size_t)c * n + b] = (T)(v[c] * (run + 0.5 * t));
+        run += t;
+    }
 }
 
-// Y = B^-T R for the lower-triangular B (ld ldb, n x n, n a multiple of 64),
-// right-looking from the last 64-row block; R (n x n) is overwritten.
-// Winv: inverses of B's diagonal blocks (k_trinv64).
-template <typename T, typename TM>
-static int trsm_lt(bdb_system* s, int n, const TM* B, int ldb, const T* Winv, T* R, T* Y)
+// S pieces: tile (i, j), i >= j, of 128 x 128 over 128 i + sk q <= k <
+// 128 i + sk (q + 1): A^T G + G^T A. The sum over k is longest where tiles are
+// fewest (k >= 128 i), so it is cut into at most 8 pieces (adj_piece): 1,000
+// pieces of 384 at n = 3072 for 296 CTA slots. k_adj_join adds a tile's pieces in order and writes the
+// tile and its mirror image.
+__host__ __device__ inline int adj_piece(int nb) { return GT * (nb > 24 ? (nb + 7) / 8 : 3); }
+__host__ __device__ inline int adj_pieces_of(int nb, int i)
 {
-    const int nb = n / 64;
-    for (int k = nb - 1; k >= 0; --k) {
-        T* Yk = Y + (size_t)k * 64 * n;
-        // Y_k = Winv_k^T R_k
-        gemm_tn<T, T>(s->stream, 64, n, 64, (T)1, Winv + (size_t)k * 64 * 64, 64, R + (size_t)k * 64 * n, n, (T)0, Yk, n);
-        // R_0..k-1 -= B[k, 0:k]^T Y_k
-        if (k > 0)
-            gemm_tn<T, TM>(s->stream, 64 * k, n, 64, (T)-1, B + (size_t)k * 64 * ldb, ldb, Yk, n, (T)1, R, n);
-        s->launches += 1 + (k > 0);
+    const int sk = adj_piece(nb);
+    return (GT * (nb - i) + sk - 1) / sk;
+}
+__host__ __device__ inline int adj_pieces_before(int nb, int i)
+{
+    int p = 0;
+    for (int q = 0; q < i; ++q) p += (q + 1) * adj_pieces_of(nb, q);
+    return p;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
+k_adj_pieces(int n, const T* __restrict__ A, const T* __restrict__ G, T* __restrict__ part)
+{
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    GemmSmem<T, GT>& sm = *reinterpret_cast<GemmSmem<T, GT>*>(gemm_smem);
+    const int nb = n / GT;
+    int i = 0, p = blockIdx.x;
+    while (p >= (i + 1) * adj_pieces_of(nb, i)) p -= (i + 1) * adj_pieces_of(nb, i++);
+    const int np = adj_pieces_of(nb, i), j = p / np, q = p % np;
+    const int sk = adj_piece(nb), k0 = GT * i + sk * q, k1 = min(n, k0 + sk);
+    T acc[8][8];
+    gemm_begin(sm, acc);
+    gemm_tile<T, true, GT>(sm, A + GT * i, n, G + GT * j, n, k0, k1, GT, GT, acc);
+    gemm_tile<T, true, GT>(sm, G + GT * i, n, A + GT * j, n, k0, k1, GT, GT, acc);
+    gemm_end(sm, acc);
+    T* O = part + (size_t)blockIdx.x * GT * GT;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) O[gemm_at<GT>(ty, r) * GT + gemm_at<GT>(tx, c)] = acc[r][c];
+}
+
+// 32 x 32 of tile (i, j) per CTA (blockIdx.z = 0..15)
+template <typename T>
+__global__ void __launch_bounds__(256) k_adj_join(int n, const T* __restrict__ part, T* __restrict__ S)
+{
+    const int i = blockIdx.y, j = blockIdx.x;
+    if (j > i) return;
+    __shared__ T t[32][33];
+    const int nb = n / GT, np = adj_pieces_of(nb, i);
+    const T* src = part + (size_t)(adj_pieces_before(nb, i) + j * np) * GT * GT;
+    const int r0 = 32 * (blockIdx.z >> 2), c0 = 32 * (blockIdx.z & 3);
+    const int x = threadIdx.x & 31;
+    for (int y = threadIdx.x >> 5; y < 32; y += 8) {
+        T a = (T)0;
+        for (int q = 0; q < np; ++q) a += src[(size_t)q * GT * GT + (r0 + y) * GT + c0 + x];
+        t[y][x] = a;
+        S[(size_t)(GT * i + r0 + y) * n + GT * j + c0 + x] = a;
     }
-    BDB_CUDA(cudaGetLastError());
-    return BDB_OK;
+    if (i == j) return;
+    __syncthreads();
+    for (int y = threadIdx.x >> 5; y < 32; y += 8) S[(size_t)(GT * j + c0 + y) * n + GT * i + r0 + x] = t[x][y];
 }
 
 // ---------------------------------------------------------------- driver
@@ -430,24 +617,43 @@ struct Scratch {
     }
 };
 
-// u = D lam and v = B^T lam from the stored matrix M (D upper, B lower),
-// then S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1 into R (T, np x
-// np); Y is scratch of the same size
-template <typename T, typename TM>
-static int adjoint_linalg(bdb_system* s, const TM* M, int np, int n3, int nrb, int ncb, const double* lam,
-                          double* colp, double* rowp, double* u, double* v, const double* Xp, T* R, T* Y, T* Winv)
+// Work buffers of adjoint_linalg, T elements: the inverse (zero above the
+// diagonal), G, S and scratch (each np x np) and the pieces of S
+template <typename T>
+struct AdjLinalg {
+    T *A = nullptr, *G = nullptr, *S = nullptr, *W = nullptr, *part = nullptr;
+    double* sums = nullptr;   // [np / 64][np]
+};
+
+// u = D lam and v = B^T lam from the stored matrix M (D upper, B lower), then
+// S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1
+template <typename T>
+static int adjoint_linalg(bdb_system* s, const T* M, int np, int n3, int nrb, int ncb, const double* lam,
+                          double* colp, double* rowp, double* u, double* v, const double* Xp, const AdjLinalg<T>& w)
 {
     cudaStream_t st = s->stream;
-    k_mv2<TM><<<dim3(ncb, nrb), 256, 0, st>>>(M, n3, np, lam, colp, rowp);
+    const int smem = (int)sizeof(GemmSmem<T, GT>), lev_smem = (int)sizeof(GemmSmem<T, 64>), tri_smem = 2 * 64 * 65 * (int)sizeof(T);
+    BDB_CUDA(cudaFuncSetAttribute(k_trinv64<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem));
+    BDB_CUDA(cudaFuncSetAttribute(k_tri_level<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lev_smem));
+    BDB_CUDA(cudaFuncSetAttribute(k_tri_level<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lev_smem));
+    BDB_CUDA(cudaFuncSetAttribute(k_adj_pieces<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_mv2<T><<<dim3(ncb, nrb), 256, 0, st>>>(M, n3, np, lam, colp, rowp);
     k_mv2_finish<<<(n3 + 255) / 256, 256, 0, st>>>(n3, nrb, ncb, colp, rowp, s->dD.p, lam, u, v);
-    k_phi<T><<<(unsigned)(((size_t)np * np + 255) / 256), 256, 0, st>>>(np, v, Xp, R);
-    k_trinv64<TM, T><<<np / 64, 64, 0, st>>>(M, np, Winv);
-    int rc = trsm_lt<T, TM>(s, np, M, np, Winv, R, Y);
-    if (rc) return rc;
-    k_transpose<T><<<dim3(np / 32, np / 32), dim3(32, 8), 0, st>>>(np, Y, R, 0);
-    if ((rc = trsm_lt<T, TM>(s, np, M, np, Winv, R, Y))) return rc;
-    k_transpose<T><<<dim3(np / 32, np / 32), dim3(32, 8), 0, st>>>(np, Y, R, 1);
-    s->launches += 6;
+    k_trinv64<T, T><<<np / 64, 256, tri_smem, st>>>(M, np, np, w.A);
+    s->launches += 7;
+    for (int h = 64; h < np; h *= 2) {
+        const dim3 grid(h / 64, std::min(h, np - h) / 64, (np + h - 1) / (2 * h));
+        k_tri_level<T, 0><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, w.W);
+        k_tri_level<T, 1><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, w.W);
+        s->launches += 2;
+    }
+    const dim3 cols((np + 127) / 128, np / 64);
+    k_phi_sums<T><<<cols, 128, 0, st>>>(np, Xp, w.A, w.sums);
+    k_phi_rows<T><<<cols, 128, 0, st>>>(np, v, Xp, w.A, w.sums, w.G);
+    const int nb = np / GT;
+    k_adj_pieces<T><<<adj_pieces_before(nb, nb), 256, smem, st>>>(np, w.A, w.G, w.part);
+    k_adj_join<T><<<dim3(nb, nb, 16), 256, 0, st>>>(np, w.part, w.S);
+    BDB_CUDA(cudaGetLastError());
     return BDB_OK;
 }
 
@@ -509,18 +715,32 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
             blist[fill[bp_h[2 * t + 1]]++] = t;
         }
     }
-    const int nck = (K + checkpoint - 1) / checkpoint;
+    const int nck = (K + checkpoint - 1) / checkpoint, seg_len = std::min(K, checkpoint);
     const int nrb = (n3 + MV2_ROWS - 1) / MV2_ROWS, ncb = (n3 + MV2_COLS - 1) / MV2_COLS;
-    Scratch<double> R, Y, Winv, lam, lam2, u, v, Xp, colp, rowp, ppart;
+    const size_t nn = (size_t)np * np, el = mixed ? sizeof(float) : sizeof(double);
+    const size_t pieces = (size_t)adj_pieces_before(np / GT, np / GT) * GT * GT;
+    Scratch<double> sums, lam, lam2, u, v, Xp, colp, rowp, ppart, Fseg;
     Scratch<double4> ckpt, seg, xK;
     Scratch<int> d_bptr, d_blist;
-    if (R.alloc((size_t)np * np) || Y.alloc((size_t)np * np) || Winv.alloc((size_t)np * 64) || lam.alloc(np) ||
+    Scratch<unsigned char> dense, Mseg;
+    if (dense.alloc((4 * nn + pieces) * el) || sums.alloc((size_t)np / 64 * np) || lam.alloc(np) ||
         lam2.alloc(np) || u.alloc(np) || v.alloc(np) || Xp.alloc(np) || colp.alloc((size_t)nrb * n3 * 2) ||
         rowp.alloc((size_t)ncb * n3) || ppart.alloc(4 * (size_t)n) || ckpt.alloc((size_t)nck * n) ||
-        seg.alloc((size_t)checkpoint * n) || xK.alloc(n) || d_bptr.alloc(n + 1) || d_blist.alloc(blist.size()))
+        seg.alloc((size_t)seg_len * n) || Fseg.alloc((size_t)seg_len * n3) || xK.alloc(n) || d_bptr.alloc(n + 1) ||
+        d_blist.alloc(blist.size()))
         return fail(BDB_ERR_NOMEM, "adjoint scratch allocation failed");
+    // a segment's stored matrices, in at most half of the memory that is free
+    bool keep = false;
+    {
+        size_t free_b = 0, total_b = 0;
+        const size_t need = (size_t)seg_len * nn * el;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= free_b / 2) keep = !Mseg.alloc(need);
+        if (!keep) cudaGetLastError();   // too little room is no error: the steps are factored again
+    }
     BDB_CUDA(h2d(s, d_bptr.p, bptr.data(), sizeof(int) * (n + 1)));
     BDB_CUDA(h2d(s, d_blist.p, blist.data(), sizeof(int) * blist.size()));
+    BDB_CUDA(cudaMemsetAsync(dense.p, 0, nn * el, st));   // the inverse: zero above its diagonal
+    BDB_CUDA(cudaMemsetAsync(ppart.p, 0, sizeof(double) * 4 * n, st));
     BDB_CUDA(cudaMemsetAsync(u.p, 0, sizeof(double) * np, st));
     BDB_CUDA(cudaMemsetAsync(v.p, 0, sizeof(double) * np, st));
     BDB_CUDA(cudaMemsetAsync(Xp.p, 0, sizeof(double) * np, st));
@@ -531,12 +751,31 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     BDB_CUDA(cudaStreamSynchronize(st));
     BDB_CUDA(cudaMemsetAsync(s->status.p, 0, sizeof(unsigned), st));
 
+    // one forward step from the current positions; slot >= 0: what its
+    // reverse needs goes to that slot of the segment
+    auto forward = [&](int slot) -> int {
+        int r = 0;
+        if (slot >= 0) {
+            if (!s->have_forces && (r = forces_run(s, false, false))) return r;
+            BDB_CUDA(cudaMemcpyAsync(seg.p + (size_t)slot * n, s->pos.p, sizeof(double4) * n, cudaMemcpyDeviceToDevice,
+                                     st));
+            BDB_CUDA(cudaMemcpyAsync(Fseg.p + (size_t)slot * n3, s->F.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice,
+                                     st));
+        }
+        if ((r = engine_step(s))) return r;
+        if (slot >= 0 && keep)   // refresh 1: the matrix still holds this step's D and B
+            BDB_CUDA(cudaMemcpyAsync(Mseg.p + (size_t)slot * nn * el,
+                                     mixed ? (const void*)s->M32.p : (const void*)s->M64.p, nn * el,
+                                     cudaMemcpyDeviceToDevice, st));
+        return BDB_OK;
+    };
     // forward, keeping the positions at every checkpoint
     for (int k = 0; k < K; ++k) {
         if (k % checkpoint == 0)
             BDB_CUDA(cudaMemcpyAsync(ckpt.p + (size_t)(k / checkpoint) * n, s->pos.p, sizeof(double4) * n,
                                      cudaMemcpyDeviceToDevice, st));
-        if ((rc = engine_step(s))) return rc;
+        const int last0 = (nck - 1) * checkpoint;
+        if ((rc = forward(k >= last0 ? k - last0 : -1))) return rc;
     }
     BDB_CUDA(cudaMemcpyAsync(xK.p, s->pos.p, sizeof(double4) * n, cudaMemcpyDeviceToDevice, st));
 
@@ -575,51 +814,55 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     std::vector<double> pph(4 * (size_t)n);
     const int warps_blocks = (n * 32 + 255) / 256;
 
-    // backward, one checkpoint segment at a time (recomputed forward)
+    // backward, one checkpoint segment at a time (recomputed forward, but for
+    // the last)
     for (int sg = nck - 1; sg >= 0; --sg) {
         const int k0 = sg * checkpoint, k1 = std::min(K, k0 + checkpoint);
-        if ((rc = set_positions(s, ckpt.p + (size_t)sg * n)) || (rc = set_counter(s, base + k0))) return rc;
-        for (int k = k0; k < k1; ++k) {
-            BDB_CUDA(cudaMemcpyAsync(seg.p + (size_t)(k - k0) * n, s->pos.p, sizeof(double4) * n,
-                                     cudaMemcpyDeviceToDevice, st));
-            if ((rc = engine_step(s))) return rc;
+        if (sg < nck - 1) {
+            if ((rc = set_positions(s, ckpt.p + (size_t)sg * n)) || (rc = set_counter(s, base + k0))) return rc;
+            for (int k = k0; k < k1; ++k)
+                if ((rc = forward(k - k0))) return rc;
         }
         for (int k = k1 - 1; k >= k0; --k) {
             // the forward quantities of step k: F(x_k), D(x_k), B(x_k), X_k
-            if ((rc = set_positions(s, seg.p + (size_t)(k - k0) * n)) || (rc = set_counter(s, base + k))) return rc;
-            if ((rc = forces_run(s, false, false)) || (rc = tensor_build(s)) || (rc = factor_run(s)) ||
-                (rc = noise_fill(s, nullptr)))
-                return rc;
+            const int slot = k - k0;
+            const double4* x = seg.p + (size_t)slot * n;
+            const double* Fk = Fseg.p + (size_t)slot * n3;
+            if (!keep && ((rc = set_positions(s, x)) || (rc = tensor_build(s)) || (rc = factor_run(s)))) return rc;
+            if ((rc = set_counter(s, base + k)) || (rc = noise_fill(s, nullptr))) return rc;
             BDB_CUDA(cudaMemcpyAsync(Xp.p, s->X.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
-            // u = D lam, v = B^T lam; S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1
-            if (mixed)
-                rc = adjoint_linalg<float, float>(s, s->M32.p, np, n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p, Xp.p,
-                                                  reinterpret_cast<float*>(R.p), reinterpret_cast<float*>(Y.p),
-                                                  reinterpret_cast<float*>(Winv.p));
-            else
-                rc = adjoint_linalg<double, double>(s, s->M64.p, np, n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p,
-                                                    Xp.p, R.p, Y.p, Winv.p);
-            if (rc) return rc;
+            // u = D lam, v = B^T lam; S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1;
             // lam_k = lam + c (dD/dx : F)^T lam + (d(BX)/dx)^T lam + c (dF/dx) u
-            BDB_CUDA(cudaMemcpyAsync(lam2.p, lam.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
-            if (mixed)
-                k_tile_grad<float><<<warps_blocks, 256, 0, st>>>(n, s->pos.p, s->preDii, s->preDij, c, lam.p, s->F.p,
-                                                                reinterpret_cast<const float*>(R.p), np, lam2.p);
-            else
-                k_tile_grad<double><<<warps_blocks, 256, 0, st>>>(n, s->pos.p, s->preDii, s->preDij, c, lam.p, s->F.p,
-                                                                 R.p, np, lam2.p);
-            k_force_jvp<<<warps_blocks, 256, 0, st>>>(n, fp, s->pos.p, s->Q.p, s->LJ.p, s->conn_ptr.p,
+            auto reverse = [&](auto type, const auto* M) -> int {
+                using T = decltype(type);
+                AdjLinalg<T> w;
+                w.A = reinterpret_cast<T*>(dense.p);
+                w.G = w.A + nn;
+                w.S = w.G + nn;
+                w.W = w.S + nn;
+                w.part = w.W + nn;
+                w.sums = sums.p;
+                const int r = adjoint_linalg<T>(s, keep ? reinterpret_cast<const T*>(Mseg.p) + (size_t)slot * nn : M, np,
+                                                n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p, Xp.p, w);
+                if (r) return r;
+                BDB_CUDA(cudaMemcpyAsync(lam2.p, lam.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
+                k_tile_grad<T><<<warps_blocks, 256, 0, st>>>(n, x, s->preDii, s->preDij, c, lam.p, Fk, w.S, np, lam2.p);
+                return BDB_OK;
+            };
+            rc = mixed ? reverse(0.0f, (const float*)s->M32.p) : reverse(0.0, (const double*)s->M64.p);
+            if (rc) return rc;
+            k_force_jvp<<<warps_blocks, 256, 0, st>>>(n, fp, x, s->Q.p, s->LJ.p, s->conn_ptr.p,
                                                      s->conn_list.p, d_bptr.p, d_blist.p, s->bond_pairs.p,
                                                      s->bond_parms.p, u.p, c, lam2.p, ppart.p);
             BDB_CUDA(cudaGetLastError());
             s->launches += 3;
-            BDB_CUDA(cudaMemcpyAsync(pph.data(), ppart.p, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st));
-            BDB_CUDA(cudaStreamSynchronize(st));
-            for (int i = 0; i < n; ++i)
-                for (int q = 0; q < 4; ++q) gp[q] += pph[4 * (size_t)i + q];
             std::swap(lam.p, lam2.p);
         }
     }
+    BDB_CUDA(cudaMemcpyAsync(pph.data(), ppart.p, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st));
+    BDB_CUDA(cudaStreamSynchronize(st));
+    for (int i = 0; i < n; ++i)
+        for (int q = 0; q < 4; ++q) gp[q] += pph[4 * (size_t)i + q];
     BDB_CUDA(cudaMemcpyAsync(grad_coord, lam.p, sizeof(double) * n3, cudaMemcpyDeviceToHost, st));
     if ((rc = set_positions(s, xK.p)) || (rc = set_counter(s, base + K))) return rc;
     unsigned stw = 0;
