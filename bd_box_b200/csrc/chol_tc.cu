@@ -1288,23 +1288,27 @@ k_syrk_tc2(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ C
 // ------------------------------------------------- FP64 trailing update
 //
 // The plain FP64 path's C -= L_i L_j^T on the FP64 tensor instruction
-// (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind): a persistent CTA of 8
-// warps per 128x128 tile, warp w owning rows 32 (w mod 4).. and columns
-// 64 (w / 4).. as 32 accumulator tiles in registers, initialised from C and
-// stored back (lower triangle only on diagonal tiles, whose upper triangle
-// holds D). The panel rows of tiles i and j stream through shared memory in
-// chunks of 32 columns (cp.async, two stages). The panel solve stores the
-// FP64 panel with each group of 8 columns permuted (column c at 2 (c mod 4)
-// + (c / 4 mod 2)), so a lane's operands of k-steps kk and kk + 4 are
-// adjacent: one 16-byte shared load feeds two k-steps. Rows padded to 40
-// doubles (an 8-row quarter-warp's 16-byte loads then hit distinct banks).
-// Per chunk a warp issues 256 DMMAs from 48 fragment loads; every
-// accumulator takes its k-steps in order, as with natural column order.
-static constexpr int S64_THREADS = 256;
-static constexpr int S64_KC = 32;                        // panel columns per staged chunk
-static constexpr int S64_LD = 40;                        // padded row stride of a staged chunk (doubles)
-static constexpr int S64_CHUNK = PW * S64_LD;            // doubles of one operand chunk
-static constexpr int S64_SMEM = 2 * 2 * S64_CHUNK * 8;   // two stages of A and B chunks: 160 KB
+// (mma.sync m8n8k4 f64; tcgen05 has no FP64): a persistent CTA of 4 warps per
+// 64x128 half tile, warp w owning rows 32 (w mod 2).. and columns 64 (w / 2)..
+// as 32 accumulator tiles in registers, initialised from C and stored back
+// (lower triangle only on diagonal tiles, whose upper triangle holds D; the
+// warp that lies above the diagonal does nothing). Two CTAs fit an SM, so that
+// one multiplies while the other loads or stores its C; a whole tile on 8
+// warps (one CTA, 242 registers a thread) left the FP64 pipe idle meanwhile,
+// and a panel of few tiles left half the SMs without one. (mean launch
+// of a factorisation, n = 1536: 29.5 us before, 18.3 now; n = 6003: 51, 44.) The panel rows
+// stream through shared memory in chunks of 16 columns (cp.async, two
+// stages). The panel solve stores the FP64 panel with each group of 8 columns
+// permuted (column c at 2 (c mod 4) + (c / 4 mod 2)), so a lane's operands of
+// k-steps kk and kk + 4 are adjacent: one 16-byte shared load feeds two
+// k-steps. Rows padded to 24 doubles (a quarter-warp's 16-byte loads then
+// hit distinct banks). Every accumulator takes its k-steps in order.
+static constexpr int S64_THREADS = 128;
+static constexpr int S64_ROWS = 64;                      // rows of a half tile
+static constexpr int S64_KC = 16;                        // panel columns per staged chunk
+static constexpr int S64_LD = 24;                        // padded row stride of a staged chunk (doubles)
+static constexpr int S64_STAGE = (S64_ROWS + PW) * S64_LD;   // doubles of one stage (A and B chunks)
+static constexpr int S64_SMEM = 2 * S64_STAGE * 8;       // two stages: 72 KB
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
 {
@@ -1317,21 +1321,20 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// columns [k0, k0 + 32) of the panel rows of tiles ra (A) and rb (B), as
-// stored (fragment order): 2 x 2048 16-byte pieces, 8 + 8 per thread
-__device__ __forceinline__ void s64_stage(double* As, double* Bs, const double* __restrict__ Lp, int ra, int rb,
-                                          int k0, int tid)
+// columns [k0, k0 + 16) of panel rows ra.. (64, A) and rb.. (128, B), as stored
+// (fragment order): 8 16-byte pieces a row, 12 a thread
+__device__ __forceinline__ void s64_stage(double* st, const double* __restrict__ Lp, int ra, int rb, int k0, int tid)
 {
-    constexpr int PIECES = S64_KC / 2;   // 16-byte pieces per row
+    constexpr int PIECES = S64_KC / 2;
 #pragma unroll
-    for (int q = tid; q < PW * PIECES; q += S64_THREADS) {
+    for (int q = tid; q < (S64_ROWS + PW) * PIECES; q += S64_THREADS) {
         const int r = q / PIECES, c = (q % PIECES) * 2;
-        cp_async16(smem_u32(As + r * S64_LD + c), Lp + (size_t)(ra + r) * PW + k0 + c);
-        cp_async16(smem_u32(Bs + r * S64_LD + c), Lp + (size_t)(rb + r) * PW + k0 + c);
+        const int row = r < S64_ROWS ? ra + r : rb + r - S64_ROWS;
+        cp_async16(smem_u32(st + r * S64_LD + c), Lp + (size_t)row * PW + k0 + c);
     }
 }
 
-__global__ void __launch_bounds__(S64_THREADS, 1) k_syrk64(double* __restrict__ M, int npad,
+__global__ void __launch_bounds__(S64_THREADS, 2) k_syrk64(double* __restrict__ M, int npad,
                                                          const double* __restrict__ Lp, int t0, int ntiles, int mode,
                                                          unsigned* __restrict__ status)
 {
@@ -1346,7 +1349,7 @@ __global__ void __launch_bounds__(S64_THREADS, 1) k_syrk64(double* __restrict__ 
     }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int fr = lane >> 2, fq = lane & 3;
-    const int wr = warp & 3, wc = warp >> 2;
+    const int wr = warp & 1, wc = warp >> 1;
     // a programmatic dependent of the previous kernel on the stream: nothing
     // it produces is read before this. Dependents launch at once after the
     // chain's and the side stream's updates (modes 1, 4), after a bulk
@@ -1355,13 +1358,15 @@ __global__ void __launch_bounds__(S64_THREADS, 1) k_syrk64(double* __restrict__ 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (mode == 1 || mode == 4) asm volatile("griddepcontrol.launch_dependents;");
     constexpr int NCH = PW / S64_KC;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        if (t + (int)gridDim.x >= ntiles) asm volatile("griddepcontrol.launch_dependents;");
+    for (int t = blockIdx.x; t < 2 * ntiles; t += gridDim.x) {
+        if (t + (int)gridDim.x >= 2 * ntiles) asm volatile("griddepcontrol.launch_dependents;");
         int ti, tj;
-        tile_of_mode(t, mode, ti, tj);
-        const int ra = (t0 + ti) * PW, rb = (t0 + tj) * PW;
+        tile_of_mode(t >> 1, mode, ti, tj);
+        const int half = t & 1;
+        const int ra = (t0 + ti) * PW + S64_ROWS * half, rb = (t0 + tj) * PW;
         const bool diag = ti == tj;
-        s64_stage(sm64, sm64 + S64_CHUNK, Lp, ra, rb, 0, tid);
+        const bool work = !(diag && half == 0 && wc == 1);   // else above the diagonal
+        s64_stage(sm64, Lp, ra, rb, 0, tid);
         cp_async_commit();
         double acc[4][8][2];
 #pragma unroll
@@ -1369,53 +1374,56 @@ __global__ void __launch_bounds__(S64_THREADS, 1) k_syrk64(double* __restrict__ 
 #pragma unroll
             for (int ct = 0; ct < 8; ++ct) {
                 const size_t row = (size_t)ra + 32 * wr + 8 * rt + fr;
-                const double2 v = *reinterpret_cast<const double2*>(M + row * npad + rb + 64 * wc + 8 * ct + 2 * fq);
+                const double2 v = work ? *reinterpret_cast<const double2*>(M + row * npad + rb + 64 * wc + 8 * ct + 2 * fq)
+                                       : make_double2(0.0, 0.0);
                 acc[rt][ct][0] = v.x;
                 acc[rt][ct][1] = v.y;
             }
 #pragma unroll 1
         for (int kc = 0; kc < NCH; ++kc) {
-            const double* As = sm64 + (kc & 1) * 2 * S64_CHUNK;
-            const double* Bs = As + S64_CHUNK;
+            const double* As = sm64 + (kc & 1) * S64_STAGE;
+            const double* Bs = As + S64_ROWS * S64_LD;
             if (kc + 1 < NCH) {
-                double* nA = sm64 + ((kc + 1) & 1) * 2 * S64_CHUNK;
-                s64_stage(nA, nA + S64_CHUNK, Lp, ra, rb, (kc + 1) * S64_KC, tid);
+                s64_stage(sm64 + ((kc + 1) & 1) * S64_STAGE, Lp, ra, rb, (kc + 1) * S64_KC, tid);
                 cp_async_commit();
                 cp_async_wait<1>();
             } else {
                 cp_async_wait<0>();
             }
             __syncthreads();
+            if (work) {
 #pragma unroll
-            for (int kk = 0; kk < S64_KC; kk += 8) {
-                // k-steps kk (.x) and kk + 4 (.y) of this lane's fragments
-                double2 a[4], b[8];
+                for (int kk = 0; kk < S64_KC; kk += 8) {
+                    // k-steps kk (.x) and kk + 4 (.y) of this lane's fragments
+                    double2 a[4], b[8];
 #pragma unroll
-                for (int rt = 0; rt < 4; ++rt) {
-                    const double2 v =
-                        *reinterpret_cast<const double2*>(As + (32 * wr + 8 * rt + fr) * S64_LD + kk + 2 * fq);
-                    a[rt] = make_double2(-v.x, -v.y);
+                    for (int rt = 0; rt < 4; ++rt) {
+                        const double2 v =
+                            *reinterpret_cast<const double2*>(As + (32 * wr + 8 * rt + fr) * S64_LD + kk + 2 * fq);
+                        a[rt] = make_double2(-v.x, -v.y);
+                    }
+#pragma unroll
+                    for (int ct = 0; ct < 8; ++ct)
+                        b[ct] = *reinterpret_cast<const double2*>(Bs + (64 * wc + 8 * ct + fr) * S64_LD + kk + 2 * fq);
+#pragma unroll
+                    for (int rt = 0; rt < 4; ++rt)
+#pragma unroll
+                        for (int ct = 0; ct < 8; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], a[rt].x, b[ct].x);
+#pragma unroll
+                    for (int rt = 0; rt < 4; ++rt)
+#pragma unroll
+                        for (int ct = 0; ct < 8; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], a[rt].y, b[ct].y);
                 }
-#pragma unroll
-                for (int ct = 0; ct < 8; ++ct)
-                    b[ct] = *reinterpret_cast<const double2*>(Bs + (64 * wc + 8 * ct + fr) * S64_LD + kk + 2 * fq);
-#pragma unroll
-                for (int rt = 0; rt < 4; ++rt)
-#pragma unroll
-                    for (int ct = 0; ct < 8; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], a[rt].x, b[ct].x);
-#pragma unroll
-                for (int rt = 0; rt < 4; ++rt)
-#pragma unroll
-                    for (int ct = 0; ct < 8; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], a[rt].y, b[ct].y);
             }
             __syncthreads();   // this stage is read; it may be staged again
         }
+        if (!work) continue;
 #pragma unroll
         for (int rt = 0; rt < 4; ++rt)
 #pragma unroll
             for (int ct = 0; ct < 8; ++ct) {
-                const int r = 32 * wr + 8 * rt + fr, c = 64 * wc + 8 * ct + 2 * fq;
-                double* dst = M + ((size_t)ra + r) * npad + rb + c;
+                const int r = S64_ROWS * half + 32 * wr + 8 * rt + fr, c = 64 * wc + 8 * ct + 2 * fq;
+                double* dst = M + ((size_t)ra + 32 * wr + 8 * rt + fr) * npad + rb + c;
                 if (!diag) {
                     *reinterpret_cast<double2*>(dst) = make_double2(acc[rt][ct][0], acc[rt][ct][1]);
                 } else {
@@ -1424,6 +1432,69 @@ __global__ void __launch_bounds__(S64_THREADS, 1) k_syrk64(double* __restrict__ 
                 }
             }
     }
+}
+
+// The chain's update of one diagonal tile (the next block to be factored),
+// C -= L_b L_b^T, spread over 10 CTAs of 32x32 outputs (lower triangle), a warp
+// 16x16, operands straight from the panel in L2 (fragment order): the chain
+// waits for it, and on one or two SMs the FP64 pipe alone takes 10 us. The same
+// bits as k_syrk64.
+static constexpr int S64D_GRID = 10;
+__global__ void __launch_bounds__(128) k_syrk64_diag(double* __restrict__ M, int npad, const double* __restrict__ Lp,
+                                                     int b)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int fr = lane >> 2, fq = lane & 3;
+    int bi, bj;
+    tri_index(blockIdx.x, bi, bj);
+    const int r0 = 32 * bi + 16 * (warp & 1), c0 = 32 * bj + 16 * (warp >> 1);   // within the tile
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (c0 > r0 + 15) return;   // above the diagonal
+    const size_t base = (size_t)b * PW;
+    double acc[2][2][2];
+#pragma unroll
+    for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+        for (int ct = 0; ct < 2; ++ct) {
+            const double2 v = *reinterpret_cast<const double2*>(M + (base + r0 + 8 * rt + fr) * npad + base + c0 + 8 * ct +
+                                                               2 * fq);
+            acc[rt][ct][0] = v.x;
+            acc[rt][ct][1] = v.y;
+        }
+    const double* pa = Lp + (base + r0 + fr) * PW + 2 * fq;
+    const double* pb = Lp + (base + c0 + fr) * PW + 2 * fq;
+#pragma unroll 1
+    for (int k0 = 0; k0 < PW; k0 += 32) {
+        double2 x[4][2], y[4][2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                x[u][h] = *reinterpret_cast<const double2*>(pa + 8 * h * PW + k0 + 8 * u);
+                y[u][h] = *reinterpret_cast<const double2*>(pb + 8 * h * PW + k0 + 8 * u);
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+#pragma unroll
+            for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[u][rt].x, y[u][ct].x);
+#pragma unroll
+            for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[u][rt].y, y[u][ct].y);
+        }
+    }
+#pragma unroll
+    for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+        for (int ct = 0; ct < 2; ++ct) {
+            const int r = r0 + 8 * rt + fr, c = c0 + 8 * ct + 2 * fq;
+            double* dst = M + (base + r) * npad + base + c;
+            if (c <= r) dst[0] = acc[rt][ct][0];
+            if (c + 1 <= r) dst[1] = acc[rt][ct][1];
+        }
 }
 
 // ---------------------------------------------------------------- host side
@@ -1660,7 +1731,7 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
         BDB_CUDA(cudaStreamWaitEvent(st3, ev_top, 0));
         if (P > 0) BDB_CUDA(cudaStreamWaitEvent(st3, ev_b, 0));   // B(P-1)
         if (rem > 1) {
-            BDB_CUDA(update(st3, std::min(rem - 1, side), set, -1, P + 1, rem - 1, 4));
+            BDB_CUDA(update(st3, kPairs ? std::min(rem - 1, side) : side, set, -1, P + 1, rem - 1, 4));
             s->launches += 1;
         }
         BDB_CUDA(cudaEventRecord(ev_side, st3));
@@ -1669,7 +1740,7 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
         BDB_CUDA(cudaStreamWaitEvent(st2, ev_rest, 0));
         phase_mark_on(s, P_SYRK_REST, st2);
         if (rem >= 2) {
-            BDB_CUDA(update(st2, std::min(bulk_sms, rem - 1), set, -1, P + 1, rem - 1, 2));
+            BDB_CUDA(update(st2, kPairs ? std::min(bulk_sms, rem - 1) : bulk_sms, set, -1, P + 1, rem - 1, 2));
             s->launches += 1;
         }
         BDB_CUDA(cudaEventRecord(ev_b, st2));
@@ -1683,7 +1754,7 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
                 // P-1 (deferred there) in the same pass
                 const int ntc = (rem - 2) * (rem - 1) / 2;
                 const int set_prev = kPairs ? (P - 1) % PANEL_SETS : -1;
-                BDB_CUDA(update(st2, std::min(bulk_sms, ntc), set, set_prev, P + 1, ntc, 3));
+                BDB_CUDA(update(st2, kPairs ? std::min(bulk_sms, ntc) : bulk_sms, set, set_prev, P + 1, ntc, 3));
             }
             s->launches += 1;
         }
@@ -1780,19 +1851,22 @@ static int tc64_setup(bdb_system* s)
     return BDB_OK;
 }
 
+// grid: SMs the update may take
 static cudaError_t launch_syrk64(bdb_system* s, int grid, cudaStream_t st, const double* Lp, int t0, int ntiles,
                                  int mode)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    const bool diag = mode == 1 && ntiles == 1;
+    cfg.gridDim = dim3(diag ? S64D_GRID : std::min(2 * grid, 2 * ntiles));
     cfg.blockDim = dim3(S64_THREADS);
-    cfg.dynamicSmemBytes = S64_SMEM;
+    cfg.dynamicSmemBytes = diag ? 0 : S64_SMEM;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (diag) return cudaLaunchKernelEx(&cfg, k_syrk64_diag, s->M64.p, s->npad, Lp, t0);
     return cudaLaunchKernelEx(&cfg, k_syrk64, s->M64.p, s->npad, Lp, t0, ntiles, mode, s->status.p);
 }
 
