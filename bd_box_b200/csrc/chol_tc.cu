@@ -4,11 +4,10 @@
 //
 // M is FP32 (lower triangle: the factor, upper: D, never written here) or
 // FP64 on the FP64 path. Super-panel P covers columns p0 = 128P .. p0+127:
-//   k_potrf128  one CTA factors the 128x128 diagonal block in FP64,
-//               right-looking by 8 columns (each 8x8 pivot block factored and
-//               inverted by the pivot warp while the other warps solve and
-//               update), and
-//               hands L_PP and the inverses W_kk of its 8x8 diagonal tiles on
+//   k_potrf128  one CTA factors the 128x128 diagonal block in FP64 by 8
+//               columns (each 8x8 pivot block factored and inverted by the
+//               pivot warp while the other warps form and solve their
+//               tiles), and hands L_PP and the inverses W_kk of its 8x8 diagonal tiles on
 //               to the panel solve;
 //   k_trsm128   the rows below, X L_PP^T = A, by blocked forward substitution
 //               in FP64 (one warp per 8 rows, DMMA); each row goes to M and,
@@ -196,17 +195,6 @@ __device__ __forceinline__ void f16_split(float x, float scale, __half& hi, __ha
 
 // ------------------------------------------------------------ FP64 panel
 
-// 1/sqrt(x) for x > 0 in FP64: the single-precision estimate (relative
-// error ~2^-22) refined by one Newton-Raphson step y <- y (3 - x y^2) / 2,
-// which squares the error to ~2^-43: far below the FP32 rounding of the
-// factor that leaves this kernel, with half the dependency chain of a
-// second step.
-__device__ __forceinline__ double rsqrt_nr(double x)
-{
-    const double y = (double)rsqrtf((float)x);
-    return y * (1.5 - 0.5 * x * y * y);
-}
-
 // FP64 tensor-core MMA (the only FP64 tensor instruction on sm_100a; the
 // tcgen05 kinds have no FP64): D = A B + C for an 8x8 tile, k = 4. Lane l
 // holds A[l/4][l%4], B[l%4][l/4] and C/D[l/4][2(l%4) + {0,1}].
@@ -217,13 +205,12 @@ __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double
                  : "d"(a), "d"(b));
 }
 
-// 8x8 FP64 tiles in shared memory are kept in MMA fragment order, two
-// k-steps per lane (one 16-byte load per operand and tile):
-//   A order: entry 2 l + h = T[l/4][4h + l%4]   (A fragments of T, and also
-//            the B fragments of T^T)
-//   B order: entry 2 l + h = T[4h + l%4][l/4]   (B fragments of T)
-__device__ __forceinline__ int apos(int r, int c) { return ((r << 2) + (c & 3)) * 2 + (c >> 2); }
-__device__ __forceinline__ int bpos(int r, int c) { return ((c << 2) + (r & 3)) * 2 + (r >> 2); }
+// Every product here is X Y^T of 8x8 tiles, summed over their columns, so the
+// columns may be taken in any order that both operands share: k-step h of a
+// DMMA takes columns 2 q + h (q = lane mod 4). A lane's A fragments of X and B
+// fragments of Y^T are then the pair [l/4][2 (l%4) + {0, 1}], the lane's own
+// elements of a C fragment: tiles are kept by rows, one 16-byte load gives
+// both k-steps, and an accumulator is the next product's operand as it is.
 // tile (g, n), n <= g, of the lower triangle of 16 x 16 tiles
 __device__ __forceinline__ int tix(int g, int n) { return g * (g + 1) / 2 + n; }
 
@@ -237,32 +224,35 @@ __device__ __forceinline__ double rcp_nr(double x)
     return fma(q, fma(-x, q, 1.0), q);
 }
 
-// Factor the 8x8 block in Dg ([8][9], lower triangle) in registers and
-// invert the factor; every lane of the pivot warp runs the whole
-// factorisation (nothing passes between lanes), lane c (c < 8) returns
-// column c of L_kk and of W_kk = L_kk^-1. The elimination runs on the
-// unscaled Schur complements with q_j = 1/a_jj: the next pivot
-// a_{j+1,j+1} -= a_{j+1,j}^2 q_j first (the square is formed while q_j is
-// computed, so one reciprocal and one FMA separate two pivots), then the
-// other entries as a_ic -= a_ij (a_cj q_j), one FMA each after the 7-j
-// scaled column entries. The columns are scaled by r_j = 1/sqrt(a_jj) at
-// the end, and column c of W follows by right-looking forward
-// substitution: w_m = acc_m r_m, then acc_i -= L_im w_m for i > m. It is
-// one straight-line block, so the substitution fills the latency of the
-// reciprocal chain. With kFull (the plain FP64 path) every reciprocal and
-// reciprocal square root takes a second Newton step, which brings it to
-// FP64 rounding.
+// 1/sqrt(x) for the pivots: the hardware's FP64 estimate (~20 bits) and one
+// Newton-Raphson step y <- y + y/2 (1 - x y^2) (2^-40), two with kFull (FP64
+// rounding)
 template <bool kFull>
-__device__ __forceinline__ bool pivot8_inv(const double* Dg, int c, double (&lcol)[8], double (&wcol)[8])
+__device__ __forceinline__ double pivot_rsqrt(double x)
 {
-    double a[8][8];
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+    if (kFull) y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+    return y;
+}
+
+// The 8x8 pivot block and every row that meets it. Dg ([8][DLD], lower
+// triangle) is factored in registers, every lane of the pivot warp the whole
+// of it (nothing passes between lanes): elimination on the unscaled Schur
+// complements with q_j = 1/a_jj, the next pivot a_{j+1,j+1} -= a_{j+1,j}^2 q_j
+// first (the square is formed while q_j is computed, so one reciprocal and
+// one FMA separate two pivots), then the other entries as a_ic -= a_ij t_c, t_c
+// = a_cj q_j. The t_c replace column j; a_jj becomes 1/sqrt(a_jj) = 1/L_jj.
+// Columns [J0, J1).
+static constexpr int DLD = 10;   // row stride of 8x8 blocks kept by rows (16-byte rows, distinct banks)
+
+template <bool kFull, int J0, int J1>
+__device__ __forceinline__ bool pivot8(double (&a)[8][8])
+{
     bool ok = true;
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int k = 0; k <= r; ++k) a[r][k] = Dg[r * 9 + k];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = J0; j < J1; ++j) {
         if (!(a[j][j] > 0.0)) ok = false;
         double q = rcp_nr(a[j][j]);
         if (kFull) q = fma(q, fma(-a[j][j], q, 1.0), q);
@@ -275,34 +265,24 @@ __device__ __forceinline__ bool pivot8_inv(const double* Dg, int c, double (&lco
 #pragma unroll
             for (int k = j + 1; k <= r; ++k)
                 if (r != j + 1) a[r][k] = fma(-a[r][j], t[k], a[r][k]);
-    }
-    double rj[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        double r = rsqrt_nr(a[j][j]);
-        if (kFull) r = r * (1.5 - 0.5 * a[j][j] * r * r);
-        rj[j] = r;
-#pragma unroll
-        for (int i = j; i < 8; ++i) a[i][j] *= r;
-    }
-    double acc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = i == c ? 1.0 : 0.0;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        wcol[m] = m >= c ? acc[m] * rj[m] : 0.0;
-#pragma unroll
-        for (int i = m + 1; i < 8; ++i) acc[i] = fma(-a[i][m], wcol[m], acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        double l = 0.0;
-#pragma unroll
-        for (int k = 0; k <= i; ++k)
-            if (k == c) l = a[i][k];
-        lcol[i] = l;
+        for (int k = j + 1; k < 8; ++k) a[k][j] = t[k];
+        a[j][j] = pivot_rsqrt<kFull>(a[j][j]);
     }
     return ok;
+}
+
+// x L^T = c for one row c per lane, columns [J0, J1), from pivot8's t and
+// 1/L_jj: the rows of L[k+1][k] from those of C[k+1][k], the columns of W_kk =
+// L_kk^-1 from unit rows, the rows of L_kk from those of the block itself. (The
+// scaling by 1/L_jj is left to the end: c_j enters the later columns unscaled.)
+template <int J0, int J1>
+__device__ __forceinline__ void pivot8_row(const double (&t)[8][8], double (&c)[8])
+{
+#pragma unroll
+    for (int j = J0; j < J1; ++j)
+#pragma unroll
+        for (int k = j + 1; k < 8; ++k) c[k] = fma(-c[j], t[k][j], c[k]);
 }
 
 // two consecutive elements of an FP32 or FP64 matrix as doubles, and back
@@ -324,10 +304,11 @@ __device__ __forceinline__ void st_pair(double* p, double a, double b)
 static constexpr int POTRF_THREADS = 512;
 static constexpr int NT = PW / 8;                  // 16 row groups of 8 rows
 static constexpr int NTILE = NT * (NT + 1) / 2;    // 136 tiles in the lower triangle
-// Lt tiles, W_kk, the 8x8 block being factored [8][9], 1/L_jj, and one
-// hand-over slot of two tiles per step
-static constexpr int POTRF_SMEM = (NTILE * 64 + NT * 64 + 80 + NT * 128) * 8;
-// factor hand-off to the panel solve: L_PP tiles then the W_kk, A order
+// Lt tiles, W_kk, the 8x8 block being factored, and per step a hand-over slot
+// of two tiles
+static constexpr int HAND = 8 * DLD + 64;
+static constexpr int POTRF_SMEM = (NTILE * 64 + NT * 64 + 8 * DLD + NT * HAND) * 8;
+// factor hand-off to the panel solve: L_PP tiles then the W_kk, by rows
 static constexpr int PANEL_FAC = (NTILE + NT) * 64;
 
 // row group owned by a warp: warp 0 runs the pivots; warps 4, 8, 12 share
@@ -338,89 +319,98 @@ __device__ __forceinline__ int row_group_of(int warp)
     return (warp & 3) ? 4 + warp - 1 - (warp >> 2) : warp >> 2;
 }
 
-// per-step mbarriers of k_potrf128, each completing exactly once
-struct PotrfBars {
-    uint64_t w[NT];      // W_kk and L_kk published by the pivot warp (32 arrivals)
-    uint64_t lcol[NT];   // every tile of block column k solved (32 per solving warp)
-    uint64_t hand[NT];   // row group k+2's last two tiles and L[k+2][k] handed over (32 arrivals)
+// progress counters of k_potrf128: each is raised by one warp at a time, after
+// what it announces
+struct PotrfFlags {
+    int piv;        // L_kk, W_kk and L[k+1][k] published for k < piv
+    int hand;       // hand-over slots 1 .. hand written
+    int row[NT];    // tiles (g, m), m < row[g], published by row group g's owner
 };
 
-// all 32 lanes wait; false on a time-out or an abort seen by this lane
-__device__ __forceinline__ bool bar_wait0(uint64_t* b, volatile int* abort_flag, uint32_t limit)
+__device__ __forceinline__ void flag_set(int* f, int v)
 {
-    return mbar_wait(smem_u32(b), 0, abort_flag, limit);
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(f)), "r"(v) : "memory");
+}
+
+// all 32 lanes poll until *f >= v, at most `limit` times; false on a time-out
+// or an abort. (An mbarrier's try_wait suspends the warp: it woke 230 cycles
+// after the arrival, a poll sees a flag within about 40; a relaxed wait polls
+// less often and leaves the issue slots to others.)
+__device__ __forceinline__ bool flag_wait(const int* f, int v, volatile int* abort_flag, uint32_t limit,
+                                          bool relaxed = false)
+{
+    bool ok = false;
+    for (uint32_t it = 0; it < limit; ++it) {
+        int x;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(x) : "r"(smem_u32(f)) : "memory");
+        if (x >= v) {
+            ok = true;
+            break;
+        }
+        if ((it & 1023) == 1023 && *abort_flag) break;
+        if (relaxed) __nanosleep(64);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *abort_flag = 1;
+    return ok;
 }
 
 // A solved off-diagonal tile X (C fragments x0, x1 of lane (fr, fq)) of
-// L_PP, tile index t = tix(g, n): to the shared tiles (A order), to the FP64
-// hand-off for the panel solve (the same order) and, in M's precision, to M
+// L_PP, tile index t = tix(g, n): to the FP64 hand-off for the panel solve and,
+// in M's precision, to M
 template <typename T>
-__device__ __forceinline__ void put_tile(double* Lt, double* Wt, T* M, size_t row0, size_t col0, int npad, int t,
-                                         int fr, int fq, double x0, double x1)
+__device__ __forceinline__ void put_tile(double* Wt, T* M, size_t row0, size_t col0, int npad, int t,
+                                         int lane, double x0, double x1)
 {
-    const int p0 = t * 64 + apos(fr, 2 * fq), p1 = t * 64 + apos(fr, 2 * fq + 1);
-    Lt[p0] = x0;
-    Lt[p1] = x1;
-    Wt[p0] = x0;
-    Wt[p1] = x1;
-    st_pair(M + (row0 + fr) * npad + col0 + 2 * fq, x0, x1);
-}
-
-// X = C W^T for an 8x8 tile C held as C fragments (c0, c1) and W in A order
-// (pairs at 2 lane): two DMMAs, the A fragments of C by shuffles
-__device__ __forceinline__ void solve_tile(double c0, double c1, const double* Wk, int lane, int fr, int fq,
-                                           double& x0, double& x1)
-{
-    x0 = 0.0;
-    x1 = 0.0;
-    const double2 wb = *reinterpret_cast<const double2*>(Wk + 2 * lane);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int src = (fr << 2) + 2 * h + (fq >> 1);
-        const double v0 = __shfl_sync(0xffffffffu, c0, src);
-        const double v1 = __shfl_sync(0xffffffffu, c1, src);
-        dmma884(x0, x1, (fq & 1) ? v1 : v0, h ? wb.y : wb.x);
-    }
+    *reinterpret_cast<double2*>(Wt + t * 64 + 2 * lane) = make_double2(x0, x1);
+    st_pair(M + (row0 + (lane >> 2)) * npad + col0 + 2 * (lane & 3), x0, x1);
 }
 
 // FP64 factorisation L_PP of the 128x128 diagonal block (P, P) and the
-// inverses W_kk of its 8x8 diagonal tiles, right-looking over 16 blocks of 8
-// columns with the trailing matrix in registers: the warp owning row group g
-// keeps its tiles (g, n), n <= g, as DMMA accumulators. No CTA-wide barrier
-// orders the steps; per-step mbarriers carry exactly what each warp needs:
-//   pivot warp, step k: factor tile (k, k) and invert it (pivot8_inv, every
-//     lane the whole factorisation) -> publish W_kk; take row group k+1's last two tiles
-//     (k+1, k) and (k+1, k+1), handed over through column k-2 together with
-//     L[k+1][k-1], and apply column k-1 to them; solve L[k+1][k] = C[k+1][k]
-//     W_kk^T -> publish; update tile (k+1, k+1) with it and go on to pivot
-//     k+1;
-//   owner g, step k < g-1: solve L[g][k] = C[g][k] W_kk^T -> publish; for
-//     k < g-2 update tiles n = k+1..g with column k once all of block column
-//     k is solved and step k's hand-over is made; at k = g-2 hand the tiles
-//     (g, g-1), (g, g) over instead and retire.
-// So the pivot chain waits only for one solve of row group k+2, made while
-// the pivot warp factors and inverts the next block, and the bulk updates
-// of a step start after that hand-over, so that they do not stand in front
-// of it on the FP64 pipes (four warps share each). Each solved tile goes to M (FP32) and
-// to the FP64 hand-off Wt for the panel solve (A order: the 136 L_PP tiles,
-// then the 16 W_kk; PANEL_FAC doubles) as soon as it is final, so nothing
-// is left to store at the end. Every wait is bounded: a time-out sets
-// ST_TIMEOUT and every warp runs out to the final barrier.
+// inverses W_kk of its 8x8 diagonal tiles, over 16 blocks of 8 columns. One
+// warp runs the pivots, the warp owning row group g forms its tiles (g, n) left
+// to right, each when its column's turn comes, from tiles in shared memory; no
+// CTA-wide barrier orders the steps, progress counters carry exactly what each
+// warp needs:
+//   pivot warp, step k: factor tile (k, k) (pivot8, every lane the whole
+//     factorisation) with one more row per lane carried along (pivot8_row),
+//     which gives in lanes 0-7 the rows of L[k+1][k], in lanes 8-15 W_kk, in
+//     lanes 16-23 L_kk -> publish all three; update tile (k+1, k+1) with
+//     L[k+1][k] and go on to pivot k+1;
+//   owner g, step k <= g-2: C[g][k] -= sum over m < k of L[g][m] L[k][m]^T (row
+//     group k is complete once pivot k-1 is published), then L[g][k] = C[g][k]
+//     W_kk^T -> publish. Its last two tiles (g, g-1) and (g, g) take every
+//     column as it comes; at k = g-2 they are complete up to it and are handed
+//     to the pivot warp.
+// So the pivot chain holds, per 8 columns, one pivot block (8 reciprocals) and
+// one rank-8 update; the hand-over of row group k+1 (one solve and one update
+// behind pivot k-1) is made while the first half of pivot block k is
+// eliminated. The owners' sums of a step are at most 56 tile products over
+// three schedulers (right-looking updates, 100 in the first steps, stood in
+// front of the hand-over on the FP64 tensor pipes: 3,700 cycles a step there,
+// against 2,000 of the chain itself).
+// Each solved tile goes to M and to the FP64 hand-off Wt for the panel solve
+// (by rows: the 136 L_PP tiles, then the 16 W_kk; PANEL_FAC doubles) as soon as
+// it is final, so nothing is left to store at the end. Every wait is bounded:
+// a time-out sets ST_TIMEOUT and every warp runs out to the final barrier.
+// Bound by the pivot chain's latency: a block by itself took 21.9 us with
+// right-looking updates and mbarriers (FP64 path 23.6);
+// now 16.3 and 17.3.
 template <typename T>
 __global__ void __launch_bounds__(POTRF_THREADS, 1) k_potrf128(T* __restrict__ M, int npad, int P,
                                                             double* __restrict__ Wt, unsigned* __restrict__ status,
                                                             uint32_t wlim)
 {
     extern __shared__ double sh[];
-    double* Lt = sh;                       // [NTILE][64] A order
-    double* Wa = Lt + NTILE * 64;          // [NT][64] W_kk in A order
-    double* Dg = Wa + NT * 64;             // [8][9] diagonal block being factored
-    double* Hd = Dg + 80;                  // [NT][2][64] hand-over slots (C layout)
-    __shared__ PotrfBars bars;
+    double* Lt = sh;                       // [NTILE][64] tiles by rows: M's, then L's
+    double* Wa = Lt + NTILE * 64;          // [NT][64] W_kk by rows
+    double* Dg = Wa + NT * 64;             // [8][DLD] diagonal block being factored
+    double* Hd = Dg + 8 * DLD;             // [NT][HAND] hand-over slots: (g, g-1) as [8][DLD], (g, g) by rows
+    __shared__ PotrfFlags fl;
     __shared__ int bad;
     __shared__ volatile int abort_flag;
     {
-        // the warp roles and barrier counts assume this exact launch shape
+        // the warp roles assume this exact launch shape
         uint32_t dyn;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
         if (blockDim.x != POTRF_THREADS || dyn < (uint32_t)POTRF_SMEM) {
@@ -432,188 +422,184 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) k_potrf128(T* __restrict__ M
     const int fr = lane >> 2, fq = lane & 3;
     const size_t base = (size_t)P * PW;
     const int g = row_group_of(warp);
-    if (tid < NT) {
-        mbar_init(smem_u32(&bars.w[tid]), 32);
-        // solvers of block column k: the pivot warp (row group k+1) and the
-        // owners of row groups k+2..15
-        mbar_init(smem_u32(&bars.lcol[tid]), 32 * (tid < NT - 1 ? NT - 1 - tid : 1));
-        mbar_init(smem_u32(&bars.hand[tid]), 32);
-    }
+    if (tid < NT) fl.row[tid] = 0;
     if (tid == 0) {
+        fl.piv = fl.hand = 0;
         bad = 0;
         abort_flag = 0;
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
     // launched as a programmatic dependent of the update of this block
     // column: the set-up above overlaps its tail, M is read only after it
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == 0) {
         // ---------------------------------------------------- pivot warp
-        // tile (0, 0) to Dg; tiles (1, 0) and (1, 1) (nothing updates them
-        // before step 0) as C fragments
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int c = 2 * fq + e;
-            Dg[fr * 9 + c] = c <= fr ? (double)M[(base + fr) * npad + base + c] : 0.0;
-        }
-        double t1[2], t2[2];
+        // tile (0, 0) to Dg, tiles (1, 0) and (1, 1) to the first hand-over
+        // slot (nothing updates them before step 0)
         {
+            const double2 d = ld_pair(M + (base + fr) * npad + base + 2 * fq);
             const double2 a = ld_pair(M + (base + 8 + fr) * npad + base + 2 * fq);
             const double2 b = ld_pair(M + (base + 8 + fr) * npad + base + 8 + 2 * fq);
-            t1[0] = a.x;
-            t1[1] = a.y;
-            t2[0] = 2 * fq <= fr ? (double)b.x : 0.0;
-            t2[1] = 2 * fq + 1 <= fr ? (double)b.y : 0.0;
+            *reinterpret_cast<double2*>(Dg + fr * DLD + 2 * fq) = d;
+            *reinterpret_cast<double2*>(Hd + fr * DLD + 2 * fq) = a;
+            *reinterpret_cast<double2*>(Hd + 8 * DLD + 2 * lane) = b;
         }
+        __syncwarp();
+        const int role = lane >> 3, row = lane & 7;   // 0: L[k+1][k], 1: W_kk, 2: L_kk, 3: none
         for (int k = 0; k < NT; ++k) {
             // the dependent (block row P+1's solve, 4 CTAs) launches for the
-            // last four steps only: launched at the start, its CTAs held 4
-            // SMs in their wait for the whole factorisation
-            if (k == NT - 4) asm volatile("griddepcontrol.launch_dependents;");
-            __syncwarp();
-            {
-                double lc[8], wc[8];
-                if (!pivot8_inv<sizeof(T) == 8>(Dg, lane & 7, lc, wc) && lane == 0) bad = 1;
-                if (lane < 8) {
+            // last steps only: launched at the start, its CTAs held 4 SMs in
+            // their wait for the whole factorisation
+            if (k == NT - 6) asm volatile("griddepcontrol.launch_dependents;");
+            double a[8][8], c[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int pa = apos(i, lane);
-                        Wa[k * 64 + pa] = wc[i];
-                        Lt[tix(k, k) * 64 + pa] = lc[i];
-                    }
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int j = 0; j <= r; j += 2) {
+                    const double2 v = *reinterpret_cast<const double2*>(Dg + r * DLD + j);
+                    a[r][j] = v.x;
+                    if (j + 1 <= r) a[r][j + 1] = v.y;
                 }
+            bool ok = pivot8<sizeof(T) == 8, 0, 4>(a);
+            // tiles (k+1, k) and (k+1, k+1) through column k-1
+            const double* h0 = Hd + (size_t)k * HAND;
+            if (k + 1 < NT && !flag_wait(&fl.hand, k, &abort_flag, wlim)) break;
+            const double* src = role == 0 ? h0 + row * DLD : Dg + row * DLD;
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const double2 v = *reinterpret_cast<const double2*>(src + j);
+                c[j] = role == 1 ? (row == j ? 1.0 : 0.0) : v.x;
+                c[j + 1] = role == 1 ? (row == j + 1 ? 1.0 : 0.0) : v.y;
             }
-            mbar_arrive(smem_u32(&bars.w[k]));   // release: this lane's writes
+            const double2 t2 = *reinterpret_cast<const double2*>(h0 + 8 * DLD + 2 * lane);
+            pivot8_row<0, 4>(a, c);
+            ok &= pivot8<sizeof(T) == 8, 4, 8>(a);
+            pivot8_row<4, 8>(a, c);
+            if (!ok && lane == 0) bad = 1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) c[j] *= a[j][j];
+            // rows of L and columns of W_kk (zero before its diagonal: so are
+            // c's entries there), one store for all three roles: branches by
+            // role took 170 cycles more. L_kk's upper half is never read.
+            double* dst = role == 0 ? Lt + tix(k + 1, k) * 64 + row * 8
+                          : role == 1 ? Wa + k * 64 + row
+                                      : Lt + tix(k, k) * 64 + row * 8;
+            const int step = role == 1 ? 8 : 1;
+            if (role < 3 && (role > 0 || k + 1 < NT)) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dst[j * step] = c[j];
+            }
+            __syncwarp();
+            if (lane == 0) flag_set(&fl.piv, k + 1);
             if (k + 1 == NT) break;
-            __syncwarp();
-            if (k > 0) {
-                // tiles (k+1, k) and (k+1, k+1) through column k-2 and
-                // L[k+1][k-1] from their owner; column k-1 applied here
-                if (!bar_wait0(&bars.hand[k - 1], &abort_flag, wlim)) break;
-                const double2 a = *reinterpret_cast<const double2*>(Hd + (size_t)(k - 1) * 128 + 2 * lane);
-                const double2 b = *reinterpret_cast<const double2*>(Hd + (size_t)(k - 1) * 128 + 64 + 2 * lane);
-                const double2 u = *reinterpret_cast<const double2*>(Lt + tix(k + 1, k - 1) * 64 + 2 * lane);
-                const double2 v = *reinterpret_cast<const double2*>(Lt + tix(k, k - 1) * 64 + 2 * lane);
-                t1[0] = a.x;
-                t1[1] = a.y;
-                t2[0] = b.x;
-                t2[1] = b.y;
-                dmma884(t1[0], t1[1], -u.x, v.x);
-                dmma884(t1[0], t1[1], -u.y, v.y);
-                dmma884(t2[0], t2[1], -u.x, u.x);
-                dmma884(t2[0], t2[1], -u.y, u.y);
-            }
-            // L[k+1][k] = C[k+1][k] W_kk^T
-            double x0, x1;
-            solve_tile(t1[0], t1[1], Wa + k * 64, lane, fr, fq, x0, x1);
-            Lt[tix(k + 1, k) * 64 + apos(fr, 2 * fq)] = x0;
-            Lt[tix(k + 1, k) * 64 + apos(fr, 2 * fq + 1)] = x1;
-            __syncwarp();
-            mbar_arrive(smem_u32(&bars.lcol[k]));
             // tile (k+1, k+1) -= L[k+1][k] L[k+1][k]^T: the next pivot block
             const double2 av = *reinterpret_cast<const double2*>(Lt + tix(k + 1, k) * 64 + 2 * lane);
-            double e0 = t2[0], e1 = t2[1];
+            double e0 = t2.x, e1 = t2.y, f0 = 0.0, f1 = 0.0;
             dmma884(e0, e1, -av.x, av.x);
-            dmma884(e0, e1, -av.y, av.y);
-            Dg[fr * 9 + 2 * fq] = e0;
-            Dg[fr * 9 + 2 * fq + 1] = e1;
+            dmma884(f0, f1, -av.y, av.y);
+            *reinterpret_cast<double2*>(Dg + fr * DLD + 2 * fq) = make_double2(e0 + f0, e1 + f1);
+            __syncwarp();
         }
     } else if (g == 1) {
         // ------------------------------------------------------ store warp
         // (row group 1 needs no owner: the pivot warp takes its tiles). It
         // copies the pivot warp's results to global memory off the pivot
-        // chain: L_kk and W_kk once published, L[k+1][k] once block column k
-        // is solved; FP64 in A order to Wt, L as FP32 to M
+        // chain, once published: L_kk, W_kk and L[k+1][k]; FP64 to Wt, L in M's
+        // precision to M
         for (int k = 0; k < NT; ++k) {
-            if (!bar_wait0(&bars.w[k], &abort_flag, wlim)) break;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int p = 2 * lane + h, r = p >> 3, c = ((p & 1) << 2) | ((p & 7) >> 1);
-                const double l = Lt[tix(k, k) * 64 + p];
-                Wt[tix(k, k) * 64 + p] = l;
-                Wt[(NTILE + k) * 64 + p] = Wa[k * 64 + p];
-                if (c <= r) M[(base + 8 * k + r) * npad + base + 8 * k + c] = (T)l;
-            }
+            if (!flag_wait(&fl.piv, k + 1, &abort_flag, wlim, true)) break;
+            const double2 l = *reinterpret_cast<const double2*>(Lt + tix(k, k) * 64 + 2 * lane);
+            *reinterpret_cast<double2*>(Wt + tix(k, k) * 64 + 2 * lane) = l;
+            *reinterpret_cast<double2*>(Wt + (NTILE + k) * 64 + 2 * lane) =
+                *reinterpret_cast<const double2*>(Wa + k * 64 + 2 * lane);
+            T* m = M + (base + 8 * k + fr) * npad + base + 8 * k + 2 * fq;
+            if (2 * fq <= fr) m[0] = (T)l.x;
+            if (2 * fq + 1 <= fr) m[1] = (T)l.y;
             if (k + 1 == NT) break;
-            if (!bar_wait0(&bars.lcol[k], &abort_flag, wlim)) break;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int p = 2 * lane + h, r = p >> 3, c = ((p & 1) << 2) | ((p & 7) >> 1);
-                const double l = Lt[tix(k + 1, k) * 64 + p];
-                Wt[tix(k + 1, k) * 64 + p] = l;
-                M[(base + 8 * (k + 1) + r) * npad + base + 8 * k + c] = (T)l;
-            }
+            const double2 x = *reinterpret_cast<const double2*>(Lt + tix(k + 1, k) * 64 + 2 * lane);
+            put_tile(Wt, M, base + 8 * (k + 1), base + 8 * k, npad, tix(k + 1, k), lane, x.x, x.y);
         }
     } else {
         // -------------------------------------------------- tile owners
-        double cacc[NT][2];
+        double s0, s1, d0, d1;   // tiles (g, g-1) and (g, g)
+        {
+            double2 v[NT];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            cacc[n][0] = cacc[n][1] = 0.0;
-            if (n <= g) {
-                const double2 v = ld_pair(M + (base + 8 * g + fr) * npad + base + 8 * n + 2 * fq);
-                cacc[n][0] = (n < g || 2 * fq <= fr) ? v.x : 0.0;
-                cacc[n][1] = (n < g || 2 * fq + 1 <= fr) ? v.y : 0.0;
+            for (int n = 0; n < NT; ++n)
+                if (n <= g) v[n] = ld_pair(M + (base + 8 * g + fr) * npad + base + 8 * n + 2 * fq);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                if (n + 2 <= g) *reinterpret_cast<double2*>(Lt + tix(g, n) * 64 + 2 * lane) = v[n];
+                if (n + 1 == g) s0 = v[n].x, s1 = v[n].y;
+                if (n == g) d0 = v[n].x, d1 = v[n].y;
             }
         }
+        double* Lg = Lt + tix(g, 0) * 64 + 2 * lane;
+        double x0 = 0.0, x1 = 0.0;   // L[g][k-1]
         for (int k = 0; k + 1 < g; ++k) {
-            if (!bar_wait0(&bars.w[k], &abort_flag, wlim)) break;
+            // C[g][k], four running sums
+            double2 c = *reinterpret_cast<const double2*>(Lg + k * 64);
+            {
+                const double* Lk = Lt + tix(k, 0) * 64 + 2 * lane;
+                double p0 = 0.0, p1 = 0.0, q0 = 0.0, q1 = 0.0, r0 = 0.0, r1 = 0.0;
+                int m = 0;
+                for (; m + 2 <= k; m += 2) {
+                    const double2 a0 = *reinterpret_cast<const double2*>(Lg + m * 64);
+                    const double2 b0 = *reinterpret_cast<const double2*>(Lk + m * 64);
+                    const double2 a1 = *reinterpret_cast<const double2*>(Lg + m * 64 + 64);
+                    const double2 b1 = *reinterpret_cast<const double2*>(Lk + m * 64 + 64);
+                    dmma884(c.x, c.y, -a0.x, b0.x);
+                    dmma884(p0, p1, -a0.y, b0.y);
+                    dmma884(q0, q1, -a1.x, b1.x);
+                    dmma884(r0, r1, -a1.y, b1.y);
+                }
+                if (m < k) {
+                    const double2 b0 = *reinterpret_cast<const double2*>(Lk + m * 64);
+                    dmma884(c.x, c.y, -x0, b0.x);
+                    dmma884(p0, p1, -x1, b0.y);
+                }
+                c.x += p0 + (q0 + r0);
+                c.y += p1 + (q1 + r1);
+            }
+            if (k > 0) {
+                // column k-1 of tile (g, g-1)
+                if (!flag_wait(&fl.row[g - 1], k, &abort_flag, wlim)) break;
+                const double2 b = *reinterpret_cast<const double2*>(Lt + tix(g - 1, k - 1) * 64 + 2 * lane);
+                dmma884(s0, s1, -x0, b.x);
+                dmma884(s0, s1, -x1, b.y);
+            }
+            if (!flag_wait(&fl.piv, k + 1, &abort_flag, wlim, k + 4 < g)) break;
             // L[g][k] = C[g][k] W_kk^T
-            double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-                if (t == k) {
-                    c0 = cacc[t][0];
-                    c1 = cacc[t][1];
-                }
-            double x0, x1;
-            solve_tile(c0, c1, Wa + k * 64, lane, fr, fq, x0, x1);
-            put_tile(Lt, Wt, M, base + 8 * g, base + 8 * k, npad, tix(g, k), fr, fq, x0, x1);
+            const double2 wb = *reinterpret_cast<const double2*>(Wa + k * 64 + 2 * lane);
+            double y0 = 0.0, y1 = 0.0;
+            x0 = x1 = 0.0;
+            dmma884(x0, x1, c.x, wb.x);
+            dmma884(y0, y1, c.y, wb.y);
+            x0 += y0;
+            x1 += y1;
+            *reinterpret_cast<double2*>(Lg + k * 64) = make_double2(x0, x1);
             if (k + 2 == g) {
-                // the last two tiles, (g, g-1) and (g, g), through column
-                // k-1, for the pivot warp
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    if (t == g - 1)
-                        *reinterpret_cast<double2*>(Hd + (size_t)k * 128 + 2 * lane) =
-                            make_double2(cacc[t][0], cacc[t][1]);
-                    if (t == g)
-                        *reinterpret_cast<double2*>(Hd + (size_t)k * 128 + 64 + 2 * lane) =
-                            make_double2(cacc[t][0], cacc[t][1]);
-                }
-                __syncwarp();
-                mbar_arrive(smem_u32(&bars.lcol[k]));
-                mbar_arrive(smem_u32(&bars.hand[k]));
-                break;
+                // the last two tiles through column k, for the pivot warp
+                // (whose row g-1 of column k came with W_kk)
+                const double2 b = *reinterpret_cast<const double2*>(Lt + tix(g - 1, k) * 64 + 2 * lane);
+                double t0 = 0.0, t1 = 0.0, u0 = 0.0, u1 = 0.0;
+                dmma884(s0, s1, -x0, b.x);
+                dmma884(t0, t1, -x1, b.y);
+                dmma884(d0, d1, -x0, x0);
+                dmma884(u0, u1, -x1, x1);
+                double* h = Hd + (size_t)(k + 1) * HAND;
+                *reinterpret_cast<double2*>(h + fr * DLD + 2 * fq) = make_double2(s0 + t0, s1 + t1);
+                *reinterpret_cast<double2*>(h + 8 * DLD + 2 * lane) = make_double2(d0 + u0, d1 + u1);
             }
             __syncwarp();
-            mbar_arrive(smem_u32(&bars.lcol[k]));
-            const double2 av = *reinterpret_cast<const double2*>(Lt + tix(g, k) * 64 + 2 * lane);
-            // the bulk updates of step k wait for its hand-over, so that the
-            // solve on the pivot chain does not queue behind them
-            if (!bar_wait0(&bars.hand[k], &abort_flag, wlim) || !bar_wait0(&bars.lcol[k], &abort_flag, wlim)) break;
-            // C[g][n] -= L[g][k] L[n][k]^T for n = k+1..g, four tiles per
-            // batch: their operand loads first (predicated, no branch), then
-            // the MMAs
-#pragma unroll
-            for (int n0 = 1; n0 < NT; n0 += 4) {
-                double2 bv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int n = n0 + u;
-                    const bool act = n < NT && n > k && n <= g;
-                    bv[u] = act ? *reinterpret_cast<const double2*>(Lt + tix(n, k) * 64 + 2 * lane)
-                                : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int n = n0 + u;
-                    if (n < NT && n > k && n <= g) {
-                        dmma884(cacc[n][0], cacc[n][1], -av.x, bv[u].x);
-                        dmma884(cacc[n][0], cacc[n][1], -av.y, bv[u].y);
-                    }
-                }
+            if (lane == 0) {
+                if (k + 2 == g) flag_set(&fl.hand, k + 1);
+                flag_set(&fl.row[g], k + 1);
+            }
+            put_tile(Wt, M, base + 8 * g, base + 8 * k, npad, tix(g, k), lane, x0, x1);
+            if (k + 2 < g) {
+                dmma884(d0, d1, -x0, x0);
+                dmma884(d0, d1, -x1, x1);
             }
         }
     }
@@ -631,7 +617,7 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) k_potrf128(T* __restrict__ M
 // as DMMA accumulators loaded straight from M. For n = 0..15:
 //   X_n = C_n W_nn^T                       (two DMMAs),
 //   C_n' -= X_n L_n'n^T for n' > n         (two DMMAs each),
-// 272 DMMAs per unit; C_n -> A fragments by shuffles. The CTA copies the
+// 272 DMMAs per unit; a C fragment is the next A fragment (k_potrf128's column order). The CTA copies the
 // factor (76 KB) into shared memory once. The grid is persistent: unit u goes
 // to warp slot u mod (8 grid), slots ordered so that the first 4 grid slots
 // put one warp on every SM sub-partition, the next 4 grid a second one.
@@ -641,16 +627,6 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) k_potrf128(T* __restrict__ M
 // doubles; Llo unused).
 static constexpr int TRSM_THREADS = 256;
 static constexpr int TRSM_SMEM = PANEL_FAC * 8;
-
-// A fragment of k-step h of an 8x8 tile held as C fragments (lane (r, q)
-// holds T[r][2q], T[r][2q+1]; the A fragment is T[r][4h + q])
-__device__ __forceinline__ double c2a(double c0, double c1, int h, int fr, int fq)
-{
-    const int src = (fr << 2) + 2 * h + (fq >> 1);
-    const double v0 = __shfl_sync(0xffffffffu, c0, src);
-    const double v1 = __shfl_sync(0xffffffffu, c1, src);
-    return (fq & 1) ? v1 : v0;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(TRSM_THREADS, 1) k_trsm128(T* __restrict__ M, int npad, int P, int unit0, int units,
@@ -707,8 +683,8 @@ __global__ void __launch_bounds__(TRSM_THREADS, 1) k_trsm128(T* __restrict__ M, 
         for (int n = 0; n < 16; ++n) {
             double x0 = 0.0, x1 = 0.0;
             const double2 w = Ws[n * 32 + lane];
-            dmma884(x0, x1, c2a(c[n][0], c[n][1], 0, fr, fq), w.x);
-            dmma884(x0, x1, c2a(c[n][0], c[n][1], 1, fr, fq), w.y);
+            dmma884(x0, x1, c[n][0], w.x);
+            dmma884(x0, x1, c[n][1], w.y);
             const int col = 8 * n + 2 * fq;
             if constexpr (sizeof(T) == 4) {
                 const float o0 = (float)x0, o1 = (float)x1;
@@ -720,19 +696,14 @@ __global__ void __launch_bounds__(TRSM_THREADS, 1) k_trsm128(T* __restrict__ M, 
                 *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(Llo) + row * PW + col) = l;
             } else {
                 st_pair(M + row * npad + base + col, x0, x1);
-                // the FP64 panel in k_syrk64's fragment order: within each
-                // group of 8 columns, column c at 2 (c mod 4) + (c / 4 mod 2)
-                double* pr = reinterpret_cast<double*>(Lhi) + row * PW + 8 * n;
-                pr[(((2 * fq) & 3) << 1) | (fq >> 1)] = x0;
-                pr[(((2 * fq + 1) & 3) << 1) | (fq >> 1)] = x1;
+                st_pair(reinterpret_cast<double*>(Lhi) + row * PW + col, x0, x1);
             }
             if (n < 15) {
-                const double xa0 = -c2a(x0, x1, 0, fr, fq), xa1 = -c2a(x0, x1, 1, fr, fq);
 #pragma unroll
                 for (int n2 = n + 1; n2 < 16; ++n2) {
                     const double2 b = Ls[tix(n2, n) * 32 + lane];
-                    dmma884(c[n2][0], c[n2][1], xa0, b.x);
-                    dmma884(c[n2][0], c[n2][1], xa1, b.y);
+                    dmma884(c[n2][0], c[n2][1], -x0, b.x);
+                    dmma884(c[n2][0], c[n2][1], -x1, b.y);
                 }
             }
         }
@@ -1298,10 +1269,8 @@ k_syrk_tc2(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ C
 // and a panel of few tiles left half the SMs without one. (mean launch
 // of a factorisation, n = 1536: 29.5 us before, 18.3 now; n = 6003: 51, 44.) The panel rows
 // stream through shared memory in chunks of 16 columns (cp.async, two
-// stages). The panel solve stores the FP64 panel with each group of 8 columns
-// permuted (column c at 2 (c mod 4) + (c / 4 mod 2)), so a lane's operands of
-// k-steps kk and kk + 4 are adjacent: one 16-byte shared load feeds two
-// k-steps. Rows padded to 24 doubles (a quarter-warp's 16-byte loads then
+// stages). k-step h of 8 columns takes columns 2 q + h (q = lane mod 4), so one
+// 16-byte shared load feeds two k-steps. Rows padded to 24 doubles (a quarter-warp's 16-byte loads then
 // hit distinct banks). Every accumulator takes its k-steps in order.
 static constexpr int S64_THREADS = 128;
 static constexpr int S64_ROWS = 64;                      // rows of a half tile
@@ -1321,8 +1290,8 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// columns [k0, k0 + 16) of panel rows ra.. (64, A) and rb.. (128, B), as stored
-// (fragment order): 8 16-byte pieces a row, 12 a thread
+// columns [k0, k0 + 16) of panel rows ra.. (64, A) and rb.. (128, B), as stored:
+// 8 16-byte pieces a row, 12 a thread
 __device__ __forceinline__ void s64_stage(double* st, const double* __restrict__ Lp, int ra, int rb, int k0, int tid)
 {
     constexpr int PIECES = S64_KC / 2;
@@ -1394,7 +1363,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_syrk64(double* __restrict__ 
             if (work) {
 #pragma unroll
                 for (int kk = 0; kk < S64_KC; kk += 8) {
-                    // k-steps kk (.x) and kk + 4 (.y) of this lane's fragments
+                    // this lane's fragments of two k-steps
                     double2 a[4], b[8];
 #pragma unroll
                     for (int rt = 0; rt < 4; ++rt) {
@@ -1436,7 +1405,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_syrk64(double* __restrict__ 
 
 // The chain's update of one diagonal tile (the next block to be factored),
 // C -= L_b L_b^T, spread over 10 CTAs of 32x32 outputs (lower triangle), a warp
-// 16x16, operands straight from the panel in L2 (fragment order): the chain
+// 16x16, operands straight from the panel in L2: the chain
 // waits for it, and on one or two SMs the FP64 pipe alone takes 10 us. The same
 // bits as k_syrk64.
 static constexpr int S64D_GRID = 10;
