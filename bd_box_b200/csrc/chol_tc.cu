@@ -14,13 +14,14 @@
 //               on the mixed path, as an FP16 hi/lo pair of the row scaled
 //               by a power of two (k_panel_scale) to two panel buffers;
 //   k_syrk_tc   C -= L_i L_j^T for single 128x128 tiles and block columns
-//               (the diagonal tile, the next two block columns), and
+//               (the next three block columns), and
 //   k_syrk_tc2  for 256x256 blocks on CTA pairs (the columns beyond), two
 //               panels per pass over C, with
 //               L_i L_j^T ~= (Lhi_i Lhi_j^T + Lhi_i Llo_j^T + Llo_i Lhi_j^T)
 //                            / scale^2
 //               (the dropped lo*lo term is ~2^-22 relative: FP32 accuracy);
-//   k_syrk64    the FP64 path's updates on mma.sync.m8n8k4.f64.
+//   k_syrk64    the FP64 path's updates on mma.sync.m8n8k4.f64;
+//   k_syrk_diag the next diagonal tile's update, on both paths.
 //
 // The update kernels are persistent and warp-specialised:
 //   warp 0    TMA producer: per K chunk of 64 columns, four 128x64 FP16
@@ -157,9 +158,8 @@ __device__ __forceinline__ void tri_index(int idx, int& ti, int& tj)
 }
 
 // tile t of a launch -> (ti, tj) relative to the first trailing block:
-// mode 0 all tiles of the lower triangle, 1 only block column 0, 2 only
-// block column 1, 3 block columns 2 and beyond, 4 block column 0 below its
-// diagonal tile, 5 only block column 2
+// mode 2 only block column 1, 3 block columns 2 and beyond, 4 block column 0
+// below its diagonal tile (which is k_syrk_diag's), 5 only block column 2
 __device__ __forceinline__ void tile_of_mode(int t, int mode, int& ti, int& tj)
 {
     if (mode == 5) {
@@ -168,15 +168,13 @@ __device__ __forceinline__ void tile_of_mode(int t, int mode, int& ti, int& tj)
     } else if (mode == 4) {
         ti = t + 1;
         tj = 0;
-    } else if (mode == 1 || mode == 2) {
-        tj = mode - 1;
-        ti = t + tj;
+    } else if (mode == 2) {
+        ti = t + 1;
+        tj = 1;
     } else {
         tri_index(t, ti, tj);
-        if (mode == 3) {
-            ti += 2;
-            tj += 2;
-        }
+        ti += 2;
+        tj += 2;
     }
 }
 
@@ -773,14 +771,13 @@ k_syrk_tc(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CU
     // stream: the set-up above overlaps its tail; nothing below may read or
     // write what it produces before this wait (a no-op for a plain launch)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // The chain's and the side stream's updates (modes 1 and 4) let their
-    // dependents launch at once (a one-CTA factorisation; a plain launch).
+    // The side stream's update (mode 4) lets its dependent launch at once.
     // A bulk update's dependent is the next bulk update, a full grid of CTAs
     // that, launched early, would sit on every free SM in its
     // griddepcontrol.wait for as long as this launch runs, SMs the chain
     // needs meanwhile: bulk updates release it only once their last loads
     // are issued (below).
-    if (mode == 1 || mode == 4) asm volatile("griddepcontrol.launch_dependents;");
+    if (mode == 4) asm volatile("griddepcontrol.launch_dependents;");
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1321,11 +1318,11 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_syrk64(double* __restrict__ 
     const int wr = warp & 1, wc = warp >> 1;
     // a programmatic dependent of the previous kernel on the stream: nothing
     // it produces is read before this. Dependents launch at once after the
-    // chain's and the side stream's updates (modes 1, 4), after a bulk
+    // side stream's update (mode 4), after a bulk
     // update only when each CTA starts its last tile (a bulk dependent
     // launched early would hold free SMs in its wait)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (mode == 1 || mode == 4) asm volatile("griddepcontrol.launch_dependents;");
+    if (mode == 4) asm volatile("griddepcontrol.launch_dependents;");
     constexpr int NCH = PW / S64_KC;
     for (int t = blockIdx.x; t < 2 * ntiles; t += gridDim.x) {
         if (t + (int)gridDim.x >= 2 * ntiles) asm volatile("griddepcontrol.launch_dependents;");
@@ -1403,66 +1400,79 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_syrk64(double* __restrict__ 
     }
 }
 
-// The chain's update of one diagonal tile (the next block to be factored),
-// C -= L_b L_b^T, spread over 10 CTAs of 32x32 outputs (lower triangle), a warp
-// 16x16, operands straight from the panel in L2: the chain
-// waits for it, and on one or two SMs the FP64 pipe alone takes 10 us. The same
-// bits as k_syrk64.
-static constexpr int S64D_GRID = 10;
-__global__ void __launch_bounds__(128) k_syrk64_diag(double* __restrict__ M, int npad, const double* __restrict__ Lp,
-                                                     int b)
+// The chain's update of one diagonal tile (block b, the next to be factored)
+// with panel b-1, C -= L_b L_b^T, in FP64 from M's own rows (in L2: the panel
+// solve has just written them), on both precisions' paths. The chain waits for
+// it, so it is spread over 10 CTAs of 32x32 outputs (lower triangle), a warp
+// 16x16, and its 2 x 32 panel rows are staged at once (one load latency). Bound
+// by launch and that latency. FP64: on one or two SMs the FP64 pipe alone takes
+// 10 us; the same bits as k_syrk64. Mixed: one tensor-core CTA set up its tensor
+// memory, loaded split panels and went through all stages for one tile (a
+// predictor-corrector step at 3N = 3003 took 1653 us with it, 1603 with this;
+// rounded once a panel as there, its products exact).
+static constexpr int SYRKD_GRID = 10, SYRKD_LD = PW + 8;   // (rows in distinct banks)
+template <typename T>
+static constexpr int SYRKD_SMEM = 64 * SYRKD_LD * (int)sizeof(T);
+template <typename T>
+__global__ void __launch_bounds__(128) k_syrk_diag(T* __restrict__ M, int npad, int b)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ __align__(16) unsigned char syrkd_smem[];
+    T* Ls = reinterpret_cast<T*>(syrkd_smem);   // [32 rows of block row bi, 32 of bj][LD]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int fr = lane >> 2, fq = lane & 3;
     int bi, bj;
     tri_index(blockIdx.x, bi, bj);
-    const int r0 = 32 * bi + 16 * (warp & 1), c0 = 32 * bj + 16 * (warp >> 1);   // within the tile
+    const int rw = 16 * (warp & 1), cw = 16 * (warp >> 1);
+    const int r0 = 32 * bi + rw, c0 = 32 * bj + cw;   // within the tile
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
-    if (c0 > r0 + 15) return;   // above the diagonal
     const size_t base = (size_t)b * PW;
+    constexpr int VE = 16 / (int)sizeof(T), PIECES = PW / VE;
+    for (int e = tid; e < 64 * PIECES; e += 128) {
+        const int r = e / PIECES, c = VE * (e % PIECES);
+        const size_t row = base + (r < 32 ? 32 * bi + r : 32 * bj + r - 32);
+        cp_async16(smem_u32(Ls + r * SYRKD_LD + c), M + row * npad + base - PW + c);
+    }
+    cp_async_commit();
     double acc[2][2][2];
 #pragma unroll
     for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
         for (int ct = 0; ct < 2; ++ct) {
-            const double2 v = *reinterpret_cast<const double2*>(M + (base + r0 + 8 * rt + fr) * npad + base + c0 + 8 * ct +
-                                                               2 * fq);
+            const double2 v = ld_pair(M + (base + r0 + 8 * rt + fr) * npad + base + c0 + 8 * ct + 2 * fq);
             acc[rt][ct][0] = v.x;
             acc[rt][ct][1] = v.y;
         }
-    const double* pa = Lp + (base + r0 + fr) * PW + 2 * fq;
-    const double* pb = Lp + (base + c0 + fr) * PW + 2 * fq;
-#pragma unroll 1
-    for (int k0 = 0; k0 < PW; k0 += 32) {
-        double2 x[4][2], y[4][2];
+    cp_async_wait<0>();
+    __syncthreads();
+    if (c0 > r0 + 15) return;   // above the diagonal
+    const T* pa = Ls + (rw + fr) * SYRKD_LD + 2 * fq;
+    const T* pb = Ls + (32 + cw + fr) * SYRKD_LD + 2 * fq;
+#pragma unroll 4
+    for (int k = 0; k < PW; k += 8) {
+        double2 x[2], y[2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                x[u][h] = *reinterpret_cast<const double2*>(pa + 8 * h * PW + k0 + 8 * u);
-                y[u][h] = *reinterpret_cast<const double2*>(pb + 8 * h * PW + k0 + 8 * u);
-            }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-            for (int rt = 0; rt < 2; ++rt)
-#pragma unroll
-                for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[u][rt].x, y[u][ct].x);
-#pragma unroll
-            for (int rt = 0; rt < 2; ++rt)
-#pragma unroll
-                for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[u][rt].y, y[u][ct].y);
+        for (int h = 0; h < 2; ++h) {
+            x[h] = ld_pair(pa + 8 * h * SYRKD_LD + k);
+            y[h] = ld_pair(pb + 8 * h * SYRKD_LD + k);
         }
+#pragma unroll
+        for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+            for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[rt].x, y[ct].x);
+#pragma unroll
+        for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+            for (int ct = 0; ct < 2; ++ct) dmma884(acc[rt][ct][0], acc[rt][ct][1], -x[rt].y, y[ct].y);
     }
 #pragma unroll
     for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
         for (int ct = 0; ct < 2; ++ct) {
             const int r = r0 + 8 * rt + fr, c = c0 + 8 * ct + 2 * fq;
-            double* dst = M + (base + r) * npad + base + c;
-            if (c <= r) dst[0] = acc[rt][ct][0];
-            if (c + 1 <= r) dst[1] = acc[rt][ct][1];
+            T* dst = M + (base + r) * npad + base + c;
+            if (c <= r) dst[0] = (T)acc[rt][ct][0];
+            if (c + 1 <= r) dst[1] = (T)acc[rt][ct][1];
         }
 }
 
@@ -1529,6 +1539,7 @@ static int tc_setup(bdb_system* s)
     BDB_CUDA(cudaFuncSetAttribute(k_syrk_tc2, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRK_SMEM));
     if (s->pscale.alloc(2)) return BDB_ERR_NOMEM;
     BDB_CUDA(cudaFuncSetAttribute(k_potrf128<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, POTRF_SMEM));
+    BDB_CUDA(cudaFuncSetAttribute(k_syrk_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRKD_SMEM<float>));
     BDB_CUDA(cudaFuncSetAttribute(k_trsm128<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM));
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1583,7 +1594,24 @@ static cudaError_t launch_syrk_pair(bdb_system* s, int clusters, cudaStream_t st
                               (uint32_t)s->wait_limit, (const float*)s->pscale.p);
 }
 
-// k_potrf128 the same way, behind the update of its block column
+// the chain's kernels the same way: the next diagonal tile's update, and its
+// factorisation behind it
+template <typename T>
+static cudaError_t launch_syrk_diag(bdb_system* s, cudaStream_t st, T* M, int b)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SYRKD_GRID);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = SYRKD_SMEM<T>;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_syrk_diag<T>, M, s->npad, b);
+}
+
 template <typename T>
 static cudaError_t launch_potrf(bdb_system* s, cudaStream_t st, T* M, int P, double* lkk)
 {
@@ -1730,7 +1758,7 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
         phase_mark_on(s, P_SYRK_REST, st2);
         // chain: the diagonal tile of block column P+1, then its factorisation
         phase_mark_on(s, P_SYRK_COL, st);
-        BDB_CUDA(update(st, 1, set, -1, P + 1, 1, 1));
+        BDB_CUDA(launch_syrk_diag(s, st, M, P + 1));
         phase_mark_on(s, P_SYRK_COL, st);
         double* lkk1;
         float *hi1, *lo1;
@@ -1810,6 +1838,7 @@ static int tc64_setup(bdb_system* s)
     if (s->panel64.alloc((size_t)PANEL_SETS * pan + (size_t)PANEL_SETS * PANEL_FAC + 64)) return BDB_ERR_NOMEM;
     BDB_CUDA(dzero(s, s->panel64.p, s->panel64.n * sizeof(double)));
     BDB_CUDA(cudaFuncSetAttribute(k_potrf128<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, POTRF_SMEM));
+    BDB_CUDA(cudaFuncSetAttribute(k_syrk_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRKD_SMEM<double>));
     BDB_CUDA(cudaFuncSetAttribute(k_trsm128<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM));
     BDB_CUDA(cudaFuncSetAttribute(k_syrk64, cudaFuncAttributeMaxDynamicSharedMemorySize, S64_SMEM));
     int dev = 0, sms = 148;
@@ -1825,17 +1854,15 @@ static cudaError_t launch_syrk64(bdb_system* s, int grid, cudaStream_t st, const
                                  int mode)
 {
     cudaLaunchConfig_t cfg = {};
-    const bool diag = mode == 1 && ntiles == 1;
-    cfg.gridDim = dim3(diag ? S64D_GRID : std::min(2 * grid, 2 * ntiles));
+    cfg.gridDim = dim3(std::min(2 * grid, 2 * ntiles));
     cfg.blockDim = dim3(S64_THREADS);
-    cfg.dynamicSmemBytes = diag ? 0 : S64_SMEM;
+    cfg.dynamicSmemBytes = S64_SMEM;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (diag) return cudaLaunchKernelEx(&cfg, k_syrk64_diag, s->M64.p, s->npad, Lp, t0);
     return cudaLaunchKernelEx(&cfg, k_syrk64, s->M64.p, s->npad, Lp, t0, ntiles, mode, s->status.p);
 }
 
