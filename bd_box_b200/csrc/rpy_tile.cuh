@@ -301,8 +301,13 @@ __device__ __forceinline__ void lattice_sum(const EwaldConst& ec, const double* 
     } else {
         const double z0 = v[2];
         const double up0 = exp(-ec.a2 * (1 + 2 * z0)), down0 = exp(-ec.a2 * (1 - 2 * z0));
-        // a Gaussian that may underflow at g = 0 is taken image by image
-        const bool run = ec.a2 * (R + 2) * (R + 2) < 600.0;
+        // The recurrence holds while up0 and down0 stay finite and the Gaussian
+        // at g = 0 does not underflow: positions in the box have |v_k| <= 1
+        // (m = 1). Beyond (strong screening; positions that a caller has set
+        // many boxes away, 0 * inf from |z0| ~ 113 at alpha = sqrt(pi)) every
+        // image takes its own exponential. a2 (1 + 2 |z0|) <= a2 (R + 1 + m)^2.
+        const double m = R + 1 + fmax(1.0, fmax(fabs(v[0]), fmax(fabs(v[1]), fabs(v[2]))));
+        const bool run = ec.a2 * m * m < 600.0;
         for (int h = -R; h <= R; ++h) {
             const double x = v[0] + h;
             const int nf = ec.extent[h * h];

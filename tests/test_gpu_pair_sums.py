@@ -91,3 +91,28 @@ def test_lattice_sums_fp64_against_oracle(method, deck_dir):
     for i, j in ((0, 1), (7, 30), (39, 2), (5, 5)):
         a, b = s.compute_Dij(i, j), np.asarray(o.tile(max(i, j), min(i, j))).reshape(3, 3)
         assert np.abs(a - b).max() <= 1e-13 * np.abs(o.tile(0, 0)).max()
+
+
+# R, Smith's ewald_alpha (0: Beenakker), box lengths; at each of them the
+# Gaussian recurrence along a row of images overflows if it is used
+@pytest.mark.parametrize("r,alpha,boxes", [(4, 0.0, 120), (3, 0.0, 120), (3, 1.7724538509055159, 120), (3, 4.8, 16),
+                                           (2, 6.0, 11), (5, 3.4, 40), (0, 1.7724538509055159, 300)])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_lattice_sums_fp64_far_outside_the_box(r, alpha, boxes, axis, deck_dir):
+    """Steps wrap positions, callers need not: a bead many box lengths away in
+    either direction has the oracle's tile, which sums image by image."""
+    import pyoracle
+    extra = {"ewald_method": "smith", "ewald_alpha": alpha} if alpha else {}
+    d = decks.read_deck(decks.write_suspension_deck(deck_dir, f"far{r}_{boxes}", 24, seed=5, ewald_r=r, extra=extra))
+    d.coord = d.coord.copy()
+    d.coord[3, axis] += boxes * d.box[0]
+    d.coord[17, axis] -= boxes * d.box[0]
+    o = pyoracle.Oracle(d)
+    s = engine.System(d, precision=engine.PREC_FP64, noise=engine.NOISE_HOST)
+    scale = np.abs(o.tile(0, 0)).max()
+    for i, j in ((3, 0), (17, 0), (17, 3), (5, 1)):
+        a, b = s.compute_Dij(i, j), np.asarray(o.tile(i, j)).reshape(3, 3)
+        # phases 2 pi k v carry v's rounding: 2 pi R |v| ulps of weights ~ 1
+        assert np.abs(a - b).max() <= 2e-16 * 8 * np.pi * (r + 1) * (2 * boxes + 1) * scale
+    assert np.isfinite(s.compute_Rf()).all()
+    assert np.isfinite(s.compute_r(np.random.default_rng(r).standard_normal(72))).all()
