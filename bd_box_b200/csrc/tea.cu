@@ -290,7 +290,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
     const double4 org = pos[i0];
     // positions in FP32 pairs: in L for the converged split
     const double unit = KIND == TILE_FAST ? A.ec.inv_L : 1.0;
-    T eps = 0;
+    double eps = 0;   // FP32: a chunk's sum at a time (at most 16 pairs a lane)
     Bead<T> b;
     // row sums of the job: in FP64 when they span several column tiles
     const bool flush = sizeof(T) == 4 && jb.nJ > 1;
@@ -343,7 +343,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
                     }
                     tea_steps<T, KIND, RS, NR>(A, E, pos, cols, row, i0, ni, j0, end - j0, s, e, jb.type == JOB_DIAG, rc,
                                                cacc, eps_c);
-                    eps += eps_c;
+                    eps += (double)eps_c;
                     __syncwarp();   // lanes take turns at a column's slot
 #pragma unroll
                     for (int k = 0; k < NV; ++k) {
@@ -398,10 +398,9 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
         rows(std::integral_constant<int, 1>{});
     }
     if (RS) {
-        double e = (double)eps;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) eps_part[job] = e;
+        for (int o = 16; o > 0; o >>= 1) eps += __shfl_xor_sync(0xffffffffu, eps, o);
+        if (lane == 0) eps_part[job] = eps;
     }
 }
 
