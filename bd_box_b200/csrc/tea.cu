@@ -266,8 +266,9 @@ __device__ __forceinline__ void tea_steps(const TensorArgs& A, const FastArg<KIN
     }
 }
 
-// One warp per job. Records are written in T; the row sums of a job with
-// several column tiles are added tile by tile in FP64 (shared memory).
+// One warp per job. Records are written in T: in FP32 a record holds one tile's
+// sums as they are; the row sums of a job with several column tiles are added
+// tile by tile in FP64 (shared memory) and take two records.
 template <typename T, int KIND, bool RS>
 __global__ void __launch_bounds__(32 * TEA_WARPS, sizeof(T) == 4 && KIND == TILE_FREE ? 4 : 3)
 k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastArg<KIND> E, const TileJob* __restrict__ jobs, int n_jobs, const int* __restrict__ col_rec,
@@ -366,9 +367,14 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
                 __syncwarp();
             }
             if (jb.type == JOB_DIAG) {
-                // row and column sums of the same beads: one record
+                // row and column sums of the same beads: one record in FP64,
+                // one each in FP32, where joining them would round again
+                if constexpr (sizeof(T) == 8) {
 #pragma unroll
-                for (int k = 0; k < NV; ++k) racc[0][k] += __shfl_sync(0xffffffffu, cacc[k], (lane - jb.s1) & 31);
+                    for (int k = 0; k < NV; ++k) racc[0][k] += __shfl_sync(0xffffffffu, cacc[k], (lane - jb.s1) & 31);
+                } else {
+                    put_record(jb.rec0 + 1, (lane + jb.s1) & 31, cacc);
+                }
             } else {
                 put_record(col_rec[jb.col0 + q], (lane + jb.s1) & 31, cacc);
             }
@@ -385,10 +391,20 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
         }
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            if (flush)
+            const int rec = r ? jb.rec1 : jb.rec0;
+            if (flush) {
+                // an FP64 sum goes out as two FP32 records, its FP32 value and
+                // what that leaves, and loses nothing
+                T lo[NV];
 #pragma unroll
-                for (int k = 0; k < NV; ++k) racc[r][k] = (T)s_row[warp][sizeof(T) == 4 ? r * NV + k : 0][lane];
-            if (NR == 1 || i0 + TT * r < end) put_record(r ? jb.rec1 : jb.rec0, lane, racc[r]);
+                for (int k = 0; k < NV; ++k) {
+                    const double v = s_row[warp][sizeof(T) == 4 ? r * NV + k : 0][lane];
+                    racc[r][k] = (T)v;
+                    lo[k] = (T)(v - (double)racc[r][k]);
+                }
+                put_record(rec + 1, lane, lo);
+            }
+            put_record(rec, lane, racc[r]);
         }
     };
     if constexpr (MAXR == 2) {
@@ -555,7 +571,8 @@ static int tea_setup(bdb_system* s)
     const int max_split = s->p.ewald ? 16 : 8;
     int split = 1, run = 1;
     while (split < max_split && pairs * split < (s->p.ewald ? 2 * fill : fill / 2)) split *= 2;
-    const bool two = !s->p.ewald && s->p.precision != BDB_PREC_FP64 && pairs >= 4 * fill;
+    const bool fp64 = s->p.precision == BDB_PREC_FP64;
+    const bool two = !s->p.ewald && !fp64 && pairs >= 4 * fill;
     while (run < 8 && pairs / (2 * run * (two ? 2 : 1)) >= 4 * fill) run *= 2;
     std::vector<TileJob> jobs;
     std::vector<int> cols;           // column record of (job, column tile): slot, turned into an index below
@@ -584,8 +601,14 @@ static int tea_setup(bdb_system* s)
             j.s1 = s1;
             j.type = type;
             j.col0 = (int)cols.size();
-            j.rec0 = nrow[t.tile0 + I]++;
-            j.rec1 = type == JOB_ROWS2 ? nrow[t.tile0 + I + 1]++ : 0;
+            const int nrec = !fp64 && (type == JOB_DIAG || nJ > 1) ? 2 : 1;   // row records of the job
+            j.rec0 = nrow[t.tile0 + I];
+            nrow[t.tile0 + I] += nrec;
+            j.rec1 = 0;
+            if (type == JOB_ROWS2) {
+                j.rec1 = nrow[t.tile0 + I + 1];
+                nrow[t.tile0 + I + 1] += nrec;
+            }
             if (type != JOB_DIAG)
                 for (int q = 0; q < nJ; ++q) {
                     cols.push_back(ncol[t.tile0 + J0 + q]++);
@@ -628,7 +651,7 @@ static int tea_setup(bdb_system* s)
     if (rec > (size_t)1 << 30) return fail(BDB_ERR_NOMEM, "too many bead tiles for the pair sums");
     s->n_jobs = (int)jobs.size();
     s->tea_tiles = (int)tiles.size();
-    const size_t el = s->p.precision == BDB_PREC_FP64 ? sizeof(double) : sizeof(float);
+    const size_t el = fp64 ? sizeof(double) : sizeof(float);
     if (s->jobs.alloc(jobs.size()) || s->tea_cols.alloc(std::max<size_t>(1, cols.size())) ||
         s->eps_part.alloc(jobs.size()) || s->part.alloc((rec * REC * el + sizeof(double) - 1) / sizeof(double)) ||
         s->tea_meta.alloc(sizeof(TeaTile) * tiles.size() + sizeof(TeaSeg) * ts.size()))
