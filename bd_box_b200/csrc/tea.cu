@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <vector>
 
@@ -72,20 +73,30 @@ struct Bead {
     T x[3], lo[3], w, inv, f[3], g[3];   // position (FP32: relative to the job's origin, hi + lo), radius, 1/D, F, X
 };
 
-// A bead's position relative to the job's origin as the FP32 pair hi + lo
-// (48 bits), so that the difference of two beads rounds like one FP32
-// operation without FP64 subtractions and conversions per pair
+// Positions in FP32 pairs: the length unit and the step of hi's grid (a power
+// of two)
+struct PairUnits {
+    double unit, step, inv_step;
+};
+
+// A bead's position relative to the job's origin as the FP32 pair hi + lo, so
+// that the difference of two beads needs no FP64 subtractions and conversions
+// per pair. hi is a multiple of `step` below 2^23 steps: the difference of two
+// is then exact, and with lo's (below a step, rounded 2^-24 of that) the
+// separation is the FP64 difference rounded to FP32 once. Farther out hi is
+// the FP32 value, and the difference rounds twice.
 template <typename T, bool RS>
 __device__ __forceinline__ void load_bead(Bead<T>& b, const TensorArgs& A, const double4* __restrict__ pos,
                                           const double* __restrict__ F, const double* __restrict__ X, int i, bool ok,
-                                          const double4& org, double unit)
+                                          const double4& org, const PairUnits& u)
 {
     const double4 p = pos[i];
     if constexpr (sizeof(T) == 4) {
-        const double d[3] = {(p.x - org.x) * unit, (p.y - org.y) * unit, (p.z - org.z) * unit};
+        const double d[3] = {(p.x - org.x) * u.unit, (p.y - org.y) * u.unit, (p.z - org.z) * u.unit};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            b.x[k] = (float)d[k];
+            const double q = rint(d[k] * u.inv_step);
+            b.x[k] = fabs(q) < 8388608.0 ? (float)(q * u.step) : (float)d[k];
             b.lo[k] = (float)(d[k] - (double)b.x[k]);
         }
     } else {
@@ -273,7 +284,7 @@ template <typename T, int KIND, bool RS>
 __global__ void __launch_bounds__(32 * TEA_WARPS, sizeof(T) == 4 && KIND == TILE_FREE ? 4 : 3)
 k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastArg<KIND> E, const TileJob* __restrict__ jobs, int n_jobs, const int* __restrict__ col_rec,
             const TeaSeg* __restrict__ segs, const double4* __restrict__ pos, const double* __restrict__ F,
-            const double* __restrict__ X, T* __restrict__ part, double* __restrict__ eps_part)
+            const double* __restrict__ X, T* __restrict__ part, double* __restrict__ eps_part, const PairUnits units)
 {
     constexpr int NV = RS ? 9 : 3;
     constexpr int MAXR = sizeof(T) == 4 && KIND == TILE_FREE ? 2 : 1;   // row tiles a job may hold
@@ -289,8 +300,6 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
     const int end = sg.begin + sg.count;
     const int i0 = sg.begin + TT * jb.I, ni = end - i0;
     const double4 org = pos[i0];
-    // positions in FP32 pairs: in L for the converged split
-    const double unit = KIND == TILE_FAST ? A.ec.inv_L : 1.0;
     double eps = 0;   // FP32: a chunk's sum at a time (at most 16 pairs a lane)
     Bead<T> b;
     // row sums of the job: in FP64 when they span several column tiles
@@ -298,7 +307,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
 
     auto columns = [&](int J) {
         const int j0 = sg.begin + TT * J, j = j0 + lane;
-        load_bead<T, RS>(b, A, pos, F, X, min(j, end - 1), j < end, org, unit);
+        load_bead<T, RS>(b, A, pos, F, X, min(j, end - 1), j < end, org, units);
         __syncwarp();
         put_col<RS>(cols, lane, b);
         __syncwarp();
@@ -315,7 +324,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const int i = i0 + TT * r + lane;
-            load_bead<T, RS>(row[r], A, pos, F, X, min(i, end - 1), i < end, org, unit);
+            load_bead<T, RS>(row[r], A, pos, F, X, min(i, end - 1), i < end, org, units);
 #pragma unroll
             for (int k = 0; k < NV; ++k) racc[r][k] = 0;
         }
@@ -510,9 +519,15 @@ __global__ void k_diag_drift(int n, double preDii, const double4* __restrict__ p
 template <typename T, int KIND, bool RS>
 static void tea_pairs(bdb_system* s, const TensorArgs& A, const FastArg<KIND>& E, const TeaSeg* segs)
 {
+    // steps of a 256th of a radius reach 2^15 radii; in L (the converged split)
+    // steps of 2^-22 reach two boxes
+    PairUnits u;
+    u.unit = KIND == TILE_FAST ? A.ec.inv_L : 1.0;
+    u.step = KIND == TILE_FAST ? std::ldexp(1.0, -22) : std::ldexp(1.0, std::ilogb(s->radius0) - 8);
+    u.inv_step = 1 / u.step;
     k_tea_pairs<T, KIND, RS><<<(s->n_jobs + TEA_WARPS - 1) / TEA_WARPS, 32 * TEA_WARPS, 0, s->stream>>>(
         A, E, s->jobs.p, s->n_jobs, s->tea_cols.p, segs, s->pos.p, s->F.p, s->X.p, reinterpret_cast<T*>(s->part.p),
-        s->eps_part.p);
+        s->eps_part.p, u);
 }
 
 template <bool RS>
