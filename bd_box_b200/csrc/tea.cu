@@ -278,8 +278,7 @@ __device__ __forceinline__ void tea_steps(const TensorArgs& A, const FastArg<KIN
 }
 
 // One warp per job. Records are written in T: in FP32 a record holds one tile's
-// sums as they are; the row sums of a job with several column tiles are added
-// tile by tile in FP64 (shared memory) and take two records.
+// sums; the row sums of a job with several column tiles take two.
 template <typename T, int KIND, bool RS>
 __global__ void __launch_bounds__(32 * TEA_WARPS, sizeof(T) == 4 && KIND == TILE_FREE ? 4 : 3)
 k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastArg<KIND> E, const TileJob* __restrict__ jobs, int n_jobs, const int* __restrict__ col_rec,
@@ -289,7 +288,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
     constexpr int NV = RS ? 9 : 3;
     constexpr int MAXR = sizeof(T) == 4 && KIND == TILE_FREE ? 2 : 1;   // row tiles a job may hold
     __shared__ ColData<T> s_col[TEA_WARPS];
-    __shared__ T s_sum[TEA_WARPS][sizeof(T) == 4 ? (1 + MAXR) * NV : 1][TT];
+    __shared__ double s_sum[TEA_WARPS][sizeof(T) == 4 ? NV : 1][TT];
     __shared__ double s_row[TEA_WARPS][sizeof(T) == 4 ? MAXR * NV : 1][TT];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int job = blockIdx.x * TEA_WARPS + warp;
@@ -302,8 +301,6 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
     const double4 org = pos[i0];
     double eps = 0;   // FP32: a chunk's sum at a time (at most 16 pairs a lane)
     Bead<T> b;
-    // row sums of the job: in FP64 when they span several column tiles
-    const bool flush = sizeof(T) == 4 && jb.nJ > 1;
 
     auto columns = [&](int J) {
         const int j0 = sg.begin + TT * J, j = j0 + lane;
@@ -338,10 +335,9 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
                 tea_steps<T, KIND, RS, NR>(A, E, pos, cols, row, i0, ni, j0, end - j0, jb.s0, jb.s1,
                                            jb.type == JOB_DIAG, racc, cacc, eps);
             } else {
-                // FP32 sums in two levels: 8 steps at a time, then the
-                // chunks' sums, in shared memory at the bead's own slot (the
-                // column's at its number), so that a sum of 32 rounds like
-                // one of 12
+                // FP32 sums of 8 steps at a time, the chunks' sums in FP64, in
+                // shared memory at the bead's own slot (the column's at its
+                // number): rows over the whole job, columns over the tile
                 for (int s = jb.s0; s < jb.s1; s += CHUNK) {
                     const int e = min(s + CHUNK, jb.s1), l = (lane + e) & 31;
                     T rc[NR][NV], eps_c = 0;
@@ -357,22 +353,18 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
                     __syncwarp();   // lanes take turns at a column's slot
 #pragma unroll
                     for (int k = 0; k < NV; ++k) {
-                        T* o = &s_sum[warp][k][l];
-                        *o = s == jb.s0 ? cacc[k] : *o + cacc[k];
+                        double* o = &s_sum[warp][k][l];
+                        *o = s == jb.s0 ? (double)cacc[k] : *o + (double)cacc[k];
 #pragma unroll
                         for (int r = 0; r < NR; ++r) {
-                            T* p = &s_sum[warp][NV * (1 + r) + k][lane];
-                            *p = s == jb.s0 ? rc[r][k] : *p + rc[r][k];
+                            double* p = &s_row[warp][NV * r + k][lane];
+                            *p = q == 0 && s == jb.s0 ? (double)rc[r][k] : *p + (double)rc[r][k];
                         }
                     }
                 }
                 __syncwarp();
 #pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    cacc[k] = s_sum[warp][k][(lane + jb.s1) & 31];
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) racc[r][k] = s_sum[warp][NV * (1 + r) + k][lane];
-                }
+                for (int k = 0; k < NV; ++k) cacc[k] = (T)s_sum[warp][k][(lane + jb.s1) & 31];
                 __syncwarp();
             }
             if (jb.type == JOB_DIAG) {
@@ -387,31 +379,21 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
             } else {
                 put_record(col_rec[jb.col0 + q], (lane + jb.s1) & 31, cacc);
             }
-            if (flush) {
-#pragma unroll
-                for (int r = 0; r < NR; ++r)
-#pragma unroll
-                    for (int k = 0; k < NV; ++k) {
-                        double* o = &s_row[warp][sizeof(T) == 4 ? r * NV + k : 0][lane];
-                        *o = q ? *o + (double)racc[r][k] : (double)racc[r][k];
-                        racc[r][k] = 0;
-                    }
-            }
         }
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const int rec = r ? jb.rec1 : jb.rec0;
-            if (flush) {
-                // an FP64 sum goes out as two FP32 records, its FP32 value and
-                // what that leaves, and loses nothing
+            if constexpr (sizeof(T) == 4) {
+                // the FP64 sum over several tiles goes out as two FP32
+                // records, its FP32 value and what that leaves
                 T lo[NV];
 #pragma unroll
                 for (int k = 0; k < NV; ++k) {
-                    const double v = s_row[warp][sizeof(T) == 4 ? r * NV + k : 0][lane];
+                    const double v = s_row[warp][NV * r + k][lane];
                     racc[r][k] = (T)v;
                     lo[k] = (T)(v - (double)racc[r][k]);
                 }
-                put_record(rec + 1, lane, lo);
+                if (jb.nJ > 1) put_record(rec + 1, lane, lo);
             }
             put_record(rec, lane, racc[r]);
         }
