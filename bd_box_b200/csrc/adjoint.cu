@@ -20,9 +20,10 @@
 //     lambda'^T dB X = <Dbar, dD>,  Dbar = B^-T Phi(v X^T) B^-1,  v = B^T lambda',
 //   formed from the inverse of B by products of full tiles (adjoint_linalg).
 // The forward pass is recomputed from checkpoints every `checkpoint` steps. A
-// segment's steps leave what their reverse needs -- positions, forces, and,
-// where the device has room for them, D and B -- so that each step is factored
+// segment's steps leave what their reverse needs -- positions and, where the
+// device has room for them, forces, D and B -- so that each step is factored
 // once more, not twice; the last segment's are kept by the forward pass itself.
+// Without that room forces, D and B are computed again from the positions.
 // Precision follows the system's: FP64 throughout for an FP64 system; for a
 // mixed-precision system (FP32 tensor, FP16-split Cholesky) the forward steps
 // are the mixed path's, and the backward's O(n^3) part -- the inverse and the
@@ -301,12 +302,35 @@ __global__ void k_mv2_finish(int n, int nrb, int ncb, const double* __restrict__
 // right-hand sides take n^3 in 190 launches of narrow updates (n = 3072, FP32:
 // 4.2 ms a step before, 1.35 now).
 
+// Room: A and G are lower triangular and share one buffer, n rows of n + 128:
+// row block C (128 rows) of G lies in row block nb - 1 - C, right of A's last
+// block there. W, the partial sums of G and then S share another (n x n): each
+// is read for the last time before the next is written. So two matrices beside
+// the system's own, as the two right-hand sides of the solves took.
+template <typename T>
+struct PlainRows {
+    const T* p;
+    size_t ld;
+    __device__ const T* at(int r) const { return p + (size_t)r * ld; }
+};
+template <typename T>
+struct GRows {
+    T* p;
+    size_t ld;
+    int nb;
+    __device__ T* at(int r) const
+    {
+        const int C = r >> 7;
+        return p + (size_t)(128 * (nb - 1 - C) + (r & 127)) * ld + 128 * (nb - C);
+    }
+};
+
 // inverses of the 64x64 diagonal blocks of the lower-triangular B (ld) into A
-// (n x n, zero above the diagonal), column c by forward substitution: four
+// (lda, zero above the diagonal), column c by forward substitution: four
 // lanes share a column's dot products (one lane each: 83 us at n = 3072),
 // accumulated in FP64 over the column's entries as stored (T)
 template <typename TM, typename T>
-__global__ void __launch_bounds__(256) k_trinv64(const TM* __restrict__ B, int ld, int n, T* __restrict__ A)
+__global__ void __launch_bounds__(256) k_trinv64(const TM* __restrict__ B, int ld, T* __restrict__ A, size_t lda)
 {
     extern __shared__ __align__(16) unsigned char trinv_smem[];
     T(*Bs)[65] = reinterpret_cast<T(*)[65]>(trinv_smem);
@@ -330,7 +354,7 @@ __global__ void __launch_bounds__(256) k_trinv64(const TM* __restrict__ B, int l
         __syncwarp();
     }
     __syncthreads();
-    for (int e = tid; e < 64 * 64; e += 256) A[(o + (e >> 6)) * n + o + (e & 63)] = W[e >> 6][e & 63];
+    for (int e = tid; e < 64 * 64; e += 256) A[(o + (e >> 6)) * lda + o + (e & 63)] = W[e >> 6][e & 63];
 }
 
 // ---- tile products: TILE x TILE (128 or 64) on TILE^2 / 64 threads with 8 x 8
@@ -367,19 +391,21 @@ __device__ __forceinline__ void load8(const double* p, double* v)
     }
 }
 
-// acc += op(A) B over k0 <= k < k1 (multiples of 16). op(A)(m, k) is
-// A[m lda + k] or, with TA, A[k lda + m]; B(k, c) is B[k ldb + c]. Rows m >= ml
-// and columns c >= nl (multiples of 8) are zero.
-template <typename T, bool TA, int TILE>
-__device__ __forceinline__ void gemm_tile(GemmSmem<T, TILE>& sm, const T* __restrict__ A, size_t lda,
-                                          const T* __restrict__ B, size_t ldb, int k0, int k1, int ml, int nl,
-                                          T (&acc)[8][8])
+// acc += op(A) B over k0 <= k < k1 (multiples of 16). op(A)(m, k) is row m of
+// A at k or, with TA, row k of A at ma + m; B(k, c) is row k of B at nb + c. Rows
+// m >= ml and columns c >= nl (multiples of 8) are zero.
+template <typename T, bool TA, int TILE, class RA, class RB>
+__device__ __forceinline__ void gemm_tile(GemmSmem<T, TILE>& sm, const RA A, int ma, const RB B, int nb, int k0, int k1,
+                                          int ml, int nl, T (&acc)[8][8])
 {
     constexpr int NT = gemm_threads(TILE), NP = 2 * TILE / NT;   // pieces of 8 per thread and operand
     constexpr int HX = TILE / 8;                                 // threads along a tile's side
     const int tid = threadIdx.x, tx = tid % HX, ty = tid / HX;
     T ra[NP][8], rb[NP][8];
     auto load = [&](int k) {
+        // 16 rows from a multiple of 16: in one row block of 128
+        const T* a0 = TA ? A.at(k) + ma : nullptr;
+        const T* b0 = B.at(k) + nb;
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             const int e = tid + NT * p, kr = e / HX, c8 = 8 * (e % HX);   // a row of TILE in pieces of 8
@@ -387,11 +413,11 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T, TILE>& sm, const T* __rest
 #pragma unroll
             for (int u = 0; u < 8; ++u) ra[p][u] = rb[p][u] = (T)0;
             if (TA) {
-                if (c8 < ml) load8(A + (size_t)(k + kr) * lda + c8, ra[p]);
+                if (c8 < ml) load8(a0 + (size_t)kr * A.ld + c8, ra[p]);
             } else {
-                if (mr < ml) load8(A + (size_t)mr * lda + k + k8, ra[p]);
+                if (mr < ml) load8(A.at(mr) + k + k8, ra[p]);
             }
-            if (c8 < nl) load8(B + (size_t)(k + kr) * ldb + c8, rb[p]);
+            if (c8 < nl) load8(b0 + (size_t)kr * B.ld + c8, rb[p]);
         }
     };
     auto store = [&](int st) {
@@ -482,7 +508,7 @@ __device__ __forceinline__ int gemm_at(int t, int u)
 // to 2048 at the last one, 0.92 ms in all levels; 0.69 with 64).
 template <typename T, int STAGE>
 __global__ void __launch_bounds__(gemm_threads(64), sizeof(T) == 4 ? 6 : 4)
-k_tri_level(int n, int s, const T* __restrict__ B, int ldb, T* __restrict__ A, T* __restrict__ W)
+k_tri_level(int n, int s, const T* __restrict__ B, int ldb, T* __restrict__ A, size_t lda, T* __restrict__ W)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
     constexpr int TL = 64;
@@ -494,46 +520,50 @@ k_tri_level(int n, int s, const T* __restrict__ B, int ldb, T* __restrict__ A, T
     T acc[8][8];
     gemm_begin(sm, acc);
     if (STAGE == 0)   // A11 is zero above its diagonal: k >= n0
-        gemm_tile<T, false, TL>(sm, B + (size_t)(r0 + m0) * ldb + c0, ldb, A + (size_t)c0 * n + c0 + n0, n, n0, s, ml, nl,
-                            acc);
+        gemm_tile<T, false, TL>(sm, PlainRows<T>{B + (size_t)(r0 + m0) * ldb + c0, (size_t)ldb}, 0,
+                                PlainRows<T>{A + (size_t)c0 * lda + c0, lda}, n0, n0, s, ml, nl, acc);
     else              // A22 likewise: k < m0 + 64
-        gemm_tile<T, false, TL>(sm, A + (size_t)(r0 + m0) * n + r0, n, W + (size_t)r0 * n + c0 + n0, n, 0,
-                            min(m0 + TL, min(s, n - r0)), ml, nl, acc);
+        gemm_tile<T, false, TL>(sm, PlainRows<T>{A + (size_t)(r0 + m0) * lda + r0, lda}, 0,
+                                PlainRows<T>{W + (size_t)r0 * n + c0, (size_t)n}, n0, 0,
+                                min(m0 + TL, min(s, n - r0)), ml, nl, acc);
     gemm_end(sm, acc);
-    T* O = (STAGE == 0 ? W : A) + (size_t)(r0 + m0) * n + c0 + n0;
+    const size_t ldo = STAGE == 0 ? (size_t)n : lda;
+    T* O = (STAGE == 0 ? W : A) + (size_t)(r0 + m0) * ldo + c0 + n0;
     const int tx = threadIdx.x % (TL / 8), ty = threadIdx.x / (TL / 8);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int r = gemm_at<TL>(ty, i), c = gemm_at<TL>(tx, j);
-            if (r < ml && c < nl) O[(size_t)r * n + c] = STAGE == 0 ? acc[i][j] : -acc[i][j];
+            if (r < ml && c < nl) O[(size_t)r * ldo + c] = STAGE == 0 ? acc[i][j] : -acc[i][j];
         }
 }
 
 // G = Phi(v X^T) A in two passes over blocks of 64 rows: the blocks' sums of
 // X_c A_c, then each block's running sum from those before it (FP64)
 template <typename T>
-__global__ void k_phi_sums(int n, const double* __restrict__ X, const T* __restrict__ A, double* __restrict__ sums)
+__global__ void k_phi_sums(int n, const double* __restrict__ X, const T* __restrict__ A, size_t lda,
+                           double* __restrict__ sums)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x, r0 = 64 * blockIdx.y;
     if (b >= n) return;
     double a = 0;
     if (b < r0 + 64)
-        for (int c = r0; c < r0 + 64; ++c) a += X[c] * (double)A[(size_t)c * n + b];
+        for (int c = r0; c < r0 + 64; ++c) a += X[c] * (double)A[(size_t)c * lda + b];
     sums[(size_t)blockIdx.y * n + b] = a;
 }
 template <typename T>
-__global__ void k_phi_rows(int n, const double* __restrict__ v, const double* __restrict__ X, const T* __restrict__ A,
-                           const double* __restrict__ sums, T* __restrict__ G)
+__global__ void k_phi_rows(int n, const double* __restrict__ v, const double* __restrict__ X, const T* A, size_t lda,
+                           const double* __restrict__ sums, const GRows<T> G)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x, r0 = 64 * blockIdx.y;
-    if (b >= n) return;
+    if (b >= (r0 / 128 + 1) * 128) return;   // G's row block ends at its diagonal block
     double run = 0;
     for (int q = b / 64; q < (int)blockIdx.y; ++q) run += sums[(size_t)q * n + b];
+    T* g = G.at(r0) + b;
     for (int c = r0; c < r0 + 64; ++c) {
-        const double t = b <= c ? X[c] * (double)A[(size_t)c * n + b] : 0.0;
-        G[(size_t)c * n + b] = (T)(v[c] * (run + 0.5 * t));
+        const double t = b <= c ? X[c] * (double)A[(size_t)c * lda + b] : 0.0;
+        g[(size_t)(c - r0) * lda] = (T)(v[c] * (run + 0.5 * t));
         run += t;
     }
 }
@@ -541,8 +571,11 @@ __global__ void k_phi_rows(int n, const double* __restrict__ v, const double* __
 // S pieces: tile (i, j), i >= j, of 128 x 128 over 128 i + sk q <= k <
 // 128 i + sk (q + 1): A^T G + G^T A. The sum over k is longest where tiles are
 // fewest (k >= 128 i), so it is cut into at most 8 pieces (adj_piece): 1,000
-// pieces of 384 at n = 3072 for 296 CTA slots. k_adj_join adds a tile's pieces in order and writes the
-// tile and its mirror image.
+// pieces of 384 at n = 3072 for 296 CTA slots. k_adj_join adds a tile's pieces
+// in order and writes the tile and its mirror image. Rows of tiles are taken
+// in rounds of at most ADJ_ROUND pieces (one row where that has more): seven
+// waves of CTAs, all of n = 3072 in one, and 128 KB (FP64) a piece of room.
+static constexpr int ADJ_ROUND = 2048;
 __host__ __device__ inline int adj_piece(int nb) { return GT * (nb > 24 ? (nb + 7) / 8 : 3); }
 __host__ __device__ inline int adj_pieces_of(int nb, int i)
 {
@@ -556,21 +589,41 @@ __host__ __device__ inline int adj_pieces_before(int nb, int i)
     return p;
 }
 
+// end of the round that starts with row i0
+static int adj_round_end(int nb, int i0)
+{
+    int i1 = i0, p = 0;
+    do p += (i1 + 1) * adj_pieces_of(nb, i1);
+    while (++i1 < nb && p + (i1 + 1) * adj_pieces_of(nb, i1) <= ADJ_ROUND);
+    return i1;
+}
+// pieces of the largest round
+static int adj_round_pieces(int nb)
+{
+    int most = 0;
+    for (int i0 = 0, i1; i0 < nb; i0 = i1) {
+        i1 = adj_round_end(nb, i0);
+        most = std::max(most, adj_pieces_before(nb, i1) - adj_pieces_before(nb, i0));
+    }
+    return most;
+}
+
+// the pieces from number p0 on
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
-k_adj_pieces(int n, const T* __restrict__ A, const T* __restrict__ G, T* __restrict__ part)
+k_adj_pieces(int n, int p0, const PlainRows<T> A, const GRows<T> G, T* __restrict__ part)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
     GemmSmem<T, GT>& sm = *reinterpret_cast<GemmSmem<T, GT>*>(gemm_smem);
     const int nb = n / GT;
-    int i = 0, p = blockIdx.x;
+    int i = 0, p = p0 + blockIdx.x;
     while (p >= (i + 1) * adj_pieces_of(nb, i)) p -= (i + 1) * adj_pieces_of(nb, i++);
     const int np = adj_pieces_of(nb, i), j = p / np, q = p % np;
     const int sk = adj_piece(nb), k0 = GT * i + sk * q, k1 = min(n, k0 + sk);
     T acc[8][8];
     gemm_begin(sm, acc);
-    gemm_tile<T, true, GT>(sm, A + GT * i, n, G + GT * j, n, k0, k1, GT, GT, acc);
-    gemm_tile<T, true, GT>(sm, G + GT * i, n, A + GT * j, n, k0, k1, GT, GT, acc);
+    gemm_tile<T, true, GT>(sm, A, GT * i, G, GT * j, k0, k1, GT, GT, acc);
+    gemm_tile<T, true, GT>(sm, G, GT * i, A, GT * j, k0, k1, GT, GT, acc);
     gemm_end(sm, acc);
     T* O = part + (size_t)blockIdx.x * GT * GT;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -580,15 +633,15 @@ k_adj_pieces(int n, const T* __restrict__ A, const T* __restrict__ G, T* __restr
         for (int c = 0; c < 8; ++c) O[gemm_at<GT>(ty, r) * GT + gemm_at<GT>(tx, c)] = acc[r][c];
 }
 
-// 32 x 32 of tile (i, j) per CTA (blockIdx.z = 0..15)
+// 32 x 32 of tile (i, j) per CTA (blockIdx.z = 0..15), rows i0 .. of tiles
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_join(int n, const T* __restrict__ part, T* __restrict__ S)
+__global__ void __launch_bounds__(256) k_adj_join(int n, int i0, int p0, const T* __restrict__ part, T* __restrict__ S)
 {
-    const int i = blockIdx.y, j = blockIdx.x;
+    const int i = i0 + blockIdx.y, j = blockIdx.x;
     if (j > i) return;
     __shared__ T t[32][33];
     const int nb = n / GT, np = adj_pieces_of(nb, i);
-    const T* src = part + (size_t)(adj_pieces_before(nb, i) + j * np) * GT * GT;
+    const T* src = part + (size_t)(adj_pieces_before(nb, i) - p0 + j * np) * GT * GT;
     const int r0 = 32 * (blockIdx.z >> 2), c0 = 32 * (blockIdx.z & 3);
     const int x = threadIdx.x & 31;
     for (int y = threadIdx.x >> 5; y < 32; y += 8) {
@@ -631,12 +684,16 @@ struct Part {
 };
 
 // Work buffers of adjoint_linalg, T elements: the inverse (zero above the
-// diagonal), G, S and scratch (each np x np) and the pieces of S
+// diagonal) with G, S (also W, and the sums of G, [np / 64][np] in FP64) and
+// the pieces of S
 template <typename T>
 struct AdjLinalg {
-    T *A = nullptr, *G = nullptr, *S = nullptr, *W = nullptr, *part = nullptr;
-    double* sums = nullptr;   // [np / 64][np]
+    T *A = nullptr, *S = nullptr, *part = nullptr;
 };
+static size_t adj_dense(int np)   // elements of the three
+{
+    return (size_t)np * (np + GT) + (size_t)np * np + (size_t)adj_round_pieces(np / GT) * GT * GT;
+}
 
 // u = D lam and v = B^T lam from the stored matrix M (D upper, B lower), then
 // S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1
@@ -652,20 +709,28 @@ static int adjoint_linalg(bdb_system* s, const T* M, int np, int n3, int nrb, in
     BDB_CUDA(cudaFuncSetAttribute(k_adj_pieces<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     k_mv2<T><<<dim3(ncb, nrb), 256, 0, st>>>(M, n3, np, lam, colp, rowp);
     k_mv2_finish<<<(n3 + 255) / 256, 256, 0, st>>>(n3, nrb, ncb, colp, rowp, s->dD.p, lam, u, v);
-    k_trinv64<T, T><<<np / 64, 256, tri_smem, st>>>(M, np, np, w.A);
-    s->launches += 7;
+    const size_t lda = (size_t)np + GT;
+    double* sums = reinterpret_cast<double*>(w.S);
+    k_trinv64<T, T><<<np / 64, 256, tri_smem, st>>>(M, np, w.A, lda);
+    s->launches += 5;
     for (int h = 64; h < np; h *= 2) {
         const dim3 grid(h / 64, std::min(h, np - h) / 64, (np + h - 1) / (2 * h));
-        k_tri_level<T, 0><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, w.W);
-        k_tri_level<T, 1><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, w.W);
+        k_tri_level<T, 0><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, lda, w.S);
+        k_tri_level<T, 1><<<grid, gemm_threads(64), lev_smem, st>>>(np, h, M, np, w.A, lda, w.S);
         s->launches += 2;
     }
     const dim3 cols((np + 127) / 128, np / 64);
-    k_phi_sums<T><<<cols, 128, 0, st>>>(np, Xp, w.A, w.sums);
-    k_phi_rows<T><<<cols, 128, 0, st>>>(np, v, Xp, w.A, w.sums, w.G);
     const int nb = np / GT;
-    k_adj_pieces<T><<<adj_pieces_before(nb, nb), 256, smem, st>>>(np, w.A, w.G, w.part);
-    k_adj_join<T><<<dim3(nb, nb, 16), 256, 0, st>>>(np, w.part, w.S);
+    const GRows<T> G{w.A, lda, nb};
+    k_phi_sums<T><<<cols, 128, 0, st>>>(np, Xp, w.A, lda, sums);
+    k_phi_rows<T><<<cols, 128, 0, st>>>(np, v, Xp, w.A, lda, sums, G);
+    for (int i0 = 0, i1; i0 < nb; i0 = i1) {
+        i1 = adj_round_end(nb, i0);
+        const int p0 = adj_pieces_before(nb, i0), p1 = adj_pieces_before(nb, i1);
+        k_adj_pieces<T><<<p1 - p0, 256, smem, st>>>(np, p0, PlainRows<T>{w.A, lda}, G, w.part);
+        k_adj_join<T><<<dim3(i1, i1 - i0, 16), 256, 0, st>>>(np, i0, p0, w.part, w.S);
+        s->launches += 2;
+    }
     BDB_CUDA(cudaGetLastError());
     return BDB_OK;
 }
@@ -731,36 +796,43 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     const int nck = (K + checkpoint - 1) / checkpoint, seg_len = std::min(K, checkpoint);
     const int nrb = (n3 + MV2_ROWS - 1) / MV2_ROWS, ncb = (n3 + MV2_COLS - 1) / MV2_COLS;
     const size_t nn = (size_t)np * np, el = mixed ? sizeof(float) : sizeof(double);
-    const size_t pieces = (size_t)adj_pieces_before(np / GT, np / GT) * GT * GT;
     // the vectors and lists share one allocation: 15 driver calls and as many
     // frees spread a call's time (40 calls at n = 3072: median 28.0 ms, mean 31
     // to 57, the slowest 941; with one 28.0, 29 to 30 and 69)
-    Part<double> sums, lam, lam2, u, v, Xp, colp, rowp, ppart, Fseg;
+    Part<double> lam, lam2, u, v, Xp, colp, rowp, ppart;
     Part<double4> ckpt, seg, xK;
     Part<int> d_bptr, d_blist;
-    Scratch<unsigned char> vecs, dense, Mseg;
+    Scratch<unsigned char> vecs, kept;
     size_t bytes = 0;
-    sums.place(bytes, (size_t)np / 64 * np), lam.place(bytes, np), lam2.place(bytes, np), u.place(bytes, np);
+    Part<unsigned char> dense;
+    dense.place(bytes, adj_dense(np) * el), lam.place(bytes, np), lam2.place(bytes, np), u.place(bytes, np);
     v.place(bytes, np), Xp.place(bytes, np), colp.place(bytes, (size_t)nrb * n3 * 2);
     rowp.place(bytes, (size_t)ncb * n3), ppart.place(bytes, 4 * (size_t)n), ckpt.place(bytes, (size_t)nck * n);
-    seg.place(bytes, (size_t)seg_len * n), Fseg.place(bytes, (size_t)seg_len * n3), xK.place(bytes, n);
+    seg.place(bytes, (size_t)seg_len * n), xK.place(bytes, n);
     d_bptr.place(bytes, n + 1), d_blist.place(bytes, blist.size());
-    if (dense.alloc((4 * nn + pieces) * el) || vecs.alloc(bytes))
-        return fail(BDB_ERR_NOMEM, "adjoint scratch allocation failed");
-    for (Part<double>* q : {&sums, &lam, &lam2, &u, &v, &Xp, &colp, &rowp, &ppart, &Fseg}) q->set(vecs.p);
+    if (vecs.alloc(bytes)) return fail(BDB_ERR_NOMEM, "adjoint scratch allocation failed");
+    dense.set(vecs.p);
+    for (Part<double>* q : {&lam, &lam2, &u, &v, &Xp, &colp, &rowp, &ppart}) q->set(vecs.p);
     for (Part<double4>* q : {&ckpt, &seg, &xK}) q->set(vecs.p);
     for (Part<int>* q : {&d_bptr, &d_blist}) q->set(vecs.p);
-    // a segment's stored matrices, in at most half of the memory that is free
+    // a segment's matrices and forces, where they fit in the bytes that the
+    // caller allows (bdb_set_adjoint_keep), by default half of what is free
     bool keep = false;
+    const size_t fbytes = (sizeof(double) * (size_t)seg_len * n3 + 255) / 256 * 256;
+    const size_t kbytes = fbytes + (size_t)seg_len * nn * el;
     {
-        size_t free_b = 0, total_b = 0;
-        const size_t need = (size_t)seg_len * nn * el;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= free_b / 2) keep = !Mseg.alloc(need);
-        if (!keep) cudaGetLastError();   // too little room is no error: the steps are factored again
+        size_t room = 0, total_b = 0;
+        if (s->adjoint_keep >= 0) room = (size_t)s->adjoint_keep;
+        else if (cudaMemGetInfo(&room, &total_b) == cudaSuccess) room /= 2;
+        else room = 0;
+        if (kbytes <= room) keep = !kept.alloc(kbytes);
+        if (!keep) cudaGetLastError();   // too little room is no error: the steps are computed again
     }
+    double* Fseg = reinterpret_cast<double*>(kept.p);
+    unsigned char* Mseg = kept.p + fbytes;
     BDB_CUDA(h2d(s, d_bptr.p, bptr.data(), sizeof(int) * (n + 1)));
     BDB_CUDA(h2d(s, d_blist.p, blist.data(), sizeof(int) * blist.size()));
-    BDB_CUDA(cudaMemsetAsync(dense.p, 0, nn * el, st));   // the inverse: zero above its diagonal
+    BDB_CUDA(cudaMemsetAsync(dense.p, 0, (nn + (size_t)np * GT) * el, st));   // the inverse: zero above its diagonal
     BDB_CUDA(cudaMemsetAsync(ppart.p, 0, sizeof(double) * 4 * n, st));
     BDB_CUDA(cudaMemsetAsync(u.p, 0, sizeof(double) * np, st));
     BDB_CUDA(cudaMemsetAsync(v.p, 0, sizeof(double) * np, st));
@@ -777,15 +849,17 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     auto forward = [&](int slot) -> int {
         int r = 0;
         if (slot >= 0) {
-            if (!s->have_forces && (r = forces_run(s, false, false))) return r;
             BDB_CUDA(cudaMemcpyAsync(seg.p + (size_t)slot * n, s->pos.p, sizeof(double4) * n, cudaMemcpyDeviceToDevice,
                                      st));
-            BDB_CUDA(cudaMemcpyAsync(Fseg.p + (size_t)slot * n3, s->F.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice,
-                                     st));
+            if (keep) {
+                if (!s->have_forces && (r = forces_run(s, false, false))) return r;
+                BDB_CUDA(cudaMemcpyAsync(Fseg + (size_t)slot * n3, s->F.p, sizeof(double) * n3,
+                                         cudaMemcpyDeviceToDevice, st));
+            }
         }
         if ((r = engine_step(s))) return r;
         if (slot >= 0 && keep)   // refresh 1: the matrix still holds this step's D and B
-            BDB_CUDA(cudaMemcpyAsync(Mseg.p + (size_t)slot * nn * el,
+            BDB_CUDA(cudaMemcpyAsync(Mseg + (size_t)slot * nn * el,
                                      mixed ? (const void*)s->M32.p : (const void*)s->M64.p, nn * el,
                                      cudaMemcpyDeviceToDevice, st));
         return BDB_OK;
@@ -848,8 +922,10 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
             // the forward quantities of step k: F(x_k), D(x_k), B(x_k), X_k
             const int slot = k - k0;
             const double4* x = seg.p + (size_t)slot * n;
-            const double* Fk = Fseg.p + (size_t)slot * n3;
-            if (!keep && ((rc = set_positions(s, x)) || (rc = tensor_build(s)) || (rc = factor_run(s)))) return rc;
+            const double* Fk = keep ? Fseg + (size_t)slot * n3 : s->F.p;
+            if (!keep && ((rc = set_positions(s, x)) || (rc = forces_run(s, false, false)) || (rc = tensor_build(s)) ||
+                          (rc = factor_run(s))))
+                return rc;
             if ((rc = set_counter(s, base + k)) || (rc = noise_fill(s, nullptr))) return rc;
             BDB_CUDA(cudaMemcpyAsync(Xp.p, s->X.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
             // u = D lam, v = B^T lam; S = Z + Z^T with Z^T = Dbar = B^-T Phi(v X^T) B^-1;
@@ -858,12 +934,9 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
                 using T = decltype(type);
                 AdjLinalg<T> w;
                 w.A = reinterpret_cast<T*>(dense.p);
-                w.G = w.A + nn;
-                w.S = w.G + nn;
-                w.W = w.S + nn;
-                w.part = w.W + nn;
-                w.sums = sums.p;
-                const int r = adjoint_linalg<T>(s, keep ? reinterpret_cast<const T*>(Mseg.p) + (size_t)slot * nn : M, np,
+                w.S = w.A + nn + (size_t)np * GT;
+                w.part = w.S + nn;
+                const int r = adjoint_linalg<T>(s, keep ? reinterpret_cast<const T*>(Mseg) + (size_t)slot * nn : M, np,
                                                 n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p, Xp.p, w);
                 if (r) return r;
                 BDB_CUDA(cudaMemcpyAsync(lam2.p, lam.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
@@ -893,5 +966,12 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     if (stw & ST_BOND) return fail(BDB_ERR_BOND, "Overstretched bond (bond.c:73-78)");
     for (int q = 0; q < 4; ++q) grad_params[q] = gp[q];
     *loss = L;
+    return BDB_OK;
+}
+
+extern "C" int bdb_set_adjoint_keep(bdb_system* s, long long bytes)
+{
+    if (!s) return fail(BDB_ERR_ARG, "null system");
+    s->adjoint_keep = bytes < 0 ? -1 : bytes;
     return BDB_OK;
 }

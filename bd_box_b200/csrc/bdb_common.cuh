@@ -168,6 +168,7 @@ struct bdb_system {
     const void* mv_map_src[3] = {};            // buffers the maps were encoded for
     int mv_ctas_per_sm = 0;                    // resident CTAs of the TMA matvec kernel per SM
     int sm_count = 148;
+    long long adjoint_keep = -1;               // bytes of a segment's matrices an adjoint may keep (< 0: half of what is free)
     unsigned wait_limit = 1u << 22;            // tries of every bounded device wait (bdb_set_wait_limit)
     int steps_since_refresh = 0;
 

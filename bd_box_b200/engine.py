@@ -47,6 +47,7 @@ EXPORTS = [
     "bdb_set_time", "bdb_get_time", "bdb_newton_resolve",
     "bdb_checkpoint_size", "bdb_checkpoint_save", "bdb_checkpoint_load", "bdb_refresh",
     "bdb_get_factor_tuning", "bdb_set_factor_tuning", "bdb_set_wait_limit", "bdb_cell_grid",
+    "bdb_set_adjoint_keep",
 ]
 
 
@@ -117,6 +118,7 @@ def load_library(path: str = LIB_PATH):
     lib.bdb_set_tuning.argtypes = [C.c_void_p, C.c_int, C.c_int]
     lib.bdb_get_factor_tuning.argtypes = [C.c_void_p, C.POINTER(C.c_int)]
     lib.bdb_set_wait_limit.argtypes = [C.c_void_p, C.c_longlong]
+    lib.bdb_set_adjoint_keep.argtypes = [C.c_void_p, C.c_longlong]
     lib.bdb_set_factor_tuning.argtypes = [C.c_void_p, C.c_int]
     lib.bdb_adjoint.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, _ip, _dp, _dp, _dp, _dp]
     lib.bdb_factor_error.argtypes = [C.c_void_p, _dp]
@@ -356,6 +358,12 @@ class System:
         self._check(self.lib.bdb_adjoint(self.h, K, checkpoint, len(pairs), pairs.ctypes.data_as(_ip), _p(targets),
                                          C.byref(loss), _p(gx), _p(gp)))
         return loss.value, gx.reshape(self.n, 3), gp
+
+    def set_adjoint_keep(self, bytes: int):
+        """Bytes that adjoint may take to keep a segment's matrices
+        (bdb_set_adjoint_keep; 0: none, < 0: the default, half of what is
+        free)."""
+        self._check(self.lib.bdb_set_adjoint_keep(self.h, int(bytes)))
 
     def autotune(self, enable: bool = True):
         self._check(self.lib.bdb_autotune(self.h, int(enable)))

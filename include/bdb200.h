@@ -298,6 +298,12 @@ int bdb_step_igt(bdb_system* s, int K, const double* gauss);
 int bdb_step_igt_predictor(bdb_system* s, const double* gauss);
 int bdb_step_igt_corrector(bdb_system* s, const double* gauss);
 
+/* Bytes that bdb_adjoint may take to keep a segment's matrices and forces (no
+ * reference counterpart): 0 keeps none, < 0 (the default) allows half of the
+ * device memory that is free at the call. The gradient agrees either way to
+ * rounding of the force sums. */
+int bdb_set_adjoint_keep(bdb_system* s, long long bytes);
+
 /* Autotuner (no reference counterpart). With autotuning on, the first use
  * of each tunable site times its candidates on the system's stream and
  * keeps the fastest: the TEA job length (16: jobs half as long as 32's; the
@@ -361,8 +367,15 @@ int bdb_set_dt(bdb_system* s, double dt);
  * epsilon, every bead's LJ sigma, every bond's H and the Debye length 1/kappa
  * (so dloss/d epsilon = grad_params[0] / epsilon for a uniform epsilon).
  * Leaves the system at the final positions. Needs one free-space system,
- * hydro cholesky, BDB_PREC_FP64, refresh 1, BDB_NOISE_PHILOX, and bonds as
- * the only bonded terms (else BDB_ERR_UNSUPPORTED). */
+ * hydro cholesky, refresh 1, BDB_NOISE_PHILOX, and bonds as the only bonded
+ * terms (else BDB_ERR_UNSUPPORTED). On the mixed path the O(N^3) part runs in
+ * FP32.
+ * Allocates, and frees when it returns, two matrices of the system's size and
+ * precision (2 (3N)^2 elements; BDB_ERR_NOMEM without that room), up to 0.3 GB
+ * of partial sums, the positions of every checkpoint and of one segment; and
+ * where they fit (bdb_set_adjoint_keep) the matrices and forces of a segment's
+ * steps, min(K, checkpoint) of each, which saves the reverse pass computing
+ * each once more. */
 int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, const int* pairs,
                 const double* targets, double* loss, double* grad_coord, double* grad_params);
 

@@ -71,3 +71,57 @@ def test_checkpoints_give_the_same_gradient(prec, deck_dir):
         tol = 1e-10 if prec == engine.PREC_FP64 else 1e-6
         assert np.linalg.norm(gx - got[0][1]) <= tol * np.linalg.norm(gx)
         assert np.linalg.norm(gp - got[0][2]) <= tol * np.linalg.norm(gp)
+
+
+@pytest.mark.parametrize("prec", [engine.PREC_FP64, engine.PREC_MIXED])
+@pytest.mark.parametrize("K,ck", [(6, 2), (5, 3), (3, 8)])
+def test_kept_and_recomputed_matrices_agree(prec, K, ck, deck_dir):
+    """With no room to keep a segment's matrices and forces the reverse pass
+    computes them again from the positions."""
+    d, pairs, targets, _ = make(60, deck_dir)
+    got = []
+    for keep in (-1, 0):
+        s = engine.System(d, precision=prec, refresh=1, seed=9)
+        s.set_adjoint_keep(keep)
+        got.append(s.adjoint(K, ck, pairs, targets) + (s.get_coord(),))
+        s.close()
+    (l0, gx0, gp0, x0), (l1, gx1, gp1, x1) = got
+    # forces from cells sorted anew: sums in another order
+    assert abs(l1 - l0) <= 1e-12 * abs(l0)
+    tol = 1e-10 if prec == engine.PREC_FP64 else 1e-6
+    assert np.linalg.norm(gx1 - gx0) <= tol * np.linalg.norm(gx0)
+    assert np.linalg.norm(gp1 - gp0) <= tol * np.linalg.norm(gp0)
+    assert np.abs(x1 - x0).max() <= 1e-9
+
+
+def test_scratch_is_two_matrices(deck_dir):
+    """At 48 tiles the pieces of S go in two rounds; FP64 and mixed agree, and
+    the call takes the room the header states: 2 (3N)^2 elements and 0.3 GB."""
+    import threading
+    import torch
+    n = 2048
+    d, pairs, targets, _ = make(n, deck_dir)
+    out = {}
+    for prec in (engine.PREC_FP64, engine.PREC_MIXED):
+        s = engine.System(d, precision=prec, refresh=1, seed=7)
+        s.set_adjoint_keep(0)
+        s.adjoint(1, 1, pairs, targets)   # the system's own buffers are made
+        s.set_coord(d.coord)
+        torch.cuda.synchronize()
+        before, least, done = torch.cuda.mem_get_info()[0], [], threading.Event()
+
+        def watch():
+            while not done.is_set():
+                least.append(torch.cuda.mem_get_info()[0])
+
+        t = threading.Thread(target=watch)
+        t.start()
+        out[prec] = s.adjoint(3, 3, pairs, targets)
+        done.set()
+        t.join()
+        s.close()
+        el = 8 if prec == engine.PREC_FP64 else 4
+        assert before - min(least) <= 2.2 * (3 * n) ** 2 * el + 3e8
+    (l64, gx, _), (l32, mx, _) = out[engine.PREC_FP64], out[engine.PREC_MIXED]
+    assert abs(l32 - l64) <= 1e-7 * abs(l64)
+    assert np.linalg.norm(mx - gx) <= 1e-5 * np.linalg.norm(gx)
