@@ -91,16 +91,28 @@ __device__ __forceinline__ void mv_tile(const T* __restrict__ M, size_t ld, int 
 #pragma unroll
         for (int u = 0; u < G; ++u) {
             const int r = r0 + g + u;
-            if (!MASK || (r < n3 && c < n3)) {
+            if (!MASK || (r < n3 - (c + 3 >= n3) && c < n3)) {
                 load4(M + (size_t)r * ld + c, m[u]);
             } else {
                 m[u][0] = m[u][1] = m[u][2] = m[u][3] = (T)0;
             }
-            if (MASK)
+        }
+        // the last row's last columns by themselves: beyond them a caller's
+        // matrix may end (the other rows are followed by the next)
+        if (MASK && c + 3 >= n3 && r0 + g < n3 && r0 + g + G >= n3)
+#pragma unroll
+            for (int u = 0; u < G; ++u)
 #pragma unroll
                 for (int v = 0; v < 4; ++v)
+                    if (r0 + g + u == n3 - 1 && c + v < n3) m[u][v] = M[(size_t)(n3 - 1) * ld + c + v];
+        if (MASK)
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const int r = r0 + g + u;
                     if (c + v >= n3 || (PART == 0 ? c + v > r : c + v <= r)) m[u][v] = (T)0;
-        }
+                }
 #pragma unroll
         for (int u = 0; u < G; ++u) {
             const double m0 = m[u][0], m1 = m[u][1], m2 = m[u][2], m3 = m[u][3];

@@ -58,3 +58,31 @@ def test_fp64_stored_products(n, warps, deck_dir):
     rs = np.linalg.cholesky(D) @ (g * np.sqrt(2 * dt))
     assert np.abs(s.compute_Rf() - df).max() <= 1e-12 * np.abs(df).max()
     assert np.abs(s.compute_r(g) - rs).max() <= 1e-12 * np.abs(rs).max()
+
+
+@pytest.mark.parametrize("n3", [1, 2, 3, 30, 33, 127, 129, 255, 1023, 3069, 3071])
+def test_noalloc_matrix_ends_with_its_last_element(n3):
+    """A caller's matrix may end with the last column of its last row; beyond
+    it nothing may be read."""
+    import torch
+    rng = np.random.default_rng(n3)
+    ld = (n3 + 3) // 4 * 4
+    flat = np.full(n3 * ld, np.nan, dtype=np.float32)
+    M = rng.standard_normal((n3, n3)).astype(np.float32)
+    for r in range(n3):
+        flat[r * ld:r * ld + n3] = M[r]
+    dD, F, X = rng.standard_normal((3, n3))
+    M = M.astype(np.float64)
+    U = np.triu(M, 1)
+    t = [torch.from_numpy(a).cuda() for a in (flat[:(n3 - 1) * ld + n3].copy(), dD, F, X)]
+    out = torch.full((2, n3), float("nan"), dtype=torch.float64, device="cuda")
+    lib = engine.load_library()
+    torch.cuda.synchronize()
+    rc = lib.bdb_stored_matvec_noalloc(t[0].data_ptr(), n3, ld, t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
+                                       1.0, out[0].data_ptr(), out[1].data_ptr(), None)
+    assert rc == 0, lib.bdb_last_error().decode()
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    bound = 4e-16 * np.sqrt(n3) * (np.abs(M).sum(axis=1).max() + 1)   # as above
+    assert np.abs(got[0] - (U @ F + U.T @ F + dD * F)).max() <= bound
+    assert np.abs(got[1] - np.tril(M) @ X).max() <= bound
