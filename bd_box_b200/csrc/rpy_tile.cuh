@@ -67,13 +67,23 @@ __device__ __forceinline__ float inv_sqrt(float x)
     return fmaf(0.5f * y, fmaf(-fmaf(x, y, -p), y, fmaf(-p, y, 1.0f)), y);
 }
 
+// A squared separation that has overflowed (beads 1.8e19 apart in FP32, 1.3e154
+// in FP64) as the largest finite number, or the residual above is inf * 0: the
+// tile is then as good as zero, not NaN. One integer (FP64) or minimum
+// operation a pair; a NaN stays one through the separation itself.
+__device__ __forceinline__ float below_inf(float x) { return fminf(x, 3.402823466e38f); }
+__device__ __forceinline__ double below_inf(double x)
+{
+    return __hiloint2double(min(__double2hiint(x), 0x7fefffff), __double2loint(x));
+}
+
 // diff_tensor_calc_pos(i, j) from the separation d = r_i - r_j and the two
 // radii (which enter symmetrically): A I + B d d^T, with one reciprocal
 // square root instead of a square root and four divisions.
 template <typename T>
 __device__ __forceinline__ void rpy_free_sep(const T* d, T si, T sj, T preDii, T preDij, T* t)
 {
-    const T r_sq = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    const T r_sq = below_inf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
     const T inv = inv_sqrt(r_sq);
     const T inv_sq = inv * inv, r = r_sq * inv;
     T A, B;

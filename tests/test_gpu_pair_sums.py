@@ -116,3 +116,28 @@ def test_lattice_sums_fp64_far_outside_the_box(r, alpha, boxes, axis, deck_dir):
         assert np.abs(a - b).max() <= 2e-16 * 8 * np.pi * (r + 1) * (2 * boxes + 1) * scale
     assert np.isfinite(s.compute_Rf()).all()
     assert np.isfinite(s.compute_r(np.random.default_rng(r).standard_normal(72))).all()
+
+
+@pytest.mark.parametrize("prec,far", [(engine.PREC_FP64, 1e155), (engine.PREC_MIXED, 1e20)])
+@pytest.mark.parametrize("hydro", ["geyer", "cholesky"])
+def test_a_bead_whose_distance_squared_overflows(prec, far, hydro, deck_dir):
+    """Its tiles with all other beads vanish: everyone else moves as without it."""
+    n = 70
+    d = decks.read_deck(decks.write_chain_deck(deck_dir, f"far_{hydro}", n, seed=6, hydro=hydro))
+    for k, w, m in (("bond", 2, 3), ("angle", 3, 2), ("angle_cos", 3, 2), ("dihe", 4, 2), ("dihe_angle", 4, 2)):
+        setattr(d, k + "_pairs", np.zeros((0, w), np.int32))
+        setattr(d, k + "_parms", np.zeros((0, m)))
+    d.coord = d.coord.copy()
+    out = []
+    for x in (300.0, far):
+        d.coord[n - 1, :3] = (x, -x, 0.5 * x)
+        s = engine.System(d, precision=prec, noise=engine.NOISE_HOST)
+        out.append((s.compute_D() if hydro == "cholesky" else s.compute_Rf()))
+        s.close()
+    near, gone = out
+    assert np.isfinite(gone).all()
+    if hydro == "cholesky":
+        assert np.array_equal(gone[:-3, :-3], near[:-3, :-3])
+        assert np.abs(gone[-3:, :-3]).max() <= 1e-15 * np.abs(gone).max()
+    else:   # no force acts on the far bead, nor does it change the others' drift
+        assert rel(gone[:-3], near[:-3]) <= (1e-13 if prec == engine.PREC_FP64 else 1e-6)
