@@ -1,0 +1,60 @@
+"""The lattice sums' own erfcx, 1/sqrt and Gaussian (rpy_tile.cuh) over their
+range, one image at a time: with R = 0 a pair's Smith tile is a single image
+and no reciprocal vector, a closed form of erfc(x) and exp(-x^2), x = alpha r."""
+import numpy as np
+import pytest
+
+from conftest import gpu_available
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="needs a CUDA device")]
+
+from bd_box_b200 import decks, engine  # noqa: E402
+
+L, RADIUS = 64.0, 1.0 / 256   # coordinates are multiples of 1/16: r/L and its square are exact in FP32 too
+
+
+@pytest.mark.parametrize("alpha", [0.25, 1.0, 1.75, 4.5, 20.0])
+@pytest.mark.parametrize("prec", [engine.PREC_FP64, engine.PREC_MIXED])
+def test_one_image(alpha, prec, deck_dir):
+    from scipy.special import erfcx
+    n = 80
+    box = {k: f"{L:.6f}" for k in ("xbox", "ybox", "zbox")}
+    d = decks.read_deck(decks.write_suspension_deck(
+        deck_dir, f"im{alpha}", n, seed=2, ewald_r=0, radius=RADIUS,
+        extra={"ewald_method": "smith", "ewald_alpha": alpha, "hydro": "cholesky", **box}))
+    d.coord = d.coord.copy()
+    rng = np.random.default_rng(int(4 * alpha))
+    # half the beads over the whole box, half near its middle: r/L from 0.001 to 1.7
+    x = rng.integers(-512, 512, size=(n, 3)) / 16
+    x[::2] = rng.integers(-24, 25, size=(n // 2, 3)) / 16
+    d.coord[:, :3] = x
+    s = engine.System(d, precision=prec, noise=engine.NOISE_HOST)
+    D = s.compute_D().reshape(n, 3, n, 3).transpose(0, 2, 1, 3)
+    s.close()
+    i, j = np.triu_indices(n, 1)
+    v = (x[i] - x[j]) / L
+    r2 = np.sum(v * v, axis=1)
+    keep = r2 > 0
+    if prec == engine.PREC_MIXED:   # images beyond erfc(4.45) are dropped there
+        keep &= alpha * alpha * r2 < 4.4 ** 2
+    i, j, v, r2 = i[keep], j[keep], v[keep], r2[keep]
+    assert len(i) > 100 and (prec == engine.PREC_MIXED or np.sqrt(r2).max() > 1)
+    r, a, s2 = np.sqrt(r2), d.prm["ewald_alpha"], (RADIUS / L) ** 2
+    g = np.exp(-(np.longdouble(a) ** 2) * r2.astype(np.longdouble))   # (its argument in 64 bits)
+    er = g * erfcx(a * r) / r
+    e = 2 * a * 0.5641895835 * g                                     # BD_BOX's 10 digits of 1/sqrt(pi)
+    sq = (er + e) / r2
+    A = 0.75 * er + 0.5 * s2 * sq
+    B = (0.75 * (er + e) - 0.5 * s2 * (3 * sq + 2 * a * a * e)) / r2
+    pre = 0.00010537375739171604 * d.prm["T"] / (d.prm["visc"] * d.prm["vfactor"]) / L
+    want = pre * (A[:, None, None] * np.eye(3) + B[:, None, None] * v[:, :, None] * v[:, None, :])
+    size = np.abs(want).max(axis=(1, 2))
+    err = np.abs(D[i, j] - want).max(axis=(1, 2)) / size
+    x2 = a * a * r2
+    if prec == engine.PREC_FP64:
+        # about 20 operations, and the rounding of the exponent, x^2 ulps
+        ok = size > 1e-290
+        assert (err[ok] <= 2.3e-16 * (24 + 2 * x2[ok].astype(float))).all()
+    else:
+        # the exponent's rounding is put back: no growth with x^2
+        assert (err <= 6e-8 * 24).all(), err.max() / 6e-8
