@@ -3,8 +3,7 @@ such a segment is sorted by several CTAs (bitonic chunks, then merge passes
 in global memory) and must give BD_BOX's forces and pair counts, not fall
 back to all pairs. Checked at N = 20,000 against the oracle's O(N^2) forces
 (oracle/bdb_oracle.c, force_single over all pairs): a free-space chain and a
-periodic suspension, before and after the beads move far enough to force a
-re-sort. Pair counts bit-exact; forces 1e-12 of the largest, energies 1e-10.
+periodic suspension, at several positions. Pair counts bit-exact; forces 1e-12 of the largest, energies 1e-10.
 """
 import numpy as np
 import pytest
@@ -50,8 +49,8 @@ def test_large_segment_cells_match_oracle(kind, tmp_path):
     rng = np.random.default_rng(11)
     c0 = check(s, o, deck.coord)
     assert c0[0] + c0[1] > 0
-    # a small move (within the skin: the old sort stays), then a large one
-    # (every bead several angstroms: a re-sort)
+    # a small move, then a large one (set_coord sorts afresh either way; what
+    # steps do is in test_gpu_cells_kept.py)
     x = deck.coord.copy()
     x[:, :3] += rng.normal(size=(deck.n, 3)) * 0.05
     check(s, o, x)

@@ -55,6 +55,27 @@ def test_mixed_batch_follows_fp64(sizes, deck_dir):
         assert rel(a, b) <= 1e-6
 
 
+def test_jobs_of_several_column_tiles(deck_dir):
+    """39,600 tile pairs: jobs of 2 column tiles on two row tiles in FP32, of 4
+    in FP64 (their row sums take two records, or one FP64). Each segment as it
+    is alone, where a job is half a tile pair."""
+    ds = [decks.read_deck(decks.write_chain_deck(deck_dir, f"jt{n}", n, seed=n, hydro="geyer")) for n in (1300, 1281)]
+    batch = [ds[0]] * 45 + [ds[1]]
+    rng = np.random.default_rng(8)
+    g = rng.standard_normal(3 * sum(d.n for d in batch))
+    for prec, tol in ((engine.PREC_FP64, 1e-13), (engine.PREC_MIXED, 1e-6)):
+        s = engine.System(batch, precision=prec, noise=engine.NOISE_HOST)
+        rf, rs = s.compute_Rf(), s.compute_r(g)
+        s.close()
+        for k in (0, 17, 44, 45):
+            lo = 3 * 1300 * k
+            sl = slice(lo, lo + 3 * batch[k].n)
+            a = engine.System(batch[k], precision=prec, noise=engine.NOISE_HOST)
+            assert rel(rf[sl], a.compute_Rf()) <= tol
+            assert rel(rs[sl], a.compute_r(g[sl])) <= tol
+            a.close()
+
+
 @pytest.mark.parametrize("method", ["beenakker", "smith"])
 @pytest.mark.parametrize("r", [2, 3, 4, 5])
 @pytest.mark.parametrize("kind", ["plain", "radii", "outside", "overlap"])
