@@ -268,6 +268,23 @@ __device__ __forceinline__ void add_image(float* o, float A, float B, float x, f
     o[5] += by * z;
 }
 
+// every image of the FP64 sum with an exponential of its own (see lattice_sum)
+static __device__ __noinline__ void images_one_by_one(const EwaldConst& ec, const double* v, double s2, double* o)
+{
+    const RealSpace<double> rs(ec, s2);
+    for (int h = -ec.R; h <= ec.R; ++h)
+        for (int f = -ec.extent[h * h]; f <= ec.extent[h * h]; ++f) {
+            const int ng = ec.extent[h * h + f * f];
+            for (int g = -ng; g <= ng; ++g) {
+                const double x = v[0] + h, y = v[1] + f, z = v[2] + g, r2 = x * x + y * y + z * z;
+                if (r2 == 0.0) continue;
+                double A, B;
+                rs.image(r2, exp(-ec.a2 * r2), A, B);
+                add_image(o, A, B, x, y, z);
+            }
+        }
+}
+
 // The lattice sum S(v) over the reference's sphere of images and reciprocal
 // vectors, v = (r_i - r_j)/L as it is (no minimum image). Bound by FP64
 // multiply-adds and their latency (about 90 a image; N = 777, R = 3, Smith:
@@ -309,16 +326,23 @@ __device__ __forceinline__ void lattice_sum(const EwaldConst& ec, const double* 
             }
         }
     } else {
-        const double z0 = v[2];
-        const double up0 = exp(-ec.a2 * (1 + 2 * z0)), down0 = exp(-ec.a2 * (1 - 2 * z0));
         // The recurrence holds while up0 and down0 stay finite and the Gaussian
         // at g = 0 does not underflow: positions in the box have |v_k| <= 1
         // (m = 1). Beyond (strong screening; positions that a caller has set
         // many boxes away, 0 * inf from |z0| ~ 113 at alpha = sqrt(pi)) every
         // image takes its own exponential. a2 (1 + 2 |z0|) <= a2 (R + 1 + m)^2.
         const double m = R + 1 + fmax(1.0, fmax(fabs(v[0]), fmax(fabs(v[1]), fabs(v[2]))));
+        const double z0 = v[2];
+        const double up0 = exp(-ec.a2 * (1 + 2 * z0)), down0 = exp(-ec.a2 * (1 - 2 * z0));
         const bool run = ec.a2 * m * m < 600.0;
-        for (int h = -R; h <= R; ++h) {
+        if (!run) {
+            const double w[3] = {v[0], v[1], v[2]};
+            double e[6] = {0, 0, 0, 0, 0, 0};
+            images_one_by_one(ec, w, s2, e);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) o[k] = e[k];
+        }
+        for (int h = run ? -R : R + 1; h <= R; ++h) {
             const double x = v[0] + h;
             const int nf = ec.extent[h * h];
             for (int f = -nf; f <= nf; ++f) {
@@ -335,7 +359,7 @@ __device__ __forceinline__ void lattice_sum(const EwaldConst& ec, const double* 
                         const double r2 = xy + z * z;
                         if (r2 != 0.0) {
                             double A, B;
-                            rs.image(r2, run ? ex : exp(-ec.a2 * r2), A, B);
+                            rs.image(r2, ex, A, B);
                             add_image(o, A, B, x, y, z);
                         }
                         z += step;
