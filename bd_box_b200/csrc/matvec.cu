@@ -84,6 +84,10 @@ __device__ __forceinline__ void mv_tile(const T* __restrict__ M, size_t ld, int 
     double x[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) x[v] = !MASK || c + v < n3 ? w[c + v] : 0.0;
+    // rows this lane loads 16 bytes of: all, but not the last where its columns
+    // end before them, since there a caller's matrix may end (mv_tail adds
+    // those; the other rows are followed by the next)
+    const int rows = c < n3 ? n3 - (c + 3 >= n3) : 0;
 #pragma unroll 1
     for (int g = 0; g < STRIP; g += G) {
         T m[G][4];
@@ -91,20 +95,12 @@ __device__ __forceinline__ void mv_tile(const T* __restrict__ M, size_t ld, int 
 #pragma unroll
         for (int u = 0; u < G; ++u) {
             const int r = r0 + g + u;
-            if (!MASK || (r < n3 - (c + 3 >= n3) && c < n3)) {
+            if (!MASK || r < rows) {
                 load4(M + (size_t)r * ld + c, m[u]);
             } else {
                 m[u][0] = m[u][1] = m[u][2] = m[u][3] = (T)0;
             }
         }
-        // the last row's last columns by themselves: beyond them a caller's
-        // matrix may end (the other rows are followed by the next)
-        if (MASK && c + 3 >= n3 && r0 + g < n3 && r0 + g + G >= n3)
-#pragma unroll
-            for (int u = 0; u < G; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    if (r0 + g + u == n3 - 1 && c + v < n3) m[u][v] = M[(size_t)(n3 - 1) * ld + c + v];
         if (MASK)
 #pragma unroll
             for (int u = 0; u < G; ++u)
@@ -142,11 +138,27 @@ __device__ __forceinline__ void mv_tile(const T* __restrict__ M, size_t ld, int 
     }
 }
 
-// the run's row sums go out and start again from zero
-__device__ __forceinline__ void mv_rows(double* sRow, double* __restrict__ dst, int r0, int n3, int lane)
+// The last row's product with its last n3 mod 4 columns (left of the diagonal
+// or on it), which its lane in mv_tile leaves out
+template <typename T>
+__device__ __forceinline__ double mv_tail(const T* __restrict__ M, size_t ld, int n3, const double* __restrict__ X)
+{
+    const T* row = M + (size_t)(n3 - 1) * ld;
+    double a = 0.0;
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        const int c = (n3 & ~3) + v;
+        if (c < n3) a += (double)row[c] * X[c];
+    }
+    return a;
+}
+
+// the run's row sums (and a lane's tail) go out and start again from zero
+__device__ __forceinline__ void mv_rows(double* sRow, double* __restrict__ dst, int r0, int n3, int lane,
+                                        double tail = 0.0)
 {
     __syncwarp();
-    if (r0 + lane < n3) dst[r0 + lane] = sRow[lane];
+    if (r0 + lane < n3) dst[r0 + lane] = sRow[lane] + tail;
     sRow[lane] = 0;
     __syncwarp();
 }
@@ -187,8 +199,9 @@ k_strip_mv(const T* __restrict__ M, int n3, size_t ld, int nseg, int seg_tiles, 
             else mv_tile<T, 0, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, X, sF, sRow, lane, pc);
         }
         if (J < J1 && J == Jd) {
+            const double tail = r0 + lane == n3 - 1 ? mv_tail(M, ld, n3, X) : 0.0;
             mv_tile<T, 0, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, X, sF, sRow, lane, pc);
-            mv_rows(sRow, rowp + (size_t)seg * n3, r0, n3, lane);
+            mv_rows(sRow, rowp + (size_t)seg * n3, r0, n3, lane, tail);
             pc[0] = pc[1] = pc[2] = pc[3] = 0;
             mv_tile<T, 1, true>(M, ld, n3, r0, MV_TILE * J + 4 * lane, F, sF, sRow, lane, pc);
             put_cols(J);
