@@ -14,11 +14,11 @@
 //    order, forms eps and beta of its segment (diff_rand.c:197-217) from the
 //    jobs' partials, and writes Rf and Rs.
 // Bound by instruction issue: per pair the tile (~30), two sets of products
-// (~60) and a ninth of the hand-over each, ~150 in all in FP32 (69% of the
-// issue slots of the 256-replica batch); in FP64 by the FP64 pipe. One row sum
-// per lane over 5 exchanges of 9 values per pair, as a warp holding rows of a
-// tile needs, took more than the tile itself: N = 3000 in FP64 124 -> 49 us, the
-// 256-replica batch 748 -> 320 us per step.
+// (~60) and a ninth of the hand-over each, ~150 in all in FP32; in FP64 by the
+// FP64 pipe. One row sum per lane over 5 exchanges of 9 values per pair, as a
+// warp holding rows of a tile needs, took more than the tile itself: N = 3000
+// in FP64 124 -> 50 us, the 256-replica batch 748 -> 342 us per step (319 with FP32 sums over whole
+// jobs and single FP32 records, which lost precision against those tiles).
 // Which warp runs a job does not change a bit: each job writes records of its
 // own, and they are added in the order of the job list.
 #include <cuda_runtime.h>
@@ -236,9 +236,9 @@ __device__ __forceinline__ void pair_tile(const TensorArgs& A, const FastArg<KIN
 // 16 only half of the lanes, so that every pair is met once).
 template <typename T, int KIND, bool RS, int NR>
 __device__ __forceinline__ void tea_steps(const TensorArgs& A, const FastArg<KIND>& E,
-                                          const double4* __restrict__ pos, const ColData<T>& cols, const Bead<T> (&row)[NR], int i0, int ni, int j0,
-                                          int nj, int s0, int s1, bool diag, T (&racc)[NR][RS ? 9 : 3],
-                                          T (&cacc)[RS ? 9 : 3], T& eps)
+                                          const double4* __restrict__ pos, const ColData<T>& cols,
+                                          const Bead<T> (&row)[NR], int i0, int ni, int j0, int nj, int s0, int s1,
+                                          bool diag, T (&racc)[NR][RS ? 9 : 3], T (&cacc)[RS ? 9 : 3], T& eps)
 {
     constexpr int NV = RS ? 9 : 3;
     const int lane = threadIdx.x & 31;
@@ -281,7 +281,8 @@ __device__ __forceinline__ void tea_steps(const TensorArgs& A, const FastArg<KIN
 // sums; the row sums of a job with several column tiles take two.
 template <typename T, int KIND, bool RS>
 __global__ void __launch_bounds__(32 * TEA_WARPS, sizeof(T) == 4 && KIND == TILE_FREE ? 4 : 3)
-k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastArg<KIND> E, const TileJob* __restrict__ jobs, int n_jobs, const int* __restrict__ col_rec,
+k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastArg<KIND> E,
+            const TileJob* __restrict__ jobs, int n_jobs, const int* __restrict__ col_rec,
             const TeaSeg* __restrict__ segs, const double4* __restrict__ pos, const double* __restrict__ F,
             const double* __restrict__ X, T* __restrict__ part, double* __restrict__ eps_part, const PairUnits units)
 {
@@ -299,6 +300,7 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
     const int end = sg.begin + sg.count;
     const int i0 = sg.begin + TT * jb.I, ni = end - i0;
     const double4 org = pos[i0];
+    const bool one = jb.nJ == 1 && jb.s1 - jb.s0 <= CHUNK;   // FP32: a single chunk
     double eps = 0;   // FP32: a chunk's sum at a time (at most 16 pairs a lane)
     Bead<T> b;
 
@@ -337,19 +339,22 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
             } else {
                 // FP32 sums of 8 steps at a time, the chunks' sums in FP64, in
                 // shared memory at the bead's own slot (the column's at its
-                // number): rows over the whole job, columns over the tile
+                // number): rows over the whole job, columns over the tile. A
+                // job of one chunk keeps its sums in registers (N = 1000:
+                // 43.0 -> 41.1 us a step).
                 for (int s = jb.s0; s < jb.s1; s += CHUNK) {
                     const int e = min(s + CHUNK, jb.s1), l = (lane + e) & 31;
-                    T rc[NR][NV], eps_c = 0;
+                    T eps_c = 0;
 #pragma unroll
                     for (int k = 0; k < NV; ++k) {
                         cacc[k] = 0;
 #pragma unroll
-                        for (int r = 0; r < NR; ++r) rc[r][k] = 0;
+                        for (int r = 0; r < NR; ++r) racc[r][k] = 0;
                     }
-                    tea_steps<T, KIND, RS, NR>(A, E, pos, cols, row, i0, ni, j0, end - j0, s, e, jb.type == JOB_DIAG, rc,
-                                               cacc, eps_c);
+                    tea_steps<T, KIND, RS, NR>(A, E, pos, cols, row, i0, ni, j0, end - j0, s, e, jb.type == JOB_DIAG,
+                                               racc, cacc, eps_c);
                     eps += (double)eps_c;
+                    if (one) break;
                     __syncwarp();   // lanes take turns at a column's slot
 #pragma unroll
                     for (int k = 0; k < NV; ++k) {
@@ -358,14 +363,16 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
 #pragma unroll
                         for (int r = 0; r < NR; ++r) {
                             double* p = &s_row[warp][NV * r + k][lane];
-                            *p = q == 0 && s == jb.s0 ? (double)rc[r][k] : *p + (double)rc[r][k];
+                            *p = q == 0 && s == jb.s0 ? (double)racc[r][k] : *p + (double)racc[r][k];
                         }
                     }
                 }
-                __syncwarp();
+                if (!one) {
+                    __syncwarp();
 #pragma unroll
-                for (int k = 0; k < NV; ++k) cacc[k] = (T)s_sum[warp][k][(lane + jb.s1) & 31];
-                __syncwarp();
+                    for (int k = 0; k < NV; ++k) cacc[k] = (T)s_sum[warp][k][(lane + jb.s1) & 31];
+                    __syncwarp();
+                }
             }
             if (jb.type == JOB_DIAG) {
                 // row and column sums of the same beads: one record in FP64,
@@ -383,13 +390,13 @@ k_tea_pairs(const __grid_constant__ TensorArgs A, const __grid_constant__ FastAr
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const int rec = r ? jb.rec1 : jb.rec0;
-            if constexpr (sizeof(T) == 4) {
+            if (sizeof(T) == 4 && !one) {
                 // the FP64 sum over several tiles goes out as two FP32
                 // records, its FP32 value and what that leaves
                 T lo[NV];
 #pragma unroll
                 for (int k = 0; k < NV; ++k) {
-                    const double v = s_row[warp][NV * r + k][lane];
+                    const double v = s_row[warp][sizeof(T) == 4 ? NV * r + k : 0][lane];
                     racc[r][k] = (T)v;
                     lo[k] = (T)(v - (double)racc[r][k]);
                 }
