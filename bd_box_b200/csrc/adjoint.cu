@@ -702,7 +702,8 @@ static int adjoint_linalg(bdb_system* s, const T* M, int np, int n3, int nrb, in
                           double* colp, double* rowp, double* u, double* v, const double* Xp, const AdjLinalg<T>& w)
 {
     cudaStream_t st = s->stream;
-    const int smem = (int)sizeof(GemmSmem<T, GT>), lev_smem = (int)sizeof(GemmSmem<T, 64>), tri_smem = 2 * 64 * 65 * (int)sizeof(T);
+    const int smem = (int)sizeof(GemmSmem<T, GT>), lev_smem = (int)sizeof(GemmSmem<T, 64>);
+    const int tri_smem = 2 * 64 * 65 * (int)sizeof(T);
     BDB_CUDA(cudaFuncSetAttribute(k_trinv64<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem));
     BDB_CUDA(cudaFuncSetAttribute(k_tri_level<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lev_smem));
     BDB_CUDA(cudaFuncSetAttribute(k_tri_level<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lev_smem));
@@ -796,9 +797,11 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     const int nck = (K + checkpoint - 1) / checkpoint, seg_len = std::min(K, checkpoint);
     const int nrb = (n3 + MV2_ROWS - 1) / MV2_ROWS, ncb = (n3 + MV2_COLS - 1) / MV2_COLS;
     const size_t nn = (size_t)np * np, el = mixed ? sizeof(float) : sizeof(double);
-    // the vectors and lists share one allocation: 15 driver calls and as many
-    // frees spread a call's time (40 calls at n = 3072: median 28.0 ms, mean 31
-    // to 57, the slowest 941; with one 28.0, 29 to 30 and 69)
+    // one allocation for the matrices, vectors and lists, one for what is
+    // kept. A call's time still spreads: 40 calls at n = 3072 in each of three
+    // processes had a median of 27.8 ms, means of 28, 29 and 47 and slowest
+    // calls of 55, 57 and 718 ms (cause not shown; with 15 more allocations the
+    // means were 31 to 57)
     Part<double> lam, lam2, u, v, Xp, colp, rowp, ppart;
     Part<double4> ckpt, seg, xK;
     Part<int> d_bptr, d_blist;
@@ -936,8 +939,8 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
                 w.A = reinterpret_cast<T*>(dense.p);
                 w.S = w.A + nn + (size_t)np * GT;
                 w.part = w.S + nn;
-                const int r = adjoint_linalg<T>(s, keep ? reinterpret_cast<const T*>(Mseg) + (size_t)slot * nn : M, np,
-                                                n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p, Xp.p, w);
+                const T* Mk = keep ? reinterpret_cast<const T*>(Mseg) + (size_t)slot * nn : M;
+                const int r = adjoint_linalg<T>(s, Mk, np, n3, nrb, ncb, lam.p, colp.p, rowp.p, u.p, v.p, Xp.p, w);
                 if (r) return r;
                 BDB_CUDA(cudaMemcpyAsync(lam2.p, lam.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
                 k_tile_grad<T><<<warps_blocks, 256, 0, st>>>(n, x, s->preDii, s->preDij, c, lam.p, Fk, w.S, np, lam2.p);

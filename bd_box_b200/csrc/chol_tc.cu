@@ -643,8 +643,8 @@ __global__ void __launch_bounds__(TRSM_THREADS, 1) k_trsm128(T* __restrict__ M, 
             return;
         }
     }
-    // block row P+1 (unit0 = 0) releases its dependent, the chain's one-CTA
-    // update, at once; the rows below only as their warps finish, because
+    // block row P+1 (unit0 = 0) releases its dependent, the chain's update of
+    // the next diagonal tile (k_syrk_diag, 10 CTAs), at once; the rows below only as their warps finish, because
     // theirs is the side stream's column update, a grid that would
     // otherwise wait on the free SMs the chain needs while this runs
     if (unit0 == 0) asm volatile("griddepcontrol.launch_dependents;");
@@ -1684,8 +1684,10 @@ static int factor_schedule(bdb_system* s, T* M, Update update)
     const int chain = std::min(std::max(s->chain_sms, 1), s->sm_count - 1);
     const int bulk_sms = std::max(1, s->sm_count - chain);
     const int per_cta = TRSM_THREADS / 32, units_top = PW / 8;
-    // the side kernels take the chain's SMs but five (the diagonal block,
-    // the four CTAs of the top panel solve); the panel solve two CTAs per SM
+    // the side kernels take the chain's SMs but five: the diagonal block and
+    // the four CTAs of the top panel solve. k_syrk_diag runs between those two,
+    // when their five SMs are free, and its small CTAs (128 threads, 35 KB; 70
+    // in FP64) also fit beside the side kernels'. The panel solve two CTAs per SM
     // (its registers and shared memory allow it), for more warps on the FP64
     // pipes
     const int side = std::max(1, chain - 5);

@@ -433,8 +433,9 @@ __global__ void k_sorted_pos(int n, const double4* __restrict__ pos, const int* 
 
 // force_single for the pair (a, b), a < b, at separation v = r_b - r_a,
 // accumulating the force on a (self_a) or b. Energies and pair counts are
-// credited only to a. conn: 1-2 bonded, with the scale factors in force. The cutoff tests and the overlap decision
-// use the exact r_norm; the magnitudes share one reciprocal of it.
+// credited only to a. conn: 1-2 bonded, with the scale factors in force. The
+// cutoff tests and the overlap decision use the exact r_norm; the magnitudes
+// share one reciprocal of it.
 template <bool kEnergy>
 __device__ __forceinline__ void pair_term(const ForceParams& fp, const double* v, double qa, double qb,
                                           const double2& la, const double2& lb, bool conn, bool self_a, double* f,
@@ -517,16 +518,15 @@ __device__ __forceinline__ void pair_sep(const double4& a, const double4& b, con
 
 // One warp per bead i over the candidate beads of its 27 neighbour cells
 // (or of the whole segment for brute-force segments). A cell is as wide as
-// the widest interaction plus the skin, so only about a seventh of the
-// candidates of a dense system interact: the lanes first keep those within
+// the widest interaction plus the skin, so only a small part of the
+// candidates of a dense system interact (173 of 1,480 at N = 20,000): the lanes first keep those within
 // `reach` (the widest interaction, padded: the exact cutoff tests follow) in
 // a list per warp, and the pair terms -- some 150 FP64 operations -- run in
 // full rounds of 32 from it, not once per round of candidates with a few
 // lanes live. What does not depend on the candidates (the bead's bonded slots
 // and neighbours) is loaded before them: a warp is bound by the latency of its
-// chain of loads. N = 20,000 at 173 neighbours of 1,480 candidates: 398 -> 240
-// us (300 from unsorted positions); 256 chains of 64..1024 beads:
-// 287 -> 260.
+// chain of loads. That N = 20,000: 398 -> 240 us (300 from unsorted
+// positions); 256 chains of 64..1024 beads: 287 -> 260.
 // Each lane accumulates in a fixed order and the warp combines the lanes with
 // a fixed xor tree, so the result is deterministic. kEnergy: energies and pair
 // counts per bead (steps need neither), for k_energy_reduce.
@@ -1072,7 +1072,7 @@ int set_force_time(bdb_system* s, double t)
 }
 
 // Energies: E[1..5] from the bonded terms (sums per type), E[6], E[7] from
-// the non-bonded block partials. One CTA, fixed order.
+// the non-bonded kernel's per-bead partials.
 struct TermRanges {
     int lim[6];   // [lim[t], lim[t+1]) are the terms of type t
 };
@@ -1381,9 +1381,10 @@ int forces_run(bdb_system* s, bool want_energy, bool want_counts)
     }
     auto nonbonded = [&](auto kern) {
         kern<<<nblk, NB_THREADS, 0, st>>>(make_fp(s), s->n, s->pos.p, s->Q.p, s->LJ.p, s->d_bead_seg.p, s->d_segs.p,
-                                          s->cell_range.p, s->cell_off.p, s->sorted_idx.p, sp, s->grid.p, s->grid_dims.p,
-                                          s->conn_ptr.p, s->conn_list.p, Fb, s->n_terms ? s->slot_ptr.p : nullptr, s->slot_list.p,
-                                          s->contrib.p, s->F.p, s->e_part.p, s->c_part.p, s->status.p);
+                                          s->cell_range.p, s->cell_off.p, s->sorted_idx.p, sp, s->grid.p,
+                                          s->grid_dims.p, s->conn_ptr.p, s->conn_list.p, Fb,
+                                          s->n_terms ? s->slot_ptr.p : nullptr, s->slot_list.p, s->contrib.p, s->F.p,
+                                          s->e_part.p, s->c_part.p, s->status.p);
     };
     if (want_energy || want_counts) sp ? nonbonded(k_nonbonded<true, true>) : nonbonded(k_nonbonded<true, false>);
     else sp ? nonbonded(k_nonbonded<false, true>) : nonbonded(k_nonbonded<false, false>);

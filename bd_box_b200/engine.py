@@ -369,7 +369,9 @@ class System:
         self._check(self.lib.bdb_autotune(self.h, int(enable)))
 
     def tuning(self):
-        """(TEA tile edge, stored-matvec warps per SM) in use."""
+        """(TEA job length, stored-matvec warps per SM) in use. The job length
+        keeps the name and values that it had as a tile's edge: 16 makes the
+        pair kernel's jobs half as long as 32."""
         a, b = C.c_int(), C.c_int()
         self._check(self.lib.bdb_get_tuning(self.h, C.byref(a), C.byref(b)))
         return a.value, b.value

@@ -543,8 +543,8 @@ def adjoint_case(torch, engine):
     every 20; loss = mean squared deviation of 128 seeded bead-pair distances
     from seeded targets in [10, 60] A. The electrostatic and LJ cutoffs lie
     beyond the chain's extent, so no pair crosses a cutoff under the finite
-    differences. The mixed-precision adjoint (FP32 forward and triangular
-    solves, FP64 sums) and the FP64 one are timed; both are checked against
+    differences. The mixed-precision adjoint (FP32 forward, inverse
+    and products, FP64 sums) and the FP64 one are timed; both are checked against
     central differences (h = 1e-4) of the FP64 forward along a random
     direction of the initial positions and for the four scale factors (LJ
     epsilon, LJ sigma, bond H, Debye length)."""

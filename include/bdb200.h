@@ -316,6 +316,7 @@ int bdb_set_adjoint_keep(bdb_system* s, long long bytes);
  * SM).
  * Switch it on before the first step. */
 int bdb_autotune(bdb_system* s, int enable);
+/* tea_tile: the TEA job length, under the name it had as a tile's edge */
 int bdb_get_tuning(bdb_system* s, int* tea_tile, int* mv_warps_per_sm);
 int bdb_set_tuning(bdb_system* s, int tea_tile, int mv_warps_per_sm);
 
