@@ -300,7 +300,7 @@ __global__ void k_mv2_finish(int n, int nrb, int ncb, const double* __restrict__
 // n^3/3 multiply-adds for one half of it and n^3/6 for the inverse, all in
 // 128 x 128 tiles, in about 18 launches; two blocked triangular solves with n
 // right-hand sides take n^3 in 190 launches of narrow updates (n = 3072, FP32:
-// 4.2 ms a step before, 1.35 now).
+// 4.2 ms a step before, 1.34 now).
 
 // Room: A and G are lower triangular and share one buffer, n rows of n + 128:
 // row block C (128 rows) of G lies in row block nb - 1 - C, right of A's last
@@ -402,10 +402,15 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T, TILE>& sm, const RA A, int
     constexpr int HX = TILE / 8;                                 // threads along a tile's side
     const int tid = threadIdx.x, tx = tid % HX, ty = tid / HX;
     T ra[NP][8], rb[NP][8];
+    // 16 rows from a multiple of 16: in one row block of 128
+    const T* a0 = TA ? A.at(k0) + ma : nullptr;
+    const T* b0 = B.at(k0) + nb;
     auto load = [&](int k) {
-        // 16 rows from a multiple of 16: in one row block of 128
-        const T* a0 = TA ? A.at(k) + ma : nullptr;
-        const T* b0 = B.at(k) + nb;
+        if (k > k0) {
+            const bool next = (k & 127) == 0;
+            if (TA) a0 = next ? A.at(k) + ma : a0 + 16 * A.ld;
+            b0 = next ? B.at(k) + nb : b0 + 16 * B.ld;
+        }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             const int e = tid + NT * p, kr = e / HX, c8 = 8 * (e % HX);   // a row of TILE in pieces of 8
@@ -798,10 +803,10 @@ extern "C" int bdb_adjoint(bdb_system* s, int K, int checkpoint, int npairs, con
     const int nrb = (n3 + MV2_ROWS - 1) / MV2_ROWS, ncb = (n3 + MV2_COLS - 1) / MV2_COLS;
     const size_t nn = (size_t)np * np, el = mixed ? sizeof(float) : sizeof(double);
     // one allocation for the matrices, vectors and lists, one for what is
-    // kept. A call's time still spreads: 40 calls at n = 3072 in each of three
-    // processes had a median of 27.8 ms, means of 28, 29 and 47 and slowest
-    // calls of 55, 57 and 718 ms (cause not shown; with 15 more allocations the
-    // means were 31 to 57)
+    // kept. A call's time spreads with the driver's share of it: 40 calls at
+    // n = 3072 in each of three processes had a median of 27.8 ms, means of 28,
+    // 29 and 47 and slowest calls of 55, 57 and 718 ms; an allocation or free of
+    // such a size by itself takes 0.4 to 0.8 ms, at times 100
     Part<double> lam, lam2, u, v, Xp, colp, rowp, ppart;
     Part<double4> ckpt, seg, xK;
     Part<int> d_bptr, d_blist;

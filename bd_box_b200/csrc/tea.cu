@@ -17,8 +17,9 @@
 // (~60) and a ninth of the hand-over each, ~150 in all in FP32; in FP64 by the
 // FP64 pipe. One row sum per lane over 5 exchanges of 9 values per pair, as a
 // warp holding rows of a tile needs, took more than the tile itself: N = 3000
-// in FP64 124 -> 50 us, the 256-replica batch 748 -> 342 us per step (319 with FP32 sums over whole
-// jobs and single FP32 records, which lost precision against those tiles).
+// in FP64 124 -> 50 us, the 256-replica batch 748 -> 342 us per step (319 with
+// FP32 sums over whole tiles, single FP32 records and eps in FP32, which lost
+// precision against that form).
 // Which warp runs a job does not change a bit: each job writes records of its
 // own, and they are added in the order of the job list.
 #include <cuda_runtime.h>
