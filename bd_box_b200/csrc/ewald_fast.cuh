@@ -7,9 +7,9 @@
 // cell matter (the next lie beyond erfc ~ 3e-10), and the rest is a Fourier
 // sum over |k|^2 <= 36 whose vectors collapse into 163 classes of signs: six
 // multiply-adds each on 21 cosines and sines built from one sincos per axis.
-// About 2,700 instructions per pair (76% of the issue slots), against ~65
+// About 2,700 instructions per pair (74% of the issue slots), against ~65
 // images of ~60 and 128 cosines in the reference's split, with lanes idle at
-// its cutoff: N = 4096, R = 4 (Beenakker): pair kernel 8.13 -> 0.85 ms.
+// its cutoff: N = 4096, R = 4 (Beenakker): pair kernel 8.13 -> 0.84 ms.
 // The near part is the RPY tensor screened as in Smith's sums (Hasimoto's
 // functions: the least Fourier tail); the Fourier weights are its complement
 // for the periodic RPY tensor (Smith) or, for Beenakker's sums, the
@@ -17,9 +17,12 @@
 // reciprocal weights. A constant on the diagonal, from the k = 0 terms, is
 // fixed by the reference's sum at given points, which also decide whether
 // the two agree (ewald_fast_setup).
-// D F and TEA noise against 64 bits at N = 4096: 5.3e-7 and 1.2e-7 relative,
-// 8.5e-7 and 9.2e-7 with the reference's split in FP32 (its sums of ~65 images
-// and 128 FP32 cosines of phases up to 4 round more).
+// Weights and sums are FP32, the Fourier sum's too, where the reference's split
+// on this path adds its reciprocal vectors in FP64 (lattice_sum). The error is
+// smaller all the same, since that split sums ~65 images in FP32: D F and TEA
+// noise against FP64 at N = 4096, R = 4: Beenakker 4.6e-7 and 1.0e-7 relative
+// (8.6e-7 and 9.4e-7 by the reference's split), Smith 7.1e-7 and 5.5e-8 (8.2e-7 and
+// 6.8e-8); N = 600, R = 4 and 5, three seeds, lower in each.
 #pragma once
 
 #include "rpy_tile.cuh"

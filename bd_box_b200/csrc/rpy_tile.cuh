@@ -52,8 +52,9 @@ struct EwaldConst {
 
 // 1/sqrt(x) for normal x: the hardware's estimate and Newton-Raphson steps in
 // residual form, y <- y + y/2 (1 - x y^2). FP64: the estimate has ~20 bits, two
-// steps leave its rounding (1 ulp). FP32: one step with the
-// product's rounding put back, 0.5 ulp (0.8 without, 2 of the estimate).
+// steps leave its rounding (1 ulp). FP32: one step, 0.8 ulp against 2 of the
+// estimate; inv_sqrt_half, for the free-space tile, which takes its cube, puts
+// the rounding of x y back as well: 0.5 ulp.
 __device__ __forceinline__ double inv_sqrt(double x)
 {
     double y;
@@ -62,6 +63,12 @@ __device__ __forceinline__ double inv_sqrt(double x)
     return fma(0.5 * y, fma(-(x * y), y, 1.0), y);
 }
 __device__ __forceinline__ float inv_sqrt(float x)
+{
+    const float y = rsqrtf(x);
+    return fmaf(0.5f * y, fmaf(-(x * y), y, 1.0f), y);
+}
+__device__ __forceinline__ double inv_sqrt_half(double x) { return inv_sqrt(x); }
+__device__ __forceinline__ float inv_sqrt_half(float x)
 {
     const float y = rsqrtf(x), p = x * y;
     return fmaf(0.5f * y, fmaf(-fmaf(x, y, -p), y, fmaf(-p, y, 1.0f)), y);
@@ -84,7 +91,7 @@ template <typename T>
 __device__ __forceinline__ void rpy_free_sep(const T* d, T si, T sj, T preDii, T preDij, T* t)
 {
     const T r_sq = below_inf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    const T inv = inv_sqrt(r_sq);
+    const T inv = inv_sqrt_half(r_sq);
     const T inv_sq = inv * inv, r = r_sq * inv;
     T A, B;
     if (r < si + sj) {
