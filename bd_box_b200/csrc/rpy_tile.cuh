@@ -35,6 +35,10 @@ struct EwaldConst {
     double L = 0, inv_L = 0;
     double alpha = 0, a2 = 0;       // alpha L and its square
     double isp = 0;                 // 1/sqrt(pi), spelled as each method spells it
+    // RealSpace's constants, [0] + [1] sigma^2/L^2, each rounded once from
+    // extended precision: their rounding is the same in every image of every
+    // pair, and with it the tensor's mean
+    double e2 = 0, as = 0, c0[2] = {0, 0}, c1[2] = {0, 0}, c2 = 0, d0[2] = {0, 0}, d1[2] = {0, 0};
     double two_pif = 0;             // 2*M_PIF evaluated in float
     double kappa = 0;               // exp(-2 a2): second ratio of the Gaussian along an axis
     // isqrt(R^2 - q), the extent of a row of the sphere, for q = 0 .. R^2
@@ -215,15 +219,14 @@ struct RealSpace {
     static constexpr bool kLo = sizeof(T) == 4;
     __device__ RealSpace(const EwaldConst& ec, double s2d)
     {
-        const double a = ec.alpha, a3 = a * ec.a2, a5 = a3 * ec.a2, isp = ec.isp;
-        alpha = Const2<T>(a);
-        e2 = Const2<T>(2 * a * isp);
-        as = Const2<T>(a * s2d * isp);
-        c0 = Const2<T>((14 * a3 * s2d - 4.5 * a) * isp);
-        c1 = Const2<T>((3 * a3 - 20 * a5 * s2d) * isp);
-        c2 = Const2<T>(4 * a5 * ec.a2 * s2d * isp);
-        d0 = Const2<T>((1.5 * a - 2 * a3 * s2d) * isp);
-        d1 = Const2<T>((16 * a5 * s2d - 3 * a3) * isp);
+        alpha = Const2<T>(ec.alpha);
+        e2 = Const2<T>(ec.e2);
+        as = Const2<T>(ec.as * s2d);
+        c0 = Const2<T>(fma(ec.c0[1], s2d, ec.c0[0]));
+        c1 = Const2<T>(fma(ec.c1[1], s2d, ec.c1[0]));
+        c2 = Const2<T>(ec.c2 * s2d);
+        d0 = Const2<T>(fma(ec.d0[1], s2d, ec.d0[0]));
+        d1 = Const2<T>(fma(ec.d1[1], s2d, ec.d1[0]));
         a2 = (T)ec.a2;
         s2 = (T)s2d;
         hs = (T)(0.5 * s2d);

@@ -35,6 +35,22 @@ static EwaldConst system_ewald(const bdb_system* s)
     e.alpha = e.smith && s->p.ewald_alpha > 0 ? s->p.ewald_alpha : BDB_SQRTPI;
     e.a2 = e.alpha * e.alpha;
     e.isp = e.smith ? BDB_M1_SQRTPI : 1 / BDB_SQRTPI;
+    // of the images' polynomials (diff_tensor.c:336-356): a multiple of
+    // alpha^n / sqrt(pi) each
+    const long double a = e.alpha, a2 = a * a;
+    const long double p1 = e.smith ? a * (long double)BDB_M1_SQRTPI : a / (long double)BDB_SQRTPI;
+    const long double p3 = p1 * a2, p5 = p3 * a2, p7 = p5 * a2;
+    e.e2 = (double)(2 * p1);
+    e.as = (double)p1;
+    e.c0[0] = (double)(-4.5L * p1);
+    e.c0[1] = (double)(14 * p3);
+    e.c1[0] = (double)(3 * p3);
+    e.c1[1] = (double)(-20 * p5);
+    e.c2 = (double)(4 * p7);
+    e.d0[0] = (double)(1.5L * p1);
+    e.d0[1] = (double)(-2 * p3);
+    e.d1[0] = (double)(-3 * p3);
+    e.d1[1] = (double)(16 * p5);
     volatile float pif = BDB_M_PIF;
     volatile float two = 2 * pif;
     e.two_pif = two;

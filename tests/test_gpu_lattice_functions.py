@@ -58,3 +58,47 @@ def test_one_image(alpha, prec, deck_dir):
     else:
         # the exponent's rounding is put back: no growth with x^2
         assert (err <= 6e-8 * 24).all(), err.max() / 6e-8
+
+
+def test_constants_do_not_bias_the_mean(deck_dir):
+    """The polynomials' constants are rounded alike in every image, so a
+    constant that is off by ulps shifts the tensor's mean, which TEA's eps is.
+    Beenakker's tiles of 250 pairs against 40 digits: single errors of 3.4e-15
+    of the tiles' size leave 6.5e-16 in their mean (three standard errors),
+    and the constants, half an ulp each of numbers up to 2.5 where a tile's sum
+    is 0.2, up to 7e-16."""
+    mp = pytest.importorskip("mpmath")
+    R, n = 2, 60
+    d = decks.read_deck(decks.write_suspension_deck(deck_dir, "bias", n, seed=3, ewald_r=R,
+                                                    extra={"hydro": "cholesky"}))
+    s = engine.System(d, precision=engine.PREC_FP64, noise=engine.NOISE_HOST)
+    D = s.compute_D()
+    s.close()
+    box = mp.mpf(float(d.box[0]))
+    root_pi = mp.mpf(1.77245385090551602729)   # as the reference spells it
+    pre = 0.00010537375739171604 * d.prm["T"] / (d.prm["visc"] * d.prm["vfactor"])
+    rng = np.random.default_rng(0)
+    err, size = [], []
+    with mp.workdps(40):
+        a = root_pi / box
+        for _ in range(250):
+            i, j = sorted(rng.choice(n, 2, replace=False))
+            r = [mp.mpf(float(d.coord[i, k])) - mp.mpf(float(d.coord[j, k])) for k in range(3)]
+            s2 = mp.mpf(float(d.coord[i, 3] ** 2 + d.coord[j, 3] ** 2)) / 2
+            tr, sq = mp.mpf(0), 0.0
+            for h, f, g in np.ndindex(2 * R + 1, 2 * R + 1, 2 * R + 1):
+                m = (h - R, f - R, g - R)
+                if sum(q * q for q in m) > R * R:
+                    continue
+                x2 = sum((r[k] + box * m[k]) ** 2 for k in range(3))
+                x, ex = mp.sqrt(x2), mp.exp(-a * a * x2) / root_pi
+                er = mp.erfc(a * x)
+                A = (a * s2 / x2 + 14 * a**3 * s2 - 4.5 * a - 20 * a**5 * s2 * x2 + 3 * a**3 * x2
+                     + 4 * a**7 * s2 * x2**2) * ex + er * (0.75 / x + s2 / (2 * x * x2))
+                B = (-3 * a * s2 / x2 - 2 * a**3 * s2 + 1.5 * a + 16 * a**5 * s2 * x2 - 3 * a**3 * x2
+                     - 4 * a**7 * s2 * x2**2) * ex + er * (0.75 / x - 3 * s2 / (2 * x * x2))
+                tr += 3 * A + B   # (the reciprocal weights are exp(-pi L^2) here)
+            t = D[3 * i:3 * i + 3, 3 * j:3 * j + 3]
+            err.append(float(mp.mpf(float(t[0, 0])) + mp.mpf(float(t[1, 1])) + mp.mpf(float(t[2, 2])) - pre * tr))
+            size.append(np.mean(t * t))
+    assert abs(np.mean(err)) <= 1.4e-15 * np.sqrt(np.mean(size))
