@@ -56,7 +56,12 @@ enum { BDB_EWALD_BEENAKKER = 0, BDB_EWALD_SMITH = 1 };
 enum {
     BDB_PREC_FP64 = 0,   /* everything in FP64 (the plain GPU path) */
     BDB_PREC_MIXED = 1   /* FP32 tensor and stored D/L, FP16-split tcgen05 Cholesky
-                            updates with FP64 diagonal tiles, FP64 sums */
+                            updates with FP64 diagonal tiles, FP64 sums. Matrix-
+                            free pair sums: FP32 over 8 to 16 pairs, FP64 beyond;
+                            lattice sums: images in FP32, reciprocal vectors in
+                            FP64, but for the converged split of the matrix-free
+                            sums (Ewald R >= 4 at the default screening), all
+                            FP32, whose error is smaller */
 };
 
 /* noise sources */
