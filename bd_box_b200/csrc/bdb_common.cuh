@@ -147,7 +147,7 @@ struct bdb_system {
     double ewald_self[2] = {0, 0};             // a bead's sum over its own images: [0] + [1] sigma^2/L^2
     bool ewald_recip = false;                  // some reciprocal weight is not zero
     std::shared_ptr<bdb::EwaldFast> ewald_fast;   // the mixed path's converged split (ewald_fast.cuh), if it holds
-    double radius0 = 0;                        // radius of bead 0 at creation
+    double radius0 = 0, radius_min = 0;        // radius of bead 0 and the least one, at creation
     bdb::DevBuf<double> M64;                   // stored D (upper) + L (lower), FP64
     bdb::DevBuf<float> M32;                    // same, FP32 (mixed path)
     // IGT predictor-corrector: the tensor at the predicted positions, the

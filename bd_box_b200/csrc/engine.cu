@@ -447,7 +447,8 @@ static int create_system(bdb_system** out, const bdb_params* p, int nseg, const 
     s->n = p->n;
     s->n3 = 3 * p->n;
     s->npad = (s->n3 + 127) / 128 * 128;
-    s->radius0 = coord[3];
+    s->radius0 = s->radius_min = coord[3];
+    for (int i = 1; i < p->n; ++i) s->radius_min = std::min(s->radius_min, coord[4 * i + 3]);
     for (int k = 0; k < 3; ++k) s->inv_L[k] = p->bc == 1 ? 1 / p->box[k] : 0.0;
     s->preDii = BDB_KB_1_6PI * p->T / (p->visc * p->vfactor);
     s->preDij = BDB_KB_1_8PI * p->T / (p->visc * p->vfactor);

@@ -509,11 +509,11 @@ __global__ void k_diag_drift(int n, double preDii, const double4* __restrict__ p
 template <typename T, int KIND, bool RS>
 static void tea_pairs(bdb_system* s, const TensorArgs& A, const FastArg<KIND>& E, const TeaSeg* segs)
 {
-    // steps of a 256th of a radius reach 2^15 radii; in L (the converged split)
+    // steps of a 256th of the least radius reach 2^15 of them; in L (the converged split)
     // steps of 2^-22 reach two boxes
     PairUnits u;
     u.unit = KIND == TILE_FAST ? A.ec.inv_L : 1.0;
-    u.step = KIND == TILE_FAST ? std::ldexp(1.0, -22) : std::ldexp(1.0, std::ilogb(s->radius0) - 8);
+    u.step = KIND == TILE_FAST ? std::ldexp(1.0, -22) : std::ldexp(1.0, std::ilogb(s->radius_min) - 8);
     u.inv_step = 1 / u.step;
     k_tea_pairs<T, KIND, RS><<<(s->n_jobs + TEA_WARPS - 1) / TEA_WARPS, 32 * TEA_WARPS, 0, s->stream>>>(
         A, E, s->jobs.p, s->n_jobs, s->tea_cols.p, segs, s->pos.p, s->F.p, s->X.p, reinterpret_cast<T*>(s->part.p),

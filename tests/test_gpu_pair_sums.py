@@ -162,3 +162,22 @@ def test_a_bead_whose_distance_squared_overflows(prec, far, hydro, deck_dir):
         assert np.abs(gone[-3:, :-3]).max() <= 1e-15 * np.abs(gone).max()
     else:   # no force acts on the far bead, nor does it change the others' drift
         assert rel(gone[:-3], near[:-3]) <= (1e-13 if prec == engine.PREC_FP64 else 1e-6)
+
+
+@pytest.mark.parametrize("first", [1.0, 3e4])
+def test_close_pairs_beside_a_large_bead(first, deck_dir):
+    """The grid on which the mixed path's separations are exact follows the
+    least radius: with a first bead 1.5e4 times as large as the others, whose
+    neighbours are a few of their radii away, every separation still rounds
+    like one FP32 operation."""
+    n = 64
+    d = decks.read_deck(decks.write_chain_deck(deck_dir, f"big{int(first)}", n, seed=4, hydro="geyer"))
+    d.coord = d.coord.copy()
+    d.coord[:, :3] *= 0.7
+    d.coord[0] = (5e4, 5e4, 5e4, first)
+    out = {}
+    for p in (engine.PREC_FP64, engine.PREC_MIXED):
+        s = engine.System(d, precision=p, noise=engine.NOISE_HOST)
+        out[p] = s.compute_r(np.random.default_rng(2).standard_normal(3 * n)).reshape(n, 3)
+        s.close()
+    assert rel(out[engine.PREC_MIXED][1:], out[engine.PREC_FP64][1:]) <= 1e-6
