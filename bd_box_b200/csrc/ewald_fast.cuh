@@ -9,7 +9,7 @@
 // multiply-adds each on 21 cosines and sines built from one sincos per axis.
 // About 2,700 instructions per pair (74% of the issue slots), against ~65
 // images of ~60 and 128 cosines in the reference's split, with lanes idle at
-// its cutoff: N = 4096, R = 4 (Beenakker): pair kernel 8.13 -> 0.84 ms.
+// its cutoff: N = 4096, R = 4 (Beenakker): pair kernel 8.13 -> 0.77 ms.
 // The near part is the RPY tensor screened as in Smith's sums (Hasimoto's
 // functions: the least Fourier tail); the Fourier weights are its complement
 // for the periodic RPY tensor (Smith) or, for Beenakker's sums, the

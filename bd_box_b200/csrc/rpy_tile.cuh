@@ -298,7 +298,7 @@ static __device__ __noinline__ void images_one_by_one(const EwaldConst& ec, cons
 // The lattice sum S(v) over the reference's sphere of images and reciprocal
 // vectors, v = (r_i - r_j)/L as it is (no minimum image). Bound by FP64
 // multiply-adds and their latency (about 90 a image; N = 777, R = 3, Smith:
-// 941 -> 356 us per pass over all pairs, against exp, erfc, two square roots or
+// 941 -> 347 us per pass over all pairs, against exp, erfc, two square roots or
 // divisions per image and a cosine per reciprocal vector).
 //
 // FP64: every image of the sphere. An image costs one Gaussian, one erfcx and
